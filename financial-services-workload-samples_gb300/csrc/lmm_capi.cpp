@@ -248,8 +248,7 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
     else if (family == 5) err = lmm::tp2_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 6) err = lmm::tps_blocks_per_sm(philox, &b);
     else if (family == 7) err = lmm::tpq_blocks_per_sm(philox, &b);
-    else if (family == 3) err = lmm::f64_blocks_per_sm(false, &b);
-    else err = lmm::f64_blocks_per_sm(true, &b);
+    else return fail(LMM_ERR_UNSUPPORTED, "unknown kernel family");
     if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
     if (b < 1) return fail(LMM_ERR_UNSUPPORTED, "kernel does not fit on this device");
     e->bps[key] = b;
@@ -298,6 +297,45 @@ int plan(lmm_engine *e, int64_t nvs, int64_t paths, int block, int bps, int nout
     // FP32 kernels: one wave of blocks, each looping over its units
     w->grid = (int)std::min<int64_t>(nvs * items, std::max<int64_t>(1, (int64_t)e->sms * bps));
     LMM_TRY(e->partial.ensure(sizeof(double) * (size_t)(nvs * items) * 2 * nout));
+    w->partial = e->partial.as<double>();
+    return LMM_OK;
+}
+
+// The FP64 launches' plan: block size, items and paths per thread. An SM
+// holds 16 (adjoint) or 20 (bump) warps of any block size, and its time goes
+// with the paths it runs, so the plan takes the block size (a multiple of 32)
+// whose busiest SM gets the fewest paths, the largest at a tie. GB300, 65,536
+// paths (431 per SM): blocks of 256 put 512 on most SMs, 224 at most 448.
+int plan_f64(lmm_engine *e, int64_t nvs, int64_t paths, bool bump, int nout, Work *w)
+{
+    int64_t best = INT64_MAX;
+    for (int block = lmm::f64_block_threads(); block >= 32; block -= 32) {
+        const int key = variant_key(bump ? 4 : 3, Mode::Fused, false) + 256 * block;
+        auto it = e->bps.find(key);
+        if (it == e->bps.end()) {
+            int b = 0;
+            const cudaError_t err = lmm::f64_blocks_per_sm(block, e->nn, e->nmat, e->nopt, bump, &b);
+            if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
+            it = e->bps.emplace(key, b).first;
+        }
+        const int64_t bps = it->second;
+        if (bps < 1) continue;
+        int64_t items = 1, ppt = 1;
+        plan_items(e, nvs, paths, block, (int)bps, &items, &ppt);
+        const int64_t waves = (nvs * items + e->sms * bps - 1) / (e->sms * bps);
+        // paths of the busiest SM; a launch that fills one wave partly leaves some slots of an SM empty
+        const int64_t perSm = waves > 1 ? waves * bps : (nvs * items + e->sms - 1) / e->sms;
+        const int64_t cost = perSm * ppt * block;
+        if (ppt > INT32_MAX || items > INT32_MAX || nvs * items > INT32_MAX || cost >= best) continue;
+        best = cost;
+        w->items = (int)items;
+        w->ppt = (int)ppt;
+        w->block = block;
+    }
+    if (best == INT64_MAX) return fail(LMM_ERR_TOO_LARGE, "launch too large");
+    w->paths = paths;
+    w->nout = nout;
+    LMM_TRY(e->partial.ensure(sizeof(double) * (size_t)(nvs * w->items) * 2 * nout));
     w->partial = e->partial.as<double>();
     return LMM_OK;
 }
@@ -414,11 +452,9 @@ int run_f64(lmm_engine *e, const double *d_z, int64_t paths, double *d_mean, dou
     LMM_TRY(check_paths(paths));
     if (!d_z || !d_mean) return fail(LMM_ERR_INVALID_ARG, "NULL device pointer");
     LMM_TRY(set_device(e));
-    int bps = 0;
-    LMM_TRY(blocks_per_sm(e, 3, Mode::Fused, false, &bps));
     const int nout = 1 + 2 * e->nn;
     Work w{};
-    LMM_TRY(plan(e, e->nscen, paths, lmm::f64_block_threads(), bps, nout, &w));
+    LMM_TRY(plan_f64(e, e->nscen, paths, false, nout, &w));
     LMM_TRY(e->flag.ensure(sizeof(int)));
     LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
     mark(e, 0);
@@ -438,11 +474,9 @@ int run_bump(lmm_engine *e, const double *d_z, int64_t paths, double h, bool cen
     if (!d_z || !d_mean) return fail(LMM_ERR_INVALID_ARG, "NULL device pointer");
     if (!(h > 0.0) || !std::isfinite(h)) return fail(LMM_ERR_INVALID_ARG, "bump h must be finite and > 0");
     LMM_TRY(set_device(e));
-    int bps = 0;
-    LMM_TRY(blocks_per_sm(e, 4, Mode::Fused, false, &bps));
     const int nb = central ? 1 + 4 * e->nn : 1 + 2 * e->nn;
     Work w{};
-    LMM_TRY(plan(e, (int64_t)e->nscen * nb, paths, lmm::f64_block_threads(), bps, 1, &w));
+    LMM_TRY(plan_f64(e, (int64_t)e->nscen * nb, paths, true, 1, &w));
     LMM_TRY(e->flag.ensure(sizeof(int)));
     // central: the 1+4nn variant means (and their standard errors) go to the
     // engine's scratch and are differenced into the caller's 1+2nn outputs

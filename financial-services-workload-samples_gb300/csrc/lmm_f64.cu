@@ -3,25 +3,33 @@
 // comparator (forward only, re-run with each input bumped).
 //
 // One thread per path, runtime NN/NMAT (<= kMaxNN), per-thread state in local
-// memory. The arithmetic follows the reference formula by formula:
-//   forward  path_calc_b1 (LiborMarketModel/liborSwaptionGreeks.cpp:50-81)
-//   payoff   portfolio_b  (:133-209, with the :178/:181 aliasing fixed)
-//   reverse  path_calc_b2 (:94-116) in log-adjoint form, running the Euler
-//            step backwards from the saved per-step drift sums (no stored
-//            trajectory), plus the vega adjoint.
+// memory. The Euler steps (path_calc_b1, LiborMarketModel/
+// liborSwaptionGreeks.cpp:50-81) run in 64-bit fixed point (lmm_fix64.h), the
+// payoff (portfolio_b :133-209, with the :178/:181 aliasing fixed) and the
+// adjoint sums (path_calc_b2 :94-116 in log-adjoint form, plus the vega
+// adjoint) in FP64. The reverse subtracts the forward's integer increments,
+// so it returns to the forward's rates bit for bit without a trajectory. A
+// path with a normal or a rate outside the fixed-point range is computed by
+// the plain FP64 code (f64_path), formula by formula as the reference.
+//
+// Measured on GB300, all in FP64 -> fixed-point steps: 65,536 paths with the
+// adjoint 25.35 -> 2.60 ms, bump-and-revalue of 16,384 paths (161 forward
+// runs) 385.5 -> 28.7 ms. In FP64 a cell took two exps and two divides, the
+// FP64 pipe 87% busy; now it takes four DFMAs, in the reverse only. Error of a
+// path against 80-bit arithmetic (root mean square, 80/40 and 160/120): 8.7e-16
+// and 1.3e-15 before, 5.7e-16 and 8.8e-16 now; of the mean over paths 5e-17 both.
 #include "lmm_device.cuh"
+#include "lmm_fix64.h"
 
 namespace lmm {
 namespace {
 
-constexpr int kF64Block = 128;
-
-struct F64Smem {
-    double *lam;     // [nn]
-    int *ost;        // [nn-nmat+1]
-    double *okd;     // [nopt]
-    double *acc;     // [NW][2*nout]
-};
+// Launches take a block of 32 to kF64Block threads (launch plan in
+// lmm_capi.cpp). Registers for 16 warps per SM with the adjoint, 20 without:
+// GB300, 65,536 paths 2.54 ms with 16 warps, 2.63 with 20 (it spills), 2.91
+// with 12; bump 16,384 paths x 161 runs 27.0 ms with 20 or 16.
+constexpr int kF64Block = 256;
+constexpr int kF64MinBlocks = 2, kF64MinBlocksBump = 2;
 
 // portfolio_b :133-171 and :186-197 in FP64; returns the discounted value.
 // Bst (if given) receives the annuity factors B[m] of :139 for the adjoint.
@@ -66,105 +74,413 @@ __device__ void forward_f64(double *L, double *Vt, const double *z, const double
     }
 }
 
-__global__ void __launch_bounds__(kF64Block)
+// One path in plain FP64: value, log-adjoints Pb = L dV/dL at step 0 and
+// vegas per sigma. L, Vt and Bs [kMaxNN] are scratch.
+__device__ __noinline__ double f64_path(const DevModel &m, const double *L0, const double *zp, const double *lam,
+                                        const int *ost, const double *okd, const double *okw, double *L, double *Vt,
+                                        double *Bs, double *Pb, double *vg)
+{
+    const int nn = m.nn, nmat = m.nmat, M = nn - nmat;
+    const double d = m.deltad, sqd = m.sqdd;
+    for (int i = 0; i < nn; ++i) {
+        L[i] = L0[i];
+        vg[i] = 0.0;
+    }
+    forward_f64(L, Vt, zp, lam, nn, nmat, d, sqd);
+    double disc;
+    unsigned long long mask;
+    const double V = payoff_value_f64(L, nn, nmat, d, ost, okd, okw, &disc, Bs, &mask);
+    // payoff adjoint (:173-184 with the rate kept apart from its adjoint,
+    // then :199-209), written as log-adjoints Pb = L * dV/dL. B[m] comes
+    // from the forward as in the reference: rebuilding it backwards from
+    // the last factor underflows on paths whose rates explode.
+    double Sb = 0.0, Bb = 0.0;
+    for (int mm = M - 1; mm >= 0; --mm) {
+        const double Bm = Bs[mm];
+        const double Ln = L[nmat + mm];
+        for (int o = ost[mm]; o < ost[mm + 1]; ++o) {
+            if ((mask >> o) & 1ull) {
+                Sb += (-100.0 * okd[o]) * okw[o];
+                Bb += -100.0 * okw[o];
+            }
+        }
+        Bb += d * Sb;
+        const double den = 1.0 + d * Ln;
+        Pb[nmat + mm] = disc * (-Bb * Bm * d / den) * Ln;
+        Bb = Bb / den;
+    }
+    for (int n = 0; n < nmat; ++n) Pb[n] = (-V * d / (1.0 + d * L[n])) * L[n];
+    for (int n = nmat - 1; n >= 0; --n) {
+        const double sqez = sqd * zp[n];
+        double v = Vt[n], v1 = 0.0;
+        for (int i = nn - 1; i > n; --i) {
+            const double l = lam[i - n - 1];
+            const double con1 = d * l;
+            const double wexp = con1 * v + l * (sqez - 0.5 * con1);
+            const double Ln = L[i] * exp(-wexp);         // L_{n,i} from L_{n+1,i}
+            const double r = 1.0 / (1.0 + d * Ln);
+            const double t = Ln * r;
+            const double pb = Pb[i];
+            v1 += l * pb;                                 // :108
+            vg[i - n - 1] += pb * (d * v + sqez - d * l) + d * d * t * v1;
+            Pb[i] = pb + d * con1 * t * r * v1;           // :110-111 in log form
+            v -= con1 * t;
+            L[i] = Ln;
+        }
+    }
+    for (int k = 0; k < nn; ++k) vg[k] /= sqd;
+    return V;
+}
+
+// Value of one path in plain FP64; L [kMaxNN] is scratch.
+__device__ __noinline__ double f64_path_value(const DevModel &m, const double *L0, int bumped, double hb,
+                                              const double *zp, const double *lam, const int *ost, const double *okd,
+                                              const double *okw, double *L)
+{
+    for (int i = 0; i < m.nn; ++i) L[i] = L0[i] + (i == bumped ? hb : 0.0);
+    forward_f64(L, nullptr, zp, lam, m.nn, m.nmat, m.deltad, m.sqdd);
+    double disc;
+    unsigned long long mask;
+    return payoff_value_f64(L, m.nn, m.nmat, m.deltad, ost, okd, okw, &disc, nullptr, &mask);
+}
+
+// The block's model in shared memory.
+struct F64Shared {
+    FxConst *fc;        // [nn] fixed-point constants by time to maturity
+    uint64_t *tab;      // [kFxTable]
+    uint64_t *x0;       // [nn] the curve
+    double *lam;        // [nn]
+    double *okd, *okw;  // [nopt] strikes, weights
+    double *acc;        // [NW][2*nout]
+    double *tile;       // [NW][kTileRows * 32] (k_f64_greeks)
+    int *ost;           // [nn-nmat+1]
+};
+constexpr int kTileCols = 8;                        // outputs transposed at a time
+constexpr int kTileRow = kTileCols + 1;             // doubles per path, padded
+static_assert(32 % kTileCols == 0, "32 / kTileCols groups of kTileCols paths");
+
+__host__ __device__ inline size_t f64_smem(int NW, int nn, int nmat, int nopt, int nout, bool tile, F64Shared *s,
+                                           unsigned char *base)
+{
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+        unsigned char *p = base + o;
+        o += (bytes + 15) & ~size_t(15);
+        return p;
+    };
+    s->fc = reinterpret_cast<FxConst *>(take(sizeof(FxConst) * nn));
+    s->tab = reinterpret_cast<uint64_t *>(take(8 * kFxTable));
+    s->x0 = reinterpret_cast<uint64_t *>(take(8 * (size_t)nn));
+    s->lam = reinterpret_cast<double *>(take(8 * (size_t)nn));
+    s->okd = reinterpret_cast<double *>(take(8 * (size_t)nopt));
+    s->okw = reinterpret_cast<double *>(take(8 * (size_t)nopt));
+    s->acc = reinterpret_cast<double *>(take(8 * (size_t)NW * 2 * nout));
+    s->tile = reinterpret_cast<double *>(take(tile ? 8 * (size_t)NW * 32 * kTileRow : 0));
+    s->ost = reinterpret_cast<int *>(take(4 * (size_t)(nn - nmat + 1)));
+    return o;
+}
+
+// Fills it; `bl`, `bx` (-1: none): the lambda and the rate bumped by hb.
+// Returns (to every thread) whether the fixed-point steps cover the model.
+__device__ bool f64_load(const DevModel &m, const F64Shared &s, int scen, int nacc, int bl, int bx, double hb)
+{
+    const int nn = m.nn, tid = threadIdx.x, nt = blockDim.x;
+    bool ok = true;
+    for (int j = tid; j < kFxTable; j += nt) s.tab[j] = fx_table_entry(j);
+    for (int i = tid; i <= nn - m.nmat; i += nt) s.ost[i] = m.opt_start[i];
+    for (int i = tid; i < m.nopt; i += nt) {
+        s.okd[i] = m.optKd[i];
+        s.okw[i] = m.optWd[i];
+    }
+    for (int i = tid; i < nacc; i += nt) s.acc[i] = 0.0;
+    for (int i = tid; i < nn; i += nt) {
+        const double l = m.lamd[i] + (i == bl ? hb : 0.0), sg = l * m.sqdd;
+        s.lam[i] = l;
+        ok = ok && sg >= 0.0 && sg <= kFxSigmaMax;
+        s.fc[i] = fx_const(sg >= 0.0 && sg <= kFxSigmaMax ? sg : 0.0, i);
+    }
+    __syncthreads();
+    for (int i = tid; i < nn; i += nt) {
+        const double v = m.deltad * (m.L0d[(size_t)scen * nn + i] + (i == bx ? hb : 0.0));
+        s.x0[i] = fx_rate(v, log2(v), s.tab);
+    }
+    return __syncthreads_and(ok);
+}
+
+// One forward cell; `range` collects the values whose top bit tells a rate or
+// a drift sum outside the fixed-point range.
+__device__ __forceinline__ void fx_fwd_cell(uint64_t &x, uint64_t &Y, const FxConst &k, const uint64_t *tab,
+                                            uint64_t &range)
+{
+    const FxT q = fx_logistic(x, tab);
+    range |= x;
+    Y += fx_drift(q, k);
+    range |= Y;
+    x = fx_step(x, Y, k);
+}
+
+// Forward over all steps from the curve: X receives the terminal rates, Yt
+// (if given) each step's Y at the top rate. Returns false if a normal or a
+// rate left the fixed-point range. Steps run in pairs as a skewed wavefront,
+// cell (n, i) next to cell (n+1, i-1): two independent drift chains, and each
+// rate is loaded and stored once per two steps.
+__device__ __forceinline__ bool fx_forward(uint64_t *X, uint64_t *Yt, const double *zp, const F64Shared &s, int nn,
+                                           int nmat)
+{
+    for (int i = 0; i < nn; ++i) X[i] = s.x0[i];
+    uint64_t range = 0;
+    bool ok = true;
+    double z0 = zp[0], z1 = nmat > 1 ? zp[1] : 0.0;
+    for (int n = 0; n < nmat; n += 2) {
+        const bool two = n + 1 < nmat;
+        ok = ok && fabs(z0) < kFxZMax && fabs(z1) < kFxZMax;
+        uint64_t Y0 = fx_normal(z0), Y1 = fx_normal(z1);
+        if (n + 2 < nmat) z0 = zp[n + 2];
+        z1 = n + 3 < nmat ? zp[n + 3] : 0.0;
+        const FxConst *k0 = s.fc - (n + 1);          // k0[i]: constants of cell (n, i)
+        if (two) {
+            uint64_t xl = X[n + 1];                  // rate i-1 after step n
+            fx_fwd_cell(xl, Y0, k0[n + 1], s.tab, range);
+            X[n + 1] = xl;
+            if (n + 2 < nn) {
+                xl = X[n + 2];
+                fx_fwd_cell(xl, Y0, k0[n + 2], s.tab, range);
+                uint64_t xn = n + 3 < nn ? X[n + 3] : 0;
+#pragma unroll 2
+                for (int i = n + 3; i < nn; ++i) {
+                    uint64_t x = xn;
+                    if (i + 1 < nn) xn = X[i + 1];
+                    fx_fwd_cell(x, Y0, k0[i], s.tab, range);
+                    fx_fwd_cell(xl, Y1, k0[i - 2], s.tab, range);
+                    X[i - 1] = xl;
+                    xl = x;
+                }
+                fx_fwd_cell(xl, Y1, k0[nn - 2], s.tab, range);
+                X[nn - 1] = xl;
+            }
+        } else {
+            for (int i = n + 1; i < nn; ++i) {
+                uint64_t x = X[i];
+                fx_fwd_cell(x, Y0, k0[i], s.tab, range);
+                X[i] = x;
+            }
+        }
+        if (Yt) {
+            Yt[n] = Y0;
+            if (two) Yt[n + 1] = Y1;
+        }
+    }
+    for (int i = 0; i < nn; ++i) range |= X[i];
+    return ok && (range >> 63) == 0;
+}
+
+// One reverse cell: undoes the step of rate x at drift sum Y and adds the
+// cell's terms, in units of sigma = lambda sqrt(delta) (path_calc_b2
+// :108-111 in log form, and the vega):
+//   S += sigma Pb, vega_k += Pb (y - sigma) + t S, Pb += sigma t (1-t) S.
+__device__ __forceinline__ void fx_rev_cell(uint64_t &x, uint64_t &Y, double &S, double &pb, double &vega,
+                                            const FxConst &k, const uint64_t *tab)
+{
+    x = fx_unstep(x, Y, k);
+    const FxT q = fx_logistic(x, tab);
+    const double t = fx_t(q), h = fx_signed((int64_t)(Y - k.h)), w = fx_slope(q, k);
+    S = fma(k.sg, pb, S);
+    vega = fma(t, S, fma(pb, h, vega));
+    pb = fma(w, S, pb);
+    Y -= fx_drift(q, k);
+}
+
+// Reverse over all steps from the terminal rates and their log-adjoints, in
+// the forward's pairs: cell (n, i) next to cell (n-1, i+1), whose constants
+// are those of k+2. Each rate, log-adjoint and vega row is loaded and stored
+// once per two steps (an open vega row passes through v0, v1, v2).
+__device__ __forceinline__ void fx_reverse(uint64_t *X, const uint64_t *Yt, double *Pb, double *vg, const F64Shared &s,
+                                           int nn, int nmat)
+{
+    int n = nmat - 1;
+    if (nmat & 1) {
+        uint64_t Y = Yt[n];
+        double S = 0.0;
+        for (int i = nn - 1; i > n; --i) fx_rev_cell(X[i], Y, S, Pb[i], vg[i - n - 1], s.fc[i - n - 1], s.tab);
+        --n;
+    }
+    for (; n > 0; n -= 2) {
+        uint64_t Y0 = Yt[n], Y1 = Yt[n - 1];
+        double S0 = 0.0, S1 = 0.0;
+        const FxConst *k0 = s.fc - (n + 1);
+        double *v = vg - (n + 1);
+        // Cell (n, i) works on row v[i], cell (n-1, i+1) on row v[i+2]. Before
+        // position i: rate i+1 after step n in xh, ph, the open rows v[i+1] in
+        // va and v[i+2] in vb, position i's own values in xn, pn, vn.
+        uint64_t xh = X[nn - 1];
+        double ph = Pb[nn - 1], va = v[nn - 1], vb = v[nn];
+        fx_rev_cell(xh, Y0, S0, ph, va, k0[nn - 1], s.tab);
+        int i = nn - 2;
+        uint64_t xn = X[i];
+        double pn = Pb[i], vn = i > n ? v[i] : 0.0;
+#pragma unroll 2
+        for (; i > n; --i) {
+            uint64_t x = xn;
+            double p = pn, vv = vn;
+            xn = X[i - 1];
+            pn = Pb[i - 1];
+            if (i - 1 > n) vn = v[i - 1];
+            fx_rev_cell(x, Y0, S0, p, vv, k0[i], s.tab);
+            fx_rev_cell(xh, Y1, S1, ph, vb, k0[i + 2], s.tab);
+            X[i + 1] = xh;
+            Pb[i + 1] = ph;
+            v[i + 2] = vb;
+            vb = va;
+            va = vv;
+            xh = x;
+            ph = p;
+        }
+        // i = n: cell (n-1, n+1) on row v[n+2] (k = 1); then (n-1, n), k = 0
+        fx_rev_cell(xh, Y1, S1, ph, vb, k0[n + 2], s.tab);
+        X[n + 1] = xh;
+        Pb[n + 1] = ph;
+        v[n + 2] = vb;
+        fx_rev_cell(xn, Y1, S1, pn, va, k0[n + 1], s.tab);
+        X[n] = xn;
+        Pb[n] = pn;
+        v[n + 1] = va;
+    }
+}
+
+// portfolio_b :133-171 and :186-197 from the terminal rates' t (1/(1+dL) =
+// 1 - t); returns the discounted value. With ADJ, Bst receives the annuity
+// factors B[m] of :139, Pb the t and Rt the 1 - t of the annuity rates.
+template <bool ADJ>
+__device__ __forceinline__ double fx_payoff(const uint64_t *X, const F64Shared &s, int nn, int nmat, double d,
+                                            double *disc_out, double *Bst, double *Pb, double *Rt,
+                                            unsigned long long *mask_out)
+{
+    double b = 1.0, sum = 0.0, vs = 0.0, disc = 1.0;
+    unsigned long long mask = 0ull;
+    for (int m = 0; m < nn - nmat; ++m) {
+        const FxT q = fx_logistic(X[nmat + m], s.tab);
+        const double r = fx_1mt(q);
+        b *= r;
+        sum = fma(d, b, sum);
+        if (ADJ) {
+            Pb[nmat + m] = fx_t(q);
+            Rt[m] = r;
+            Bst[m] = b;
+        }
+        for (int o = s.ost[m]; o < s.ost[m + 1]; ++o) {
+            const double sw = fma(s.okd[o], sum, b) - 1.0;
+            if (sw < 0.0) {
+                vs = fma(-100.0 * sw, s.okw[o], vs);
+                mask |= 1ull << o;
+            }
+        }
+    }
+    for (int n = 0; n < nmat; ++n) {
+        const FxT q = fx_logistic(X[n], s.tab);
+        disc *= fx_1mt(q);
+        if (ADJ) Pb[n] = fx_t(q);
+    }
+    *disc_out = disc;
+    *mask_out = mask;
+    return disc * vs;
+}
+
+__global__ void __launch_bounds__(kF64Block, kF64MinBlocks)
 k_f64_greeks(const DevModel m, const double *__restrict__ z, const Work w)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nn = m.nn, nmat = m.nmat, M = nn - nmat, nout = w.nout;
-    const int NW = kF64Block / 32;
-    double *lam_s = reinterpret_cast<double *>(smem);
-    double *okd_s = lam_s + kMaxNN;
-    double *okw_s = okd_s + kMaxNopt;
-    double *acc_s = okw_s + kMaxNopt;
-    int *ost_s = reinterpret_cast<int *>(acc_s + NW * 2 * nout);
+    const int nt = blockDim.x, NW = nt / 32;
+    F64Shared s;
+    f64_smem(NW, nn, nmat, m.nopt, nout, true, &s, smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int scen = blockIdx.x / w.items, item = blockIdx.x % w.items;
-    for (int i = tid; i < nn; i += kF64Block) lam_s[i] = m.lamd[i];
-    for (int i = tid; i <= M; i += kF64Block) ost_s[i] = m.opt_start[i];
-    for (int i = tid; i < m.nopt; i += kF64Block) {
-        okd_s[i] = m.optKd[i];
-        okw_s[i] = m.optWd[i];
-    }
-    for (int i = tid; i < NW * 2 * nout; i += kF64Block) acc_s[i] = 0.0;
-    __syncthreads();
-    double *acc = acc_s + warp * 2 * nout;
-    const double d = m.deltad, sqd = m.sqdd;
+    const bool fixed = f64_load(m, s, scen, NW * 2 * nout, -1, -1, 0.0);
+    double *acc = s.acc + warp * 2 * nout;
+    double *tile = s.tile + warp * 32 * kTileRow;
+    const double d = m.deltad;
     const double *L0 = m.L0d + (size_t)scen * nn;
 
-    double L[kMaxNN], Pb[kMaxNN], vg[kMaxNN], Vt[kMaxNN], Bs[kMaxNN];
-    const int64_t ibase = (int64_t)item * w.ppt * kF64Block;
+    uint64_t X[kMaxNN], Yt[kMaxNN];
+    double Pb[kMaxNN], vg[kMaxNN], Rt[kMaxNN];   // vg holds the annuity factors until the reverse
+    const int64_t ibase = (int64_t)item * w.ppt * nt;
     for (int j = 0; j < w.ppt; ++j) {
-        if (ibase + (int64_t)j * kF64Block >= w.paths) break;
-        const int64_t pl = ibase + (int64_t)j * kF64Block + tid;
+        if (ibase + (int64_t)j * nt >= w.paths) break;
+        const int64_t pl = ibase + (int64_t)j * nt + tid;
         const bool active = pl < w.paths;
         const double *zp = z + (active ? pl : w.paths - 1) * nmat;
-        for (int i = 0; i < nn; ++i) {
-            L[i] = L0[i];
-            vg[i] = 0.0;
-        }
-        forward_f64(L, Vt, zp, lam_s, nn, nmat, d, sqd);
-        double disc;
-        unsigned long long mask;
-        const double V = payoff_value_f64(L, nn, nmat, d, ost_s, okd_s, okw_s, &disc, Bs, &mask);
-        // payoff adjoint (:173-184 with the rate kept apart from its adjoint,
-        // then :199-209), written as log-adjoints Pb = L * dV/dL. B[m] comes
-        // from the forward as in the reference: rebuilding it backwards from
-        // the last factor underflows on paths whose rates explode.
-        {
+        double V = 0.0;
+        if (fixed && fx_forward(X, Yt, zp, s, nn, nmat)) {
+            double disc;
+            unsigned long long mask;
+            V = fx_payoff<true>(X, s, nn, nmat, d, &disc, vg, Pb, Rt, &mask);
+            // payoff adjoint (:173-184 with the rate kept apart from its
+            // adjoint, then :199-209) as log-adjoints Pb = L dV/dL
             double Sb = 0.0, Bb = 0.0;
             for (int mm = M - 1; mm >= 0; --mm) {
-                const double Bm = Bs[mm];
-                const double Ln = L[nmat + mm];
-                for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
+                for (int o = s.ost[mm]; o < s.ost[mm + 1]; ++o) {
                     if ((mask >> o) & 1ull) {
-                        Sb += (-100.0 * okd_s[o]) * okw_s[o];
-                        Bb += -100.0 * okw_s[o];
+                        Sb = fma(-100.0 * s.okd[o], s.okw[o], Sb);
+                        Bb = fma(-100.0, s.okw[o], Bb);
                     }
                 }
-                Bb += d * Sb;
-                const double den = 1.0 + d * Ln;
-                Pb[nmat + mm] = disc * (-Bb * Bm * d / den) * Ln;
-                Bb = Bb / den;
+                Bb = fma(d, Sb, Bb);
+                const double t = Pb[nmat + mm];
+                Pb[nmat + mm] = -disc * Bb * vg[mm] * t;
+                Bb *= Rt[mm];
             }
-            for (int n = 0; n < nmat; ++n) Pb[n] = (-V * d / (1.0 + d * L[n])) * L[n];
+            for (int n = 0; n < nmat; ++n) Pb[n] = -V * Pb[n];
+            for (int k = 0; k < nn; ++k) vg[k] = 0.0;
+            fx_reverse(X, Yt, Pb, vg, s, nn, nmat);
+        } else {
+            V = f64_path(m, L0, zp, s.lam, s.ost, s.okd, s.okw, reinterpret_cast<double *>(X),
+                         reinterpret_cast<double *>(Yt), Rt, Pb, vg);
         }
-        for (int n = nmat - 1; n >= 0; --n) {
-            const double sqez = sqd * zp[n];
-            double v = Vt[n], v1 = 0.0;
-            for (int i = nn - 1; i > n; --i) {
-                const double l = lam_s[i - n - 1];
-                const double con1 = d * l;
-                const double wexp = con1 * v + l * (sqez - 0.5 * con1);
-                const double Ln = L[i] * exp(-wexp);         // L_{n,i} from L_{n+1,i}
-                const double r = 1.0 / (1.0 + d * Ln);
-                const double t = Ln * r;
-                const double pb = Pb[i];
-                v1 += l * pb;                                 // :108
-                vg[i - n - 1] += pb * (d * v + sqez - d * l) + d * d * t * v1;
-                Pb[i] = pb + d * con1 * t * r * v1;           // :110-111 in log form
-                v -= con1 * t;
-                L[i] = Ln;
+        // reduce this batch: value, L0 delta, vega per sigma. kTileCols outputs at a
+        // time through a shared-memory tile: lane (c, q) adds column c over
+        // 8 of the warp's 32 paths (a DADD and a DFMA per output and path,
+        // where a shuffle tree takes ten).
+        __syncwarp();
+        for (int o0 = 0; o0 < nout; o0 += kTileCols) {
+            for (int c = 0; c < kTileCols && o0 + c < nout; ++c) {
+                const int o = o0 + c;
+                double x;
+                if (o == 0) x = V;
+                else if (o <= nn) x = Pb[o - 1];
+                else x = vg[o - 1 - nn];
+                tile[lane * kTileRow + c] = active ? x : 0.0;
             }
-        }
-        // reduce this batch: value, deltas Pb/L0, vegas
-        for (int o = 0; o < nout; ++o) {
-            double x;
-            if (o == 0) x = V;
-            else if (o <= nn) x = Pb[o - 1] / L0[o - 1];
-            else x = vg[o - 1 - nn];
-            x = active ? x : 0.0;
-            const double s1 = warp_sum(x), s2 = warp_sum(x * x);
-            if (lane == 0) {
-                acc[o] += s1;
-                acc[nout + o] += s2;
+            __syncwarp();
+            const int c = lane & (kTileCols - 1), q = lane / kTileCols;
+            double s1 = 0.0, s2 = 0.0;
+            if (o0 + c < nout) {
+#pragma unroll
+                for (int p = 0; p < kTileCols; ++p) {
+                    const double x = tile[(q * kTileCols + p) * kTileRow + c];
+                    s1 += x;
+                    s2 = fma(x, x, s2);
+                }
             }
+#pragma unroll
+            for (int x = kTileCols; x < 32; x *= 2) {
+                s1 += __shfl_xor_sync(0xffffffffu, s1, x);
+                s2 += __shfl_xor_sync(0xffffffffu, s2, x);
+            }
+            if (q == 0 && o0 + c < nout) {
+                acc[o0 + c] += s1;
+                acc[nout + o0 + c] += s2;
+            }
+            __syncwarp();
         }
     }
     __syncthreads();
-    for (int o = tid; o < 2 * nout; o += kF64Block) {
-        double s = 0.0;
-        for (int q = 0; q < NW; ++q) s += acc_s[q * 2 * nout + o];
-        w.partial[(size_t)blockIdx.x * 2 * nout + o] = s;
+    for (int o = tid; o < 2 * nout; o += nt) {
+        double sum = 0.0;
+        for (int q = 0; q < NW; ++q) sum += s.acc[q * 2 * nout + o];
+        // the sums in the outputs' units: deltas per L0, vegas per lambda
+        const int c = o < nout ? o : o - nout;
+        const double f = c == 0 ? 1.0 : (c <= nn ? 1.0 / L0[c - 1] : m.sqdd);
+        w.partial[(size_t)blockIdx.x * 2 * nout + o] = sum * (o < nout ? f : f * f);
     }
 }
 
@@ -172,17 +488,14 @@ k_f64_greeks(const DevModel m, const double *__restrict__ z, const Work w)
 // = (scenario, variant j); j = 0 is the base, j = 1..nn bumps L0[j-1] by h,
 // j = nn+1..2nn bumps lambda[j-nn-1] by h; with `central`, j = 2nn+1..4nn
 // repeat those 2nn inputs bumped by -h. Output per variant: mean value.
-__global__ void __launch_bounds__(kF64Block)
+__global__ void __launch_bounds__(kF64Block, kF64MinBlocksBump)
 k_f64_bump(const DevModel m, const double *__restrict__ z, double h, int central, const Work w)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int nn = m.nn, nmat = m.nmat, M = nn - nmat;
-    const int NW = kF64Block / 32;
-    double *lam_s = reinterpret_cast<double *>(smem);
-    double *okd_s = lam_s + kMaxNN;
-    double *okw_s = okd_s + kMaxNopt;
-    double *acc_s = okw_s + kMaxNopt;
-    int *ost_s = reinterpret_cast<int *>(acc_s + NW * 2);
+    const int nn = m.nn, nmat = m.nmat;
+    const int nt = blockDim.x, NW = nt / 32;
+    F64Shared s;
+    f64_smem(NW, nn, nmat, m.nopt, 1, false, &s, smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = central ? 1 + 4 * nn : 1 + 2 * nn;
     const int vs = blockIdx.x / w.items, item = blockIdx.x % w.items;
@@ -190,72 +503,75 @@ k_f64_bump(const DevModel m, const double *__restrict__ z, double h, int central
     // input bumped: 1..nn the rate L0[var-1], nn+1..2nn lambda[var-nn-1]; by hb
     const int var = vb > 2 * nn ? vb - 2 * nn : vb;
     const double hb = vb > 2 * nn ? -h : h;
-    for (int i = tid; i < nn; i += kF64Block)
-        lam_s[i] = m.lamd[i] + ((var > nn && i == var - nn - 1) ? hb : 0.0);
-    for (int i = tid; i <= M; i += kF64Block) ost_s[i] = m.opt_start[i];
-    for (int i = tid; i < m.nopt; i += kF64Block) {
-        okd_s[i] = m.optKd[i];
-        okw_s[i] = m.optWd[i];
-    }
-    if (tid < NW * 2) acc_s[tid] = 0.0;
-    __syncthreads();
-    const double d = m.deltad, sqd = m.sqdd;
+    const int bx = var >= 1 && var <= nn ? var - 1 : -1, bl = var > nn ? var - nn - 1 : -1;
+    const bool fixed = f64_load(m, s, scen, NW * 2, bl, bx, hb);
+    double *acc = s.acc + warp * 2;
     const double *L0 = m.L0d + (size_t)scen * nn;
-    double L[kMaxNN];
-    const int64_t ibase = (int64_t)item * w.ppt * kF64Block;
+    uint64_t X[kMaxNN];
+    const int64_t ibase = (int64_t)item * w.ppt * nt;
     for (int j = 0; j < w.ppt; ++j) {
-        if (ibase + (int64_t)j * kF64Block >= w.paths) break;
-        const int64_t pl = ibase + (int64_t)j * kF64Block + tid;
+        if (ibase + (int64_t)j * nt >= w.paths) break;
+        const int64_t pl = ibase + (int64_t)j * nt + tid;
         const bool active = pl < w.paths;
         const double *zp = z + (active ? pl : w.paths - 1) * nmat;
-        for (int i = 0; i < nn; ++i) L[i] = L0[i] + ((var >= 1 && var <= nn && i == var - 1) ? hb : 0.0);
-        forward_f64(L, nullptr, zp, lam_s, nn, nmat, d, sqd);
-        double disc;
-        unsigned long long mask;
-        double V = payoff_value_f64(L, nn, nmat, d, ost_s, okd_s, okw_s, &disc, nullptr, &mask);
+        double V;
+        if (fixed && fx_forward(X, nullptr, zp, s, nn, nmat)) {
+            double disc;
+            unsigned long long mask;
+            V = fx_payoff<false>(X, s, nn, nmat, m.deltad, &disc, nullptr, nullptr, nullptr, &mask);
+        } else {
+            V = f64_path_value(m, L0, bx, hb, zp, s.lam, s.ost, s.okd, s.okw, reinterpret_cast<double *>(X));
+        }
         V = active ? V : 0.0;
+        __syncwarp();
         const double s1 = warp_sum(V), s2 = warp_sum(V * V);
         if (lane == 0) {
-            acc_s[warp * 2] += s1;
-            acc_s[warp * 2 + 1] += s2;
+            acc[0] += s1;
+            acc[1] += s2;
         }
     }
     __syncthreads();
     if (tid < 2) {
-        double s = 0.0;
-        for (int q = 0; q < NW; ++q) s += acc_s[q * 2 + tid];
-        w.partial[(size_t)blockIdx.x * 2 + tid] = s;
+        double sum = 0.0;
+        for (int q = 0; q < NW; ++q) sum += s.acc[q * 2 + tid];
+        w.partial[(size_t)blockIdx.x * 2 + tid] = sum;
     }
 }
 
-size_t f64_smem_bytes(int nout)
+size_t f64_smem_bytes(int block, int nn, int nmat, int nopt, bool bump)
 {
-    return sizeof(double) * (kMaxNN + 2 * kMaxNopt + (kF64Block / 32) * 2 * (size_t)nout) +
-           sizeof(int) * (kMaxNN + 1);
+    F64Shared s;
+    return f64_smem(block / 32, nn, nmat, nopt, bump ? 1 : 1 + 2 * nn, !bump, &s, nullptr);
+}
+
+// Allows k the shared memory of the largest accepted shape that fits an SM.
+template <class K>
+cudaError_t f64_allow(K k)
+{
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
 }  // namespace
 
 int f64_block_threads() { return kF64Block; }
 
-cudaError_t f64_blocks_per_sm(bool bump, int *blocks)
+cudaError_t f64_blocks_per_sm(int block, int nn, int nmat, int nopt, bool bump, int *blocks)
 {
-    if (bump) {
-        const size_t sm = f64_smem_bytes(1);
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_f64_bump, kF64Block, sm);
-    }
-    const size_t sm = f64_smem_bytes(1 + 2 * kMaxNN);
-    cudaError_t e = cudaFuncSetAttribute(k_f64_greeks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const size_t sm = f64_smem_bytes(block, nn, nmat, nopt, bump);
+    *blocks = 0;
+    if (sm > 227 * 1024) return cudaSuccess;
+    cudaError_t e = bump ? f64_allow(k_f64_bump) : f64_allow(k_f64_greeks);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_f64_greeks, kF64Block, sm);
+    return bump ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_f64_bump, block, sm)
+                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_f64_greeks, block, sm);
 }
 
 cudaError_t launch_f64_greeks(const DevModel &m, const double *z, const Work &w, cudaStream_t s)
 {
-    const size_t sm = f64_smem_bytes(w.nout);
-    cudaError_t e = cudaFuncSetAttribute(k_f64_greeks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f64_smem_bytes(1 + 2 * kMaxNN));
+    cudaError_t e = f64_allow(k_f64_greeks);
     if (e != cudaSuccess) return e;
-    k_f64_greeks<<<(unsigned)((int64_t)m.nscen * w.items), kF64Block, sm, s>>>(m, z, w);
+    k_f64_greeks<<<(unsigned)((int64_t)m.nscen * w.items), w.block, f64_smem_bytes(w.block, m.nn, m.nmat, m.nopt, false),
+                   s>>>(m, z, w);
     return cudaGetLastError();
 }
 
@@ -263,8 +579,10 @@ cudaError_t launch_f64_bump(const DevModel &m, const double *z, double h, bool c
                             cudaStream_t s)
 {
     const int nb = central ? 1 + 4 * m.nn : 1 + 2 * m.nn;
-    const size_t sm = f64_smem_bytes(1);
-    k_f64_bump<<<(unsigned)((int64_t)m.nscen * nb * w.items), kF64Block, sm, s>>>(m, z, h, central ? 1 : 0, w);
+    cudaError_t e = f64_allow(k_f64_bump);
+    if (e != cudaSuccess) return e;
+    k_f64_bump<<<(unsigned)((int64_t)m.nscen * nb * w.items), w.block,
+                 f64_smem_bytes(w.block, m.nn, m.nmat, m.nopt, true), s>>>(m, z, h, central ? 1 : 0, w);
     return cudaGetLastError();
 }
 

@@ -46,6 +46,7 @@ struct Work {
     int nout;             // outputs per scenario reduced by this launch
     int grid = 0;         // FP32 kernels: blocks launched (0: one per unit); block b
                           // runs units b, b+grid, ... of the nscen*items units
+    int block = 0;        // FP64 kernels: threads per block
 };
 
 enum class Mode : int { Fused = 0, Forward = 1, Backward = 2 };
@@ -106,9 +107,10 @@ cudaError_t launch_wpp_any(const DevModel &m, Mode mode, const float *z, uint64_
                            int64_t path0, bool philox, const Work &w, float *tape,
                            const double *vbar, cudaStream_t s);
 
-// FP64 kernels: thread per path, runtime shape.
+// FP64 kernels: thread per path, runtime shape, blocks of 32 to
+// f64_block_threads() threads (Work::block).
 int f64_block_threads();
-cudaError_t f64_blocks_per_sm(bool bump, int *blocks);
+cudaError_t f64_blocks_per_sm(int block, int nn, int nmat, int nopt, bool bump, int *blocks);
 cudaError_t launch_f64_greeks(const DevModel &m, const double *z, const Work &w, cudaStream_t s);
 // Bumped forward re-runs: 1 + 2nn variants per scenario (1 + 4nn with
 // `central`: each input bumped by +h and by -h); the launch's virtual
