@@ -188,9 +188,11 @@ LMM_HD uint64_t fx_recip(uint64_t D)
 #endif
     const uint32_t r0 = bits << 9;                                   // Q0.32
     const uint64_t phi = (uint64_t)dh * r0 + (((uint64_t)dl * r0) >> 32);
-    const uint64_t e = (1ull << 62) - phi;                           // Q2.62, below 2^42
+    // e = 2^62 - 1 - phi, Q2.62, below 2^42, as the complement: nvcc 13.0.88
+    // drops a carry in 2^63 - phi + x where the low word of phi is 0.
+    const uint64_t e = phi ^ ((1ull << 62) - 1);
     const uint32_t es = (uint32_t)(e >> 15);
-    const uint64_t g2 = e + (1ull << 62) + fx_mulhi32(es, es);       // 1 + e + e^2
+    const uint64_t g2 = (e | (1ull << 62)) + fx_mulhi32(es, es);     // 1 + e + e^2
     return (uint64_t)r0 * (uint32_t)(g2 >> 32) + (((uint64_t)r0 * (uint32_t)g2) >> 32);
 }
 

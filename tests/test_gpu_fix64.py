@@ -58,6 +58,18 @@ def test_paths_outside_the_range_beside_others():
     assert np.array_equal(again[0], alone)
 
 
+def test_rates_at_powers_of_two():
+    """delta L0 = 2^-6 puts zero low words through every integer sum of the first
+    steps. The oracle's and the kernel's sums over 4,096 paths each round to a
+    few units in 2^53."""
+    cfg = _cfg(24, 11, 4096, L0=(0.0625, 0.0625))
+    z = O.normals_f64(8, cfg.paths, cfg.nmat)
+    with pkg().Engine(cfg) as e:
+        g, _ = e.greeks_f64(z)
+    m, _ = O.greeks(cfg, z)
+    np.testing.assert_allclose(g[0], m, rtol=2e-14, atol=2e-14 * np.abs(m).max())
+
+
 @pytest.mark.parametrize("nn,nmat,central", [(12, 5, False), (9, 4, True)])
 def test_bump_values_match_oracle(nn, nmat, central):
     """Each difference against the oracle's values at the bumped inputs: V is
