@@ -5,46 +5,92 @@
 namespace lmm {
 namespace {
 
-constexpr int kFinX = 32, kFinY = 8;
+constexpr int kFinThreads = 256, kFinU = 4;
 
-// Block b covers scenario b / nchunk and outputs (b % nchunk)*32 .. +31;
-// thread (x = output, y = item group): group y adds items y, y+8, ... in
-// order, then group 0 adds the 8 group sums in order.
-__global__ void __launch_bounds__(kFinX *kFinY)
+// Ordered sums of the items' rows. Block b covers scenario b / nchunk and X
+// outputs; thread (x = output, y = item group of Y = 256 / X) adds items y,
+// y+Y, ... in kFinU interleaved sums, then a warp (or one thread, of few
+// groups) adds an output over the groups as a tree: the rounding of these last additions is in every mean
+// (that of the ones before averages out over the groups), and a bump's
+// difference of two means divides it by h, so it is kept below a unit in the
+// last place. What bounds it is the FP64 pipe (2 lanes a clock and SM), so a
+// call with many items spreads over the SMs: X = 4 outputs (one 32-byte
+// sector) a block beyond 64 items, X = 32 for the many scenarios with few
+// items. *flag becomes `stamp` if a result is not finite.
+template <int X>
+__global__ void __launch_bounds__(kFinThreads)
 k_finalize(const double *__restrict__ partial, int items, int nout, int64_t paths,
-           double *__restrict__ mean, double *__restrict__ se, int *__restrict__ flag)
+           double *__restrict__ mean, double *__restrict__ se, int *__restrict__ flag, int stamp)
 {
-    __shared__ double s1[kFinY][kFinX], s2[kFinY][kFinX];
-    const int nchunk = (nout + kFinX - 1) / kFinX;
-    const int scen = blockIdx.x / nchunk;
-    const int o = (blockIdx.x % nchunk) * kFinX + threadIdx.x;
-    double a = 0.0, b = 0.0;
+    constexpr int Y = kFinThreads / X;
+    __shared__ double s1[X][Y + 1], s2[X][Y + 1];
+    const int nchunk = (nout + X - 1) / X;
+    const int scen = blockIdx.x / nchunk, o0 = (blockIdx.x % nchunk) * X;
+    const int x = threadIdx.x % X, y = threadIdx.x / X, o = o0 + x;
+    double a[kFinU] = {}, b[kFinU] = {};
     if (o < nout) {
-        for (int it = threadIdx.y; it < items; it += kFinY) {
-            const double *p = partial + ((size_t)scen * items + it) * 2 * nout;
-            a += p[o];
-            b += p[nout + o];
+        const double *p0 = partial + (size_t)scen * items * 2 * nout + o;
+        int it = y;
+        for (; it + (kFinU - 1) * Y < items; it += kFinU * Y) {
+#pragma unroll
+            for (int u = 0; u < kFinU; ++u) {
+                const double *p = p0 + (size_t)(it + u * Y) * 2 * nout;
+                a[u] += p[0];
+                b[u] += p[nout];
+            }
+        }
+        for (; it < items; it += Y) {
+            const double *p = p0 + (size_t)it * 2 * nout;
+            a[0] += p[0];
+            b[0] += p[nout];
         }
     }
-    s1[threadIdx.y][threadIdx.x] = a;
-    s2[threadIdx.y][threadIdx.x] = b;
+    s1[x][y] = (a[0] + a[1]) + (a[2] + a[3]);
+    s2[x][y] = (b[0] + b[1]) + (b[2] + b[3]);
     __syncthreads();
-    if (threadIdx.y == 0 && o < nout) {
-        double sa = 0.0, sb = 0.0;
-#pragma unroll
-        for (int g = 0; g < kFinY; ++g) {
-            sa += s1[g][threadIdx.x];
-            sb += s2[g][threadIdx.x];
-        }
+    auto put = [&](int c, double sa, double sb) {
         const double n = (double)paths;
         const double mu = sa / n;
         double var = paths > 1 ? (sb - sa * mu) / (n - 1.0) : 0.0;
         var = var > 0.0 ? var : 0.0;
         const double e = sqrt(var / n);
-        mean[(size_t)scen * nout + o] = mu;
-        if (se) se[(size_t)scen * nout + o] = e;
-        if (!isfinite(mu) || !isfinite(e)) atomicOr(flag, 1);
+        mean[(size_t)scen * nout + o0 + c] = mu;
+        if (se) se[(size_t)scen * nout + o0 + c] = e;
+        if (!isfinite(mu) || !isfinite(e)) *flag = stamp;
+    };
+    if constexpr (Y >= 32) {
+        const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+        if (c < X) {
+            double sa = s1[c][lane], sb = s2[c][lane];
+#pragma unroll
+            for (int g = 32; g < Y; g += 32) {
+                sa += s1[c][lane + g];
+                sb += s2[c][lane + g];
+            }
+            sa = warp_sum(sa);
+            sb = warp_sum(sb);
+            if (lane == 0 && o0 + c < nout) put(c, sa, sb);
+        }
+    } else if (y == 0 && o < nout) {
+#pragma unroll
+        for (int h = Y / 2; h > 0; h /= 2)
+#pragma unroll
+            for (int g = 0; g < h; ++g) {
+                s1[x][g] += s1[x][g + h];
+                s2[x][g] += s2[x][g + h];
+            }
+        put(x, s1[x][0], s2[x][0]);
     }
+}
+
+template <int X>
+cudaError_t finalize(const double *partial, int nscen, int items, int nout, int64_t paths, double *mean, double *se,
+                     int *flag, int stamp, cudaStream_t s)
+{
+    const int64_t blocks = (int64_t)nscen * ((nout + X - 1) / X);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    k_finalize<X><<<(unsigned)blocks, kFinThreads, 0, s>>>(partial, items, nout, paths, mean, se, flag, stamp);
+    return cudaGetLastError();
 }
 
 __global__ void k_bump_diff(double *mean, double *se, int nscen, int nout, double h)
@@ -198,13 +244,10 @@ unsigned grid_for(int64_t work, int block)
 }  // namespace
 
 cudaError_t launch_finalize(const double *partial, int nscen, int items, int nout, int64_t paths,
-                            double *mean, double *se, int *flag, cudaStream_t s)
+                            double *mean, double *se, int *flag, int stamp, cudaStream_t s)
 {
-    const int64_t blocks = (int64_t)nscen * ((nout + kFinX - 1) / kFinX);
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    dim3 block(kFinX, kFinY);
-    k_finalize<<<(unsigned)blocks, block, 0, s>>>(partial, items, nout, paths, mean, se, flag);
-    return cudaGetLastError();
+    return items > 64 ? finalize<4>(partial, nscen, items, nout, paths, mean, se, flag, stamp, s)
+                      : finalize<32>(partial, nscen, items, nout, paths, mean, se, flag, stamp, s);
 }
 
 cudaError_t launch_bump_central(const double *mean, const double *se_in, double *out, double *se, int nscen,

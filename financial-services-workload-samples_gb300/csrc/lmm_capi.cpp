@@ -112,6 +112,7 @@ struct lmm_engine {
     float *wf_rows = nullptr;      // [1+nopt][nopt] weights: row 0 the caller's, row 1+g unit at g
     double *wd_rows = nullptr;
     DevBuf partial, z32, z64, out, se, flag, vbar;
+    int stamp = 0;                 // of the last call: what *flag becomes on a non-finite result
     DevBuf wscratch;               // warp-per-path kernels: Y_top per warp, step and lane
     DevBuf bumpvar;                // central bumps: the variants' means and standard errors
     std::vector<float4> kc_host;   // the per-maturity constants, host copy
@@ -340,6 +341,18 @@ int plan_f64(lmm_engine *e, int64_t nvs, int64_t paths, bool bump, int nout, Wor
     return LMM_OK;
 }
 
+// A call's own stamp in the non-finite flag: nothing has to clear the flag
+// between calls (a memset on the stream took 2 us of a small call).
+int next_stamp(lmm_engine *e)
+{
+    if (!e->flag.p) {
+        LMM_TRY(e->flag.ensure(sizeof(int)));
+        LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
+    }
+    e->stamp = e->stamp == INT32_MAX ? 1 : e->stamp + 1;
+    return LMM_OK;
+}
+
 int check_paths(int64_t paths)
 {
     if (paths < 1) return fail(LMM_ERR_INVALID_ARG, "paths must be >= 1");
@@ -413,14 +426,13 @@ int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t p
     if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &tape));
     if (fam == 6) LMM_TRY(tps_scratch(e, w.grid, &tape));
     if (fam == 7) LMM_TRY(tpq_scratch(e, w.grid, &tape));
-    LMM_TRY(e->flag.ensure(sizeof(int)));
-    LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
+    LMM_TRY(next_stamp(e));
     mark(e, 0);
     cudaError_t err = launch_f32_family(fam, e->dm, mode, d_z, seed, path0, philox, w, tape, d_vbar, e->stream);
     if (err != cudaSuccess) return cuda_fail(err, "FP32 LMM kernel launch");
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(w.partial, e->nscen, w.items, nout, paths, d_mean, d_se,
-                                e->flag.as<int>(), e->stream));
+                                e->flag.as<int>(), e->stamp, e->stream));
     mark(e, 2);
     e->last_launches = 2;
     return LMM_OK;
@@ -435,7 +447,7 @@ int fetch(lmm_engine *e, int nout, double *out, double *se)
     if (se) LMM_CK(cudaMemcpyAsync(se, e->se.p, sizeof(double) * n, cudaMemcpyDeviceToHost, e->stream));
     LMM_CK(cudaMemcpyAsync(&flag, e->flag.p, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     LMM_CK(cudaStreamSynchronize(e->stream));
-    if (flag) return fail(LMM_ERR_NONFINITE, "a result is NaN or Inf");
+    if (flag == e->stamp) return fail(LMM_ERR_NONFINITE, "a result is NaN or Inf");
     return LMM_OK;
 }
 
@@ -455,13 +467,12 @@ int run_f64(lmm_engine *e, const double *d_z, int64_t paths, double *d_mean, dou
     const int nout = 1 + 2 * e->nn;
     Work w{};
     LMM_TRY(plan_f64(e, e->nscen, paths, false, nout, &w));
-    LMM_TRY(e->flag.ensure(sizeof(int)));
-    LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
+    LMM_TRY(next_stamp(e));
     mark(e, 0);
     LMM_CK(lmm::launch_f64_greeks(e->dm, d_z, w, e->stream));
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(w.partial, e->nscen, w.items, nout, paths, d_mean, d_se,
-                                e->flag.as<int>(), e->stream));
+                                e->flag.as<int>(), e->stamp, e->stream));
     mark(e, 2);
     e->last_launches = 2;
     return LMM_OK;
@@ -477,7 +488,7 @@ int run_bump(lmm_engine *e, const double *d_z, int64_t paths, double h, bool cen
     const int nb = central ? 1 + 4 * e->nn : 1 + 2 * e->nn;
     Work w{};
     LMM_TRY(plan_f64(e, (int64_t)e->nscen * nb, paths, true, 1, &w));
-    LMM_TRY(e->flag.ensure(sizeof(int)));
+    LMM_TRY(next_stamp(e));
     // central: the 1+4nn variant means (and their standard errors) go to the
     // engine's scratch and are differenced into the caller's 1+2nn outputs
     double *vmean = d_mean, *vse = d_se;
@@ -486,12 +497,11 @@ int run_bump(lmm_engine *e, const double *d_z, int64_t paths, double h, bool cen
         vmean = e->bumpvar.as<double>();
         vse = vmean + (size_t)e->nscen * nb;
     }
-    LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
     mark(e, 0);
     LMM_CK(lmm::launch_f64_bump(e->dm, d_z, h, central, w, e->stream));
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(w.partial, e->nscen * nb, w.items, 1, paths, vmean, vse,
-                                e->flag.as<int>(), e->stream));
+                                e->flag.as<int>(), e->stamp, e->stream));
     if (central)
         LMM_CK(lmm::launch_bump_central(vmean, vse, d_mean, d_se, e->nscen, e->nn, h, e->stream));
     else
@@ -1003,7 +1013,7 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
                          : fam == 5 ? tp2_scratch(e, most, &wscr)
                                     : fam == 6 ? tps_scratch(e, most, &wscr) : tpq_scratch(e, most, &wscr));
     }
-    LMM_TRY(e->flag.ensure(sizeof(int)));
+    LMM_TRY(next_stamp(e));
     if (!e->copy_stream) LMM_CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
     if (!e->ready_ev) LMM_CK(cudaEventCreateWithFlags(&e->ready_ev, cudaEventDisableTiming));
     for (int c = 0; c < C; ++c)
@@ -1017,7 +1027,6 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
         LMM_CK(cudaMemcpyAsync(dz + off, z + off, sizeof(float) * n, cudaMemcpyHostToDevice, e->copy_stream));
         LMM_CK(cudaEventRecord(e->copy_ev[c], e->copy_stream));
     }
-    LMM_CK(cudaMemsetAsync(e->flag.p, 0, sizeof(int), e->stream));
     mark(e, 0);
     double *part = e->partial.as<double>();
     for (int c = 0; c < C; ++c) {
@@ -1036,7 +1045,7 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
     }
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(e->partial.as<double>(), 1, (int)total_items, nout, paths,
-                                e->out.as<double>(), e->se.as<double>(), e->flag.as<int>(), e->stream));
+                                e->out.as<double>(), e->se.as<double>(), e->flag.as<int>(), e->stamp, e->stream));
     mark(e, 2);
     e->last_launches = C + 1;
     return LMM_OK;

@@ -120,9 +120,9 @@ cudaError_t launch_f64_bump(const DevModel &m, const double *z, double h, bool c
                             cudaStream_t s);
 
 // Sums the per-item partials of each scenario in a fixed order and writes
-// mean and standard error; sets *flag if a result is not finite.
+// mean and standard error; *flag becomes `stamp` if a result is not finite.
 cudaError_t launch_finalize(const double *partial, int nscen, int items, int nout, int64_t paths,
-                            double *mean, double *se, int *flag, cudaStream_t s);
+                            double *mean, double *se, int *flag, int stamp, cudaStream_t s);
 // Turns bumped means into one-sided differences in place: out[j] =
 // (out[j]-out[0])/h for j >= 1, per scenario.
 cudaError_t launch_bump_diff(double *mean, double *se, int nscen, int nout, double h,

@@ -243,7 +243,7 @@ extern "C" int lmm_greeks_f32_device_noalloc(const lmm_params *p, const float *d
 
     ce = lmm::launch_tpp_any(m, lmm::Mode::Fused, d_z, 0, 0, false, w, nullptr, nullptr, st);
     if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "FP32 LMM kernel launch");
-    ce = lmm::launch_finalize(partial, p->nscen, w.items, kNout, paths, d_out, d_se, flag, st);
+    ce = lmm::launch_finalize(partial, p->nscen, w.items, kNout, paths, d_out, d_se, flag, 1, st);
     if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "finalize launch");
     return LMM_OK;
 }
