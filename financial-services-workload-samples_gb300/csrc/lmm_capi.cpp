@@ -223,6 +223,26 @@ int batch_paths(const lmm_engine *e, int fam, Mode mode)
     return lmm::wpp_block_threads() / 32;
 }
 
+// Paths that share a warp (warp-per-path kernels: the block's paths).
+int batch_gran(int fam) { return fam == 2 ? lmm::wpp_block_threads() / 32 : 32; }
+
+// Kernels whose batches may be ragged (run by the warps that have paths):
+// k_tps as a variant of its own, the 80/40 forward-only kernel, warp per path.
+// The others run whole batches of the block.
+bool ragged_batches(int fam, Mode mode) { return fam == 2 || fam == 6 || (fam == 1 && mode == Mode::Forward); }
+
+// Time of a ragged batch of n paths relative to a full one. GB300, one batch
+// per SM, one / two / three warps per scheduler: k_tps 0.113, 0.125, 0.156 ms
+// (0.150 in its whole-batch variant), the forward of the 80/40 pair 0.037,
+// 0.048, 0.059.
+double batch_cost(int fam, int n)
+{
+    const int wps = (n + 127) / 128;
+    if (fam == 6) return wps == 1 ? 0.75 : wps == 2 ? 0.84 : 1.04;
+    if (fam == 1) return wps == 1 ? 0.63 : wps == 2 ? 0.82 : 1.0;
+    return 1.0;
+}
+
 cudaError_t launch_f32_family(int fam, const lmm::DevModel &m, Mode mode, const float *z, uint64_t seed,
                               int64_t path0, bool philox, const Work &w, float *tape, const double *vbar,
                               cudaStream_t s)
@@ -257,13 +277,30 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
     return LMM_OK;
 }
 
-// Items per virtual scenario (and paths per thread) of a launch. Each block
-// runs ppt batches of paths, all blocks equally long, so a launch costs
+// The family of a call of `paths` paths: the warp-per-path kernels for few
+// paths, family_for above. A thread-per-path kernel takes one path's latency
+// (80/40 fused 0.113 ms, 160/120 0.47 ms) for anything from one path to a
+// device full of single warps; a warp per path takes 0.04 ms (0.096) for one
+// path and its throughput beyond the device's resident warps (3,648 on GB300):
+// 80/40 fused, kernel alone, 3,001 / 4,864 / 9,728 paths 0.055 / 0.086 / 0.152
+// against 0.113 ms, 160/120 0.15 / 0.25 / 0.48 against 0.47-0.48 ms. The line
+// is two fills of the device, for every mode alike: the fused call and the
+// forward/backward pair of the same size must round alike.
+int family_at(lmm_engine *e, Mode mode, int64_t paths, int *fam)
+{
+    *fam = family_for(e, mode);
+    if (*fam == 0 || *fam == 2 || !lmm::f32_wpp_supports(e->nn, e->nmat)) return LMM_OK;
+    int bps = 0;
+    LMM_TRY(blocks_per_sm(e, 2, Mode::Fused, false, &bps));
+    if (paths <= 2 * (int64_t)e->sms * bps * batch_paths(e, 2, Mode::Fused) / e->nscen) *fam = 2;
+    return LMM_OK;
+}
+
+// Items per virtual scenario and batches per item (ppt) of an FP64 launch.
+// Each block runs ppt batches, all blocks equally long, so a launch costs
 // ceil(blocks / slots) block-times, slots = SMs x resident blocks per SM.
 // The plan takes the fewest waves (1..8) whose blocks fill at least 97% of
-// the slots they occupy: one wave for one scenario (every block starts at
-// once, no staggered tail), three waves for 256 scenarios (256 x 7 blocks
-// of 608 slots) where one wave would leave a quarter-full second wave.
+// the slots they occupy.
 void plan_items(const lmm_engine *e, int64_t nvs, int64_t paths, int block, int bps, int64_t *items,
                 int64_t *ppt)
 {
@@ -284,18 +321,79 @@ void plan_items(const lmm_engine *e, int64_t nvs, int64_t paths, int block, int 
     }
 }
 
-// plan_items, and sizes the partial-sum scratch.
-int plan(lmm_engine *e, int64_t nvs, int64_t paths, int block, int bps, int nout, Work *w)
+// Path ranges of an FP32 launch: units of one scenario's paths, run in whole
+// batches of the block, or (ragged_batches) in batches of whole warps and a last
+// partial one; one wave of blocks loops over the units, so a launch takes
+// ceil(units / blocks) times the longest unit. A ragged batch's time goes with
+// the warps on the busiest of an SM's four schedulers (batch_cost), hardly with
+// its paths. The plan is the cheapest split: 20,000 paths take every SM with
+// five warps (0.125 ms) where whole batches took 53 SMs with twelve (0.150),
+// and 131,072 paths two full batches and one of three warps on each of 147 SMs
+// where they took three full ones on 114 (0.440 -> 0.423 ms a call).
+struct PathPlan {
+    int64_t items = 1, ipaths = 1;
+    int bpaths = 1;
+    int ppt = 0;      // whole batches of the block per item (0: ragged ones)
+    void put(Work *w) const
+    {
+        w->items = (int)items;
+        w->ipaths = ipaths;
+        w->bpaths = bpaths;
+        w->ppt = ppt;
+    }
+};
+PathPlan plan_paths(const lmm_engine *e, int fam, Mode mode, int64_t nvs, int64_t paths, int bps)
 {
-    int64_t items = 1, ppt = 1;
-    plan_items(e, nvs, paths, block, bps, &items, &ppt);
-    if (ppt > INT32_MAX || items > INT32_MAX || nvs * items > INT32_MAX)
-        return fail(LMM_ERR_TOO_LARGE, "launch too large");
+    const int batch = batch_paths(e, fam, mode), gran = batch_gran(fam);
+    const int64_t cap = std::max<int64_t>(1, (int64_t)e->sms * bps);
+    const bool ragged = ragged_batches(fam, mode), whole = !ragged || fam == 6;
+    const double unit = 0.015;     // a unit's own cost: accumulators cleared and written out
+    PathPlan best;
+    double best_cost = 1e300;
+    auto take = [&](double cost, const PathPlan &p) {
+        if (cost >= best_cost * (1.0 - 1e-9)) return;
+        best_cost = cost;
+        best = p;
+    };
+    // Several scenarios: short units too, which end within a few batches of each
+    // other (256 curves of 43 batches on 152 SMs: 7 units of 11 batches on the
+    // busiest SM, or 73 of one; GB300 10.47 -> 10.07 ms).
+    if (whole && nvs > 1)
+        for (int64_t ppt = 1; ppt <= 64; ++ppt) {
+            const int64_t n = (paths + ppt * batch - 1) / (ppt * batch);
+            if (nvs * n <= 16384)
+                take((double)((nvs * n + cap - 1) / cap) * ((double)ppt + unit), PathPlan{n, ppt * batch, batch, (int)ppt});
+        }
+    // units per scenario: what fills 1 .. 16 waves of blocks
+    for (int w = 1; w <= 16; ++w) {
+        const int64_t it = std::min(std::max<int64_t>(1, w * cap / nvs), (paths + gran - 1) / gran);
+        const int64_t per = ((paths + it - 1) / it + gran - 1) / gran * gran;
+        auto waves = [&](int64_t n) { return (double)((nvs * n + cap - 1) / cap); };
+        if (whole) {
+            const int64_t ppt = (per + batch - 1) / batch, n = (paths + ppt * batch - 1) / (ppt * batch);
+            if (ppt <= INT32_MAX) take(waves(n) * ((double)ppt + unit), PathPlan{n, ppt * batch, batch, (int)ppt});
+        }
+        for (int bp = (int)std::min<int64_t>(batch, per); ragged; bp -= 128) {
+            const int64_t n = (paths + per - 1) / per;
+            take(waves(n) * ((double)(per / bp) * batch_cost(fam, bp) +
+                             (per % bp ? batch_cost(fam, (int)(per % bp)) : 0.0) + unit),
+                 PathPlan{n, per, bp, 0});
+            if (bp <= 128) break;
+        }
+    }
+    return best;
+}
+
+// plan_paths, and sizes the partial-sum scratch.
+int plan(lmm_engine *e, int fam, Mode mode, int64_t nvs, int64_t paths, int bps, int nout, Work *w)
+{
+    const PathPlan p = plan_paths(e, fam, mode, nvs, paths, bps);
+    const int64_t items = p.items;
+    if (items > INT32_MAX || nvs * items > INT32_MAX) return fail(LMM_ERR_TOO_LARGE, "launch too large");
     w->paths = paths;
-    w->items = (int)items;
-    w->ppt = (int)ppt;
+    p.put(w);
     w->nout = nout;
-    // FP32 kernels: one wave of blocks, each looping over its units
+    // one wave of blocks, each looping over its units
     w->grid = (int)std::min<int64_t>(nvs * items, std::max<int64_t>(1, (int64_t)e->sms * bps));
     LMM_TRY(e->partial.ensure(sizeof(double) * (size_t)(nvs * items) * 2 * nout));
     w->partial = e->partial.as<double>();
@@ -409,19 +507,19 @@ int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t p
     if (!philox && !d_z) return fail(LMM_ERR_INVALID_ARG, "normals pointer is NULL");
     if (!d_mean) return fail(LMM_ERR_INVALID_ARG, "output pointer is NULL");
     if (philox && (path0 < 0 || path0 > kMaxPaths)) return fail(LMM_ERR_INVALID_ARG, "path0 out of range");
-    const int fam = family_for(e, mode);
+    LMM_TRY(set_device(e));
+    int fam = 0;
+    LMM_TRY(family_at(e, mode, paths, &fam));
     if (fam == 0)
         return fail(LMM_ERR_UNSUPPORTED, "no FP32 kernel for nn=" + std::to_string(e->nn) +
                                              ", nmat=" + std::to_string(e->nmat));
     if (philox && mode != Mode::Fused)
         return fail(LMM_ERR_UNSUPPORTED, "the forward/backward pair reads its normals from memory");
-    LMM_TRY(set_device(e));
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, fam, mode, philox, &bps));
     const int nout = mode == Mode::Fused ? 1 + 2 * e->nn : (mode == Mode::Forward ? 1 : 2 * e->nn);
-    const int per_batch = batch_paths(e, fam, mode);
     Work w{};
-    LMM_TRY(plan(e, e->nscen, paths, per_batch, bps, nout, &w));
+    LMM_TRY(plan(e, fam, mode, e->nscen, paths, bps, nout, &w));
     if (fam == 2) LMM_TRY(wpp_scratch(e, w.grid, &tape));
     if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &tape));
     if (fam == 6) LMM_TRY(tps_scratch(e, w.grid, &tape));
@@ -969,13 +1067,15 @@ constexpr int64_t kPipelineMinPaths = int64_t(1) << 18;
 
 int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
 {
-    const int fam = family_for(e, Mode::Fused);
+    int fam = 0;
+    LMM_TRY(family_at(e, Mode::Fused, paths, &fam));
     if (fam == 0) return fail(LMM_ERR_UNSUPPORTED, "no FP32 kernel for this shape");
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, fam, Mode::Fused, false, &bps));
     const int per_batch = batch_paths(e, fam, Mode::Fused);
     const int nout = 1 + 2 * e->nn;
-    int64_t cpaths[kHostChunks], cfirst[kHostChunks], citems[kHostChunks], cppt[kHostChunks];
+    int64_t cpaths[kHostChunks], cfirst[kHostChunks];
+    PathPlan cplan[kHostChunks];
     int64_t total_items = 0, wsum = 0, wcum = 0;
     for (int c = 0; c < kHostChunks; ++c) wsum += kHostSplit[c];
     // Piece boundaries on whole waves of the device (SMs x resident blocks x
@@ -999,15 +1099,15 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
         ++C;
     }
     for (int c = 0; c < C; ++c) {
-        plan_items(e, 1, cpaths[c], per_batch, bps, &citems[c], &cppt[c]);
-        if (cppt[c] > INT32_MAX || citems[c] > INT32_MAX) return fail(LMM_ERR_TOO_LARGE, "launch too large");
-        total_items += citems[c];
+        cplan[c] = plan_paths(e, fam, Mode::Fused, 1, cpaths[c], bps);
+        if (cplan[c].items > INT32_MAX) return fail(LMM_ERR_TOO_LARGE, "launch too large");
+        total_items += cplan[c].items;
     }
     LMM_TRY(e->partial.ensure(sizeof(double) * (size_t)total_items * 2 * nout));
     float *wscr = nullptr;
     if (fam == 2 || fam == 5 || fam == 6 || fam == 7) {
         int64_t most = 0;
-        for (int c = 0; c < C; ++c) most = std::max(most, std::min<int64_t>(citems[c], (int64_t)e->sms * bps));
+        for (int c = 0; c < C; ++c) most = std::max(most, std::min<int64_t>(cplan[c].items, (int64_t)e->sms * bps));
         // the pieces run one after another
         LMM_TRY(fam == 2 ? wpp_scratch(e, most, &wscr)
                          : fam == 5 ? tp2_scratch(e, most, &wscr)
@@ -1033,15 +1133,14 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
         LMM_CK(cudaStreamWaitEvent(e->stream, e->copy_ev[c], 0));
         Work w{};
         w.paths = cpaths[c];
-        w.items = (int)citems[c];
-        w.ppt = (int)cppt[c];
+        cplan[c].put(&w);
         w.nout = nout;
-        w.grid = (int)std::min<int64_t>(citems[c], (int64_t)e->sms * bps);
+        w.grid = (int)std::min<int64_t>(cplan[c].items, (int64_t)e->sms * bps);
         w.partial = part;
         const float *zc = dz + (size_t)cfirst[c] * e->nmat;
         cudaError_t err = launch_f32_family(fam, e->dm, Mode::Fused, zc, 0, 0, false, w, wscr, nullptr, e->stream);
         if (err != cudaSuccess) return cuda_fail(err, "FP32 LMM kernel launch");
-        part += (size_t)citems[c] * 2 * nout;
+        part += (size_t)cplan[c].items * 2 * nout;
     }
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(e->partial.as<double>(), 1, (int)total_items, nout, paths,
@@ -1103,7 +1202,8 @@ int lmm_tape_create(lmm_engine *e, int64_t paths, lmm_tape **out)
     // kernels keep the terminal rates and the per-step drift sums; the
     // warp-per-path backward recomputes its forward from the same normals and
     // needs no tape.
-    const int fam = family_for(e, Mode::Forward);
+    int fam = 0;
+    LMM_TRY(family_at(e, Mode::Forward, paths, &fam));
     if (fam == 1 || fam == 5) {
         // thread pair: also the drift sums at the half boundary
         const size_t rows = (size_t)e->nn + (size_t)e->nmat * (fam == 5 ? 2 : 1);

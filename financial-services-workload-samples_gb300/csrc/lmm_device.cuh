@@ -118,6 +118,10 @@ __device__ __forceinline__ void box_muller_f64(uint32_t a, uint32_t b, double &z
     z1 = r * s;
 }
 
+// Barrier of the block's first n threads (n a multiple of 32), for the step
+// loops of batches that do not fill the block.
+__device__ __forceinline__ void sync_threads(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v)
 {
 #pragma unroll

@@ -195,6 +195,20 @@ struct TppLayout {
     static constexpr int bytes = acc + 8 * NW * 2 * NOUT;
 };
 
+// Paths of batch jb of an item (0 or less: there is none).
+__device__ __forceinline__ int batch_left(const Work &w, int item, int jb)
+{
+    const int64_t p0 = (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths;
+    const int64_t iend = min((int64_t)(item + 1) * w.ipaths, w.paths);
+    return (int)max(min(iend - p0, (int64_t)w.bpaths), (int64_t)0);
+}
+
+// A batch's paths, kept per warp in shared memory (batch_left): the step loops
+// have no register to spare for it. The batch runs in the first threads of the
+// block, whole warps.
+__device__ __forceinline__ int read_left(const int *left) { return *reinterpret_cast<const volatile int *>(left); }
+__device__ __forceinline__ void sync_batch(const int *left) { sync_threads((read_left(left) + 31) & ~31); }
+
 __device__ __forceinline__ float pick4(const float4 &q, int j)
 {
     float r = q.x;
@@ -711,6 +725,8 @@ k_tpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     double *acc_s = reinterpret_cast<double *>(smem + Lay::acc);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // The forward-only kernel has no barrier in its steps: its batches run in the warps that have paths.
+    constexpr bool RAGGED = MODE == Mode::Forward;
     constexpr bool kKcParam = LMM_TPP_KCPARAM && MODE == Mode::Fused;
     if (!kKcParam) {
         for (int i = tid; i < PAD + NN; i += B) {
@@ -746,13 +762,14 @@ k_tpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
         for (int i = tid; i < Lay::NW * 2 * NOUT; i += B) acc_s[i] = 0.0;
         __syncthreads();
 
-        const int64_t ibase = (int64_t)item * w.ppt * B;
         const float vb = MODE == Mode::Backward ? (float)vbar[scen] : 1.0f;
-        for (int j = 0; j < w.ppt; ++j) {
-            if (ibase + (int64_t)j * B >= w.paths) break;          // block-uniform
-            const int64_t pl = ibase + (int64_t)j * B + tid;
-            const bool active = pl < w.paths;
-            const int64_t pc = active ? pl : w.paths - 1;
+        for (int jb = 0; RAGGED || jb < w.ppt; ++jb) {
+            const int64_t p0 = RAGGED ? (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths
+                                      : ((int64_t)item * w.ppt + jb) * B;
+            const int left = RAGGED ? batch_left(w, item, jb) : 0;
+            if (RAGGED ? (tid & ~31) >= left : p0 >= w.paths) break;      // whole warps, later batches no larger; the block
+            const bool active = RAGGED ? tid < left : p0 + tid < w.paths;
+            const int64_t pc = active ? p0 + tid : w.paths - 1;
             const int64_t tp = (int64_t)scen * w.paths + pc;
             const float *zp = PHILOX ? nullptr : z + pc * NMAT;
             const uint64_t gpath = (uint64_t)(path0 + pc);
@@ -993,7 +1010,21 @@ __device__ __forceinline__ void rev_half_window(float (&X)[H], float (&Pb)[H], R
     }
 }
 
-template <int NN, int NMAT, bool PHILOX>
+template <bool RAGGED>
+__device__ __forceinline__ void tps_sync(const int *left)
+{
+    if (RAGGED)
+        sync_batch(left);
+    else
+        __syncthreads();
+}
+
+// RAGGED: batches of w.bpaths paths and a last partial one per item, each run
+// by the warps that have paths. Otherwise whole batches of the block (w.ppt per
+// item), in which every warp runs: the ragged batches' bookkeeping costs 40
+// more bytes of spills and 4% of a full batch's time (curves 10.48 -> 10.94 ms),
+// so the plan takes it only where it saves more.
+template <int NN, int NMAT, bool PHILOX, bool RAGGED>
 __global__ void __launch_bounds__(LMM_TPS_BLOCK, 384 / LMM_TPS_BLOCK)
 k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w,
       float *__restrict__ scr, const __grid_constant__ TppConst<NN, NMAT> kp)
@@ -1015,6 +1046,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     double *acc_s = reinterpret_cast<double *>(smem + Lay::acc);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ int left_s[Lay::NW];
     for (int i = tid; i <= M; i += B) ost_s[i] = m.opt_start[i];
     for (int i = tid; i < m.nopt; i += B) {
         okf_s[i] = m.optKf[i];
@@ -1040,12 +1072,21 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
         for (int i = tid; i < Lay::NW * 2 * NOUT; i += B) acc_s[i] = 0.0;
         __syncthreads();
 
-        const int64_t ibase = (int64_t)item * w.ppt * B;
-        for (int jb = 0; jb < w.ppt; ++jb) {
-            if (ibase + (int64_t)jb * B >= w.paths) break;          // block-uniform
-            const int64_t pl = ibase + (int64_t)jb * B + tid;
-            const bool active = pl < w.paths;
-            const int64_t pc = active ? pl : w.paths - 1;
+        for (int jb = 0; RAGGED || jb < w.ppt; ++jb) {
+            int64_t pl;
+            if (RAGGED) {
+                const int left = batch_left(w, item, jb);
+                if ((tid & ~31) >= left) break;      // whole warps; later batches are no larger
+                if (lane == 0) left_s[warp] = left;
+                __syncwarp();
+                pl = tid < left ? (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths + tid : w.paths;
+            } else {
+                const int64_t p0 = ((int64_t)item * w.ppt + jb) * B;
+                if (p0 >= w.paths) break;            // block-uniform
+                pl = p0 + tid;
+            }
+            const bool act = pl < w.paths;
+            const int64_t pc = act ? pl : w.paths - 1;
             const float *zp = PHILOX ? nullptr : z + pc * NMAT;
             const uint64_t gpath = (uint64_t)(path0 + pc);
 
@@ -1060,7 +1101,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 float4 zq, zq_next = zquad<PHILOX, NMAT>(zp, seed, gpath, 0);
                 for (int n = 0; n < NMAT; n += 2) {
                     if (LMM_TPS_SYNC && (n % (2 * (PHILOX ? LMM_TPS_FSYNC_PHILOX : LMM_TPS_FSYNC))) == 0)
-                        __syncthreads();
+                        tps_sync<RAGGED>(left_s + warp);
                     if ((n & 3) == 0) {
                         zq = zq_next;
                         if ((n >> 2) + 1 < NMAT / 4) zq_next = zquad<PHILOX, NMAT>(zp, seed, gpath, (n >> 2) + 1);
@@ -1093,7 +1134,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 
             // ---- R1: the upper half's reverse, every step ----
             for (int n = NMAT - 1; n > 0; n -= G) {
-                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) __syncthreads();
+                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) tps_sync<RAGGED>(left_s + warp);
                 RevStep st[G];
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
@@ -1109,7 +1150,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 for (int g = 0; g < G; ++g) sc[(Lay::s_s + n - g) * B] = st[g].S;
             }
 #pragma unroll
-            for (int i = 0; i < H; ++i) sc[(Lay::s_d + i) * B] = active ? Pu[i] * il0_s[H + i] : 0.0f;
+            for (int i = 0; i < H; ++i) sc[(Lay::s_d + i) * B] = Pu[i] * il0_s[H + i];
 
             // ---- R2: the lower half's reverse ----
             float Xl[H], Pl[H];
@@ -1125,7 +1166,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 ns[g] = sc[(Lay::s_s + NMAT - 1 - g) * B];
             }
             for (int n = NMAT - 1; n > 0; n -= G) {
-                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) __syncthreads();
+                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) tps_sync<RAGGED>(left_s + warp);
                 RevStep st[G];
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
@@ -1147,6 +1188,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             }
 
             // ---- cross-path reduction of this batch of B paths ----
+            const bool active = RAGGED ? tid < read_left(left_s + warp) : act;
             {
                 const float v = active ? V : 0.0f;
                 const float s1 = warp_sum(v), s2 = warp_sum(v * v);
@@ -1166,7 +1208,7 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll
             for (int i = 0; i < H; ++i) {
                 vg0[i * B] = active ? Pl[i] * il0_s[i] : 0.0f;
-                vg0[(H + i) * B] = sc[(Lay::s_d + i) * B];
+                vg0[(H + i) * B] = active ? sc[(Lay::s_d + i) * B] : 0.0f;
             }
             __syncwarp();
             column_reduce<NN, B>(vgw, warp, lane, acc, NOUT, 1);
@@ -1183,12 +1225,12 @@ k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     }  // units
 }
 
-template <int NN, int NMAT, bool PHILOX>
+template <int NN, int NMAT, bool PHILOX, bool RAGGED>
 cudaError_t launch_tps(const DevModel &m, const float *z, uint64_t seed, int64_t path0, const Work &w,
                        float *scr, cudaStream_t s)
 {
     using Lay = TpsLayout<NN, NMAT>;
-    auto kern = k_tps<NN, NMAT, PHILOX>;
+    auto kern = k_tps<NN, NMAT, PHILOX, RAGGED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::bytes);
     if (e != cudaSuccess) return e;
     TppConst<NN, NMAT> kp;
@@ -1199,11 +1241,11 @@ cudaError_t launch_tps(const DevModel &m, const float *z, uint64_t seed, int64_t
     return cudaGetLastError();
 }
 
-template <int NN, int NMAT, bool PHILOX>
+template <int NN, int NMAT, bool PHILOX, bool RAGGED>
 cudaError_t occ_tps(int *blocks)
 {
     using Lay = TpsLayout<NN, NMAT>;
-    auto kern = k_tps<NN, NMAT, PHILOX>;
+    auto kern = k_tps<NN, NMAT, PHILOX, RAGGED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::bytes);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, Lay::B, Lay::bytes);
@@ -1774,14 +1816,17 @@ size_t tps_scratch_floats_per_block(int nn, int nmat) { return (size_t)(2 * nmat
 
 cudaError_t tps_blocks_per_sm(bool philox, int *blocks)
 {
-    return philox ? occ_tps<80, 40, true>(blocks) : occ_tps<80, 40, false>(blocks);
+    return philox ? occ_tps<80, 40, true, false>(blocks) : occ_tps<80, 40, false, false>(blocks);
 }
 
 cudaError_t launch_tps_any(const DevModel &m, const float *z, uint64_t seed, int64_t path0, bool philox,
                            const Work &w, float *scratch, cudaStream_t s)
 {
-    return philox ? launch_tps<80, 40, true>(m, z, seed, path0, w, scratch, s)
-                  : launch_tps<80, 40, false>(m, z, seed, path0, w, scratch, s);
+    if (w.ppt > 0)
+        return philox ? launch_tps<80, 40, true, false>(m, z, seed, path0, w, scratch, s)
+                      : launch_tps<80, 40, false, false>(m, z, seed, path0, w, scratch, s);
+    return philox ? launch_tps<80, 40, true, true>(m, z, seed, path0, w, scratch, s)
+                  : launch_tps<80, 40, false, true>(m, z, seed, path0, w, scratch, s);
 }
 
 int tpp_block_threads(Mode mode)

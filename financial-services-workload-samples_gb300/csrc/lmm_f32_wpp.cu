@@ -290,10 +290,8 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
         __syncthreads();
 
         const float vb = MODE == Mode::Backward ? (float)vbar[scen] : 1.0f;
-        const int64_t ibase = (int64_t)item * w.ppt * kWppWarps;
-        for (int j = 0; j < w.ppt; ++j) {
-            const int64_t p = ibase + (int64_t)j * kWppWarps + warp;
-            if (p >= w.paths) break;                                  // warp-uniform
+        const int64_t iend = min((int64_t)(item + 1) * w.ipaths, w.paths);
+        for (int64_t p = (int64_t)item * w.ipaths + warp; p < iend; p += kWppWarps) {  // warp-uniform
             const float *zp = PHILOX ? nullptr : z + p * nmat;
             const uint64_t gpath = (uint64_t)(path0 + p);
             ZChunk<PHILOX> zc;

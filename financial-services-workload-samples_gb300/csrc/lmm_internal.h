@@ -36,12 +36,15 @@ struct DevModel {
                                           // FP32 reverse sweeps restore (0: none)
 };
 
-// Path partition of one launch: grid = nscen * items blocks; block b takes
-// scenario b / items and the path range [item*ipaths, (item+1)*ipaths) of it.
+// Path partition of one launch: nscen * items units; unit u takes scenario
+// u / items and the path range [item*ipaths, (item+1)*ipaths) of it, item =
+// u % items, in batches of bpaths. FP64 kernels: ppt batches of a block each.
 struct Work {
     int64_t paths;        // per scenario
     int items;            // items per scenario
-    int ppt;              // paths per thread per item
+    int64_t ipaths = 0;   // FP32 kernels: paths per item
+    int bpaths = 0;       // FP32 kernels: paths per batch, at most the kernel's batch size
+    int ppt = 0;          // FP64 kernels, and k_tps where every batch is full: batches per item
     double *partial;      // [nscen*items][2*nout]: per-item sums and sums of squares
     int nout;             // outputs per scenario reduced by this launch
     int grid = 0;         // FP32 kernels: blocks launched (0: one per unit); block b
