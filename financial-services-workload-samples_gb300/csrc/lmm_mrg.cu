@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "lmm_internal.h"
+#include "lmm_soft64.h"
 
 namespace lmm {
 namespace {
@@ -37,6 +38,10 @@ constexpr int kSpan = 512;        // elements per lane per chunk (multiple of 32
 constexpr int64_t kHalfM1p1 = 2147483544;            // (m1 + 1) / 2
 constexpr float kNormF = (float)(1.0 / 4294967088.0); // 1 / (m1 + 1), rounded to FP32
 constexpr int kWarps = 4;         // warps per block
+// FP64 normals: tile columns and resident blocks. GB300, 167,772,160 normals:
+// 32 columns and 5 blocks (shared memory) 8.97 ms, 16 columns and 6 / 7 / 8 / 10
+// blocks 8.81 / 8.71 / 8.63 / 8.63 ms.
+constexpr int kCols64 = 16, kBlocks64 = 8;
 
 __device__ __forceinline__ void jump(const uint32_t *m, uint64_t v[3], uint64_t mod)
 {
@@ -53,39 +58,48 @@ __device__ __forceinline__ void jump(const uint32_t *m, uint64_t v[3], uint64_t 
     v[2] = r[2];
 }
 
-// One step of both recurrences; returns z in [1, m1].
-__device__ __forceinline__ uint32_t mrg_step(uint64_t x[3], uint64_t y[3])
+// v mod m1 and v mod m2 for v < 2^54: 2^32 is 209 mod m1 and 22853 mod m2, so
+// the high word folds into the low one.
+__device__ __forceinline__ uint32_t mod_m1(uint64_t v)
 {
-    int64_t p1 = ((int64_t)(1403580ULL * x[1]) - (int64_t)(810728ULL * x[0])) % (int64_t)kM1;
-    int64_t p2 = ((int64_t)(527612ULL * y[2]) - (int64_t)(1370589ULL * y[0])) % (int64_t)kM2;
-    if (p1 < 0) p1 += (int64_t)kM1;
-    if (p2 < 0) p2 += (int64_t)kM2;
-    x[0] = x[1];
-    x[1] = x[2];
-    x[2] = (uint64_t)p1;
-    y[0] = y[1];
-    y[1] = y[2];
-    y[2] = (uint64_t)p2;
-    return (uint32_t)(p1 > p2 ? p1 - p2 : p1 - p2 + (int64_t)kM1);
+    const uint64_t w = (v >> 32) * 209u + (uint32_t)v;                        // < 2^32 + 2^30
+    const uint32_t r = (uint32_t)w + 209u * (uint32_t)(w >> 32);
+    return r >= (uint32_t)kM1 ? r - (uint32_t)kM1 : r;
 }
 
-__device__ __forceinline__ double horner_rn(const double (&c)[8], double x)
+__device__ __forceinline__ uint32_t mod_m2(uint64_t v)
+{
+    const uint64_t w = (v >> 32) * 22853u + (uint32_t)v;                      // < 2^37
+    const uint64_t x = (uint64_t)(uint32_t)(w >> 32) * 22853u + (uint32_t)w;  // < 2^32 + 2^20
+    const uint32_t r = (uint32_t)x + 22853u * (uint32_t)(x >> 32);
+    return r >= (uint32_t)kM2 ? r - (uint32_t)kM2 : r;
+}
+
+// One step of both recurrences; returns z in [1, m1].
+__device__ __forceinline__ uint32_t mrg_step(uint32_t x[3], uint32_t y[3])
+{
+    const uint32_t p1 = mod_m1(1403580ULL * x[1] + 810728ULL * ((uint32_t)kM1 - x[0]));
+    const uint32_t p2 = mod_m2(527612ULL * y[2] + 1370589ULL * ((uint32_t)kM2 - y[0]));
+    x[0] = x[1];
+    x[1] = x[2];
+    x[2] = p1;
+    y[0] = y[1];
+    y[1] = y[2];
+    y[2] = p2;
+    return p1 > p2 ? p1 - p2 : p1 - p2 + (uint32_t)kM1;
+}
+
+__device__ __forceinline__ double horner(const double (&c)[8], double x)
 {
     double r = c[7];
 #pragma unroll
-    for (int i = 6; i >= 0; --i) r = __dadd_rn(__dmul_rn(r, x), c[i]);
+    for (int i = 6; i >= 0; --i) r = fma(r, x, c[i]);
     return r;
 }
 
-// AS241 PPND16.
-__device__ double ppnd16(double p)
+// AS241 PPND16 beyond |p - 1/2| = 0.425 (the central branch: lmm_soft64.h).
+__device__ double ppnd16_tail(double p)
 {
-    const double a[8] = {3.3871328727963666080e0, 1.3314166789178437745e+2, 1.9715909503065514427e+3,
-                         1.3731693765509461125e+4, 4.5921953931549871457e+4, 6.7265770927008700853e+4,
-                         3.3430575583588128105e+4, 2.5090809287301226727e+3};
-    const double b[8] = {1.0, 4.2313330701600911252e+1, 6.8718700749205790830e+2, 5.3941960214247511077e+3,
-                         2.1213794301586595867e+4, 3.9307895800092710610e+4, 2.8729085735721942674e+4,
-                         5.2264952788528545610e+3};
     const double c[8] = {1.42343711074968357734e0, 4.63033784615654529590e0, 5.76949722146069140550e0,
                          3.64784832476320460504e0, 1.27045825245236838258e0, 2.41780725177450611770e-1,
                          2.27238449892691845833e-2, 7.74545014278341407640e-4};
@@ -99,19 +113,15 @@ __device__ double ppnd16(double p)
                          7.86869131145613259100e-4, 1.84631831751005468180e-5, 1.42151175831644588870e-7,
                          2.04426310338993978564e-15};
     const double q = __dadd_rn(p, -0.5);
-    if (fabs(q) <= 0.425) {
-        const double r = __dadd_rn(0.180625, -__dmul_rn(q, q));
-        return __dmul_rn(q, horner_rn(a, r)) / horner_rn(b, r);
-    }
     double r = q < 0.0 ? p : __dadd_rn(1.0, -p);
     r = sqrt(-log(r));
     double v;
     if (r <= 5.0) {
         r = __dadd_rn(r, -1.6);
-        v = horner_rn(c, r) / horner_rn(d, r);
+        v = horner(c, r) / horner(d, r);
     } else {
         r = __dadd_rn(r, -5.0);
-        v = horner_rn(e, r) / horner_rn(f, r);
+        v = horner(e, r) / horner(f, r);
     }
     return q < 0.0 ? -v : v;
 }
@@ -141,32 +151,51 @@ __device__ float ppnd7(float q, float pt)
     return q < 0.0f ? -v : v;
 }
 
+// FP64 normals: the FP64 pipe bound them, with both branches of the inversion
+// run by nearly every warp (15% of the elements are tails): 64 clocks of an SM
+// an element. The central branch now runs mostly in integer arithmetic with the
+// same roundings (lmm_soft64.h) and a tile's tails are queued and evaluated in
+// full warps; integer instructions (about 1,400 an element) and the FP64 pipe
+// (9 clocks) share the 15 clocks left. GB300, 167,772,160 normals: 39.55 -> 8.63
+// ms; FP32 normals, by the recurrences' folded remainders, 1.11 -> 0.85 ms.
 template <int KIND>  // 0: uniforms (double), 1: normals (double), 2: normals (float)
-__global__ void __launch_bounds__(32 * kWarps)
+__global__ void __launch_bounds__(32 * kWarps, KIND == 1 ? kBlocks64 : 1)
 k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, double mean, double sd, void *out)
 {
     using T = typename std::conditional<KIND == 2, float, double>::type;
-    __shared__ T tile[kWarps][32][33];
+    constexpr int C = KIND == 1 ? kCols64 : 32;       // columns: elements per lane between stores
+    __shared__ T tile[kWarps][32][C + 1];
+    __shared__ uint16_t queue[KIND == 1 ? kWarps : 1][KIND == 1 ? 32 * C : 1];   // the tile's tails, row * (C + 1) + column
+    constexpr int kUnroll = KIND == 1 ? 1 : 4;         // GB300, FP64 normals: 2 elements a body 11.5 ms, 1 8.6 (instruction cache)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t chunk = ((int64_t)blockIdx.x * kWarps + w) * (32 * (int64_t)kSpan);
     if (chunk >= count) return;  // warp-uniform
 
-    uint64_t x[3] = {seed % kM1, 1, 1}, y[3] = {1, 1, 1};
+    uint64_t x64[3] = {seed % kM1, 1, 1}, y64[3] = {1, 1, 1};
     const uint64_t e0 = (uint64_t)(first + chunk);
     for (int k = 0; k < 64; ++k) {
         if ((e0 >> k) & 1ULL) {  // the same k for every lane: broadcast reads
-            jump(J.p1[k], x, kM1);
-            jump(J.p2[k], y, kM2);
+            jump(J.p1[k], x64, kM1);
+            jump(J.p2[k], y64, kM2);
         }
     }
-    jump(J.l1[lane], x, kM1);
-    jump(J.l2[lane], y, kM2);
+    jump(J.l1[lane], x64, kM1);
+    jump(J.l2[lane], y64, kM2);
+    uint32_t x[3], y[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        x[i] = (uint32_t)x64[i];
+        y[i] = (uint32_t)y64[i];
+    }
 
     T *o = static_cast<T *>(out);
     const float fmean = (float)mean, fsd = (float)sd;
-    for (int t = 0; t < kSpan / 32; ++t) {
-#pragma unroll 4
-        for (int i = 0; i < 32; ++i) {
+    auto scaled = [&](double v) { return __dadd_rn(mean, __dmul_rn(sd, v)); };
+    const bool plain = mean == 0.0 && sd == 1.0;      // mean + sd v = v for every v but -0, which does not occur
+    for (int t = 0; t < kSpan / C; ++t) {
+        int queued = 0;                               // warp-uniform
+#pragma unroll kUnroll
+        for (int i = 0; i < C; ++i) {
             const uint32_t z = mrg_step(x, y);
             if constexpr (KIND == 2) {
                 // q = u - 1/2 and min(u, 1-u) from the integer z, in FP32 (no FP64)
@@ -174,19 +203,31 @@ k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, doubl
                 const uint32_t zt = min(z, (uint32_t)(2 * kHalfM1p1) - z);
                 const float pt = __fmul_rn(__uint2float_rn(zt), kNormF);
                 tile[w][lane][i] = __fadd_rn(fmean, __fmul_rn(fsd, ppnd7(q, pt)));
+            } else if constexpr (KIND == 1) {
+                uint64_t u;
+                bool central;
+                const double v = __longlong_as_double((long long)as241_central(z, &u, &central));
+                const unsigned tails = __ballot_sync(0xffffffffu, !central);
+                if (!central) queue[w][queued + __popc(tails & ((1u << lane) - 1))] = (uint16_t)(lane * (C + 1) + i);
+                queued += __popc(tails);
+                tile[w][lane][i] = central ? (plain ? v : scaled(v)) : __longlong_as_double((long long)u);
             } else {
-                const double u = (double)z * (1.0 / 4294967088.0);
-                if constexpr (KIND == 0)
-                    tile[w][lane][i] = (T)u;
-                else
-                    tile[w][lane][i] = (T)__dadd_rn(mean, __dmul_rn(sd, ppnd16(u)));
+                tile[w][lane][i] = (T)((double)z * (1.0 / 4294967088.0));
             }
         }
         __syncwarp();
+        if constexpr (KIND == 1) {
+            double *flat = &tile[w][0][0];
+            for (int j = lane; j < queued; j += 32) {
+                const int at = queue[w][j];
+                flat[at] = scaled(ppnd16_tail(flat[at]));
+            }
+            __syncwarp();
+        }
 #pragma unroll 4
-        for (int r = 0; r < 32; ++r) {
-            const int64_t e = chunk + (int64_t)r * kSpan + t * 32 + lane;
-            if (e < count) o[e] = tile[w][r][lane];
+        for (int r = lane / C; r < 32; r += 32 / C) {
+            const int64_t e = chunk + (int64_t)r * kSpan + t * C + lane % C;
+            if (e < count) o[e] = tile[w][r][lane % C];
         }
         __syncwarp();
     }
