@@ -38,7 +38,7 @@ METRIC = "paths/s value+all Greeks: FP32 adjoint vs FP64 bump, 1 GB300, rel err<
 WORKLOAD = 2
 # The timed fused kernel and its ncu DRAM-traffic summary, per workload that
 # --workload accepts (normals in HBM).
-KERNELS = {2: ("k_tps<80,40,hbm>", os.path.join(ROOT, "profiles", "lmm_fused_f32_80x40.json")),
+KERNELS = {2: ("k_tpb<80,40,hbm>", os.path.join(ROOT, "profiles", "lmm_fused_f32_80x40.json")),
            3: ("k_tpq<160,120,hbm>", os.path.join(ROOT, "profiles", "lmm_fused_f32_160x120.json"))}
 
 # Algorithmic operations per path (reference formulas, liborSwaptionGreeks.cpp),
@@ -487,7 +487,7 @@ def run_ours(args):
                 kms = sorted(kt)[1]
                 others[c.name] = {"paths_per_s": c.nscen * c.paths / (kms * 1e-3), "ms": kms,
                                   "nn": c.nn, "nmat": c.nmat, "scenarios": c.nscen, "normals": mode,
-                                  "kernel": "k_tps (thread per path, reverse split over the rate halves)" if c.nn == 80 else
+                                  "kernel": "k_tpb (thread per path; reverse in blocks of 20 rates)" if c.nn == 80 else
                                   "k_tpq (thread per path; reverse in passes over blocks of 40 rates, rebuilt "
                                   "from each block's top drift sums, rates saved every 8 steps)"}
                 del zw

@@ -181,26 +181,14 @@ void mark(lmm_engine *e, int i)
 // Kernel variant keys for the blocks-per-SM cache.
 int variant_key(int family, Mode mode, bool philox) { return family * 16 + (int)mode * 2 + (philox ? 1 : 0); }
 
-int f32_family(const lmm_engine *e)
-{
-    if (lmm::f32_tpp_supports(e->nn, e->nmat)) return 1;
-    if (lmm::f32_wpp_supports(e->nn, e->nmat)) return 2;
-    return 0;
-}
-
-// Kernel family of an FP32 call: 7 (one thread per path, the forward in two
-// passes of 80 rates and the reverse in passes over blocks of 40 rates,
-// k_tpq) for fused nn=160, nmat=120 calls (LMM_USE_TPQ; GB300, 1,048,576
-// paths: 14.15 ms against 18.29 for the thread pair); 5 (two threads per
-// path, lmm_f32_tp2.cu) for that shape's forward/backward pair (and its fused
-// calls without LMM_USE_TPQ; 2.1x the warp-per-path rate); 6 (one thread per
-// path with the reverse split over the rate halves, k_tps) for fused 80/40
-// calls (LMM_USE_TPS); otherwise f32_family. At 80/40 the thread pair ran
-// 13.4-15.5 ms against 11.7 ms for the thread-per-path kernel (4,194,304
-// paths), so it does not take that shape.
-#ifndef LMM_USE_TPS
-#define LMM_USE_TPS 1
-#endif
+// Kernel family of an FP32 call of many paths (family_at):
+//   6 thread per path in rate blocks (k_tpb): fused 80/40 calls, and every mode
+//     of the shapes below without a kernel of their own;
+//   1 thread per path (k_tpp): the 80/40 forward/backward pair, on a tape;
+//   7 thread per path in blocks of 40 rates (k_tpq): fused 160/120 calls (GB300,
+//     1,048,576 paths: 14.2 ms; thread pair 18.3);
+//   5 two threads per path (lmm_f32_tp2.cu): the 160/120 pair, on a tape;
+//   2 warp per path (k_wpp): checkpoint intervals that are no multiple of 4.
 #ifndef LMM_USE_TPQ
 #define LMM_USE_TPQ 1
 #endif
@@ -208,9 +196,9 @@ int family_for(const lmm_engine *e, Mode mode)
 {
     if (lmm::f32_tp2_supports(e->nn, e->nmat))
         return LMM_USE_TPQ && mode == Mode::Fused && lmm::f32_tpq_supports(e->nn, e->nmat) ? 7 : 5;
-    const int f = f32_family(e);
-    if (LMM_USE_TPS && f == 1 && mode == Mode::Fused) return 6;
-    return f;
+    if (lmm::f32_tpp_supports(e->nn, e->nmat) && mode != Mode::Fused) return 1;
+    if (lmm::f32_tpb_supports(e->nn, e->nmat, e->dm.ckpt)) return 6;
+    return lmm::f32_wpp_supports(e->nn, e->nmat) ? 2 : 0;
 }
 
 // Paths one block takes per batch.
@@ -218,7 +206,7 @@ int batch_paths(const lmm_engine *e, int fam, Mode mode)
 {
     if (fam == 1) return lmm::tpp_block_threads(mode);
     if (fam == 5) return lmm::tp2_paths_per_block(e->nn);
-    if (fam == 6) return lmm::tps_block_threads();
+    if (fam == 6) return lmm::tpb_block_threads(e->nn, e->nmat);
     if (fam == 7) return lmm::tpq_block_threads();
     return lmm::wpp_block_threads() / 32;
 }
@@ -226,19 +214,18 @@ int batch_paths(const lmm_engine *e, int fam, Mode mode)
 // Paths that share a warp (warp-per-path kernels: the block's paths).
 int batch_gran(int fam) { return fam == 2 ? lmm::wpp_block_threads() / 32 : 32; }
 
-// Kernels whose batches may be ragged (run by the warps that have paths):
-// k_tps as a variant of its own, the 80/40 forward-only kernel, warp per path.
-// The others run whole batches of the block.
+// Kernels whose batches may be ragged (run by the warps that have paths): rate
+// blocks, the 80/40 forward-only kernel, warp per path. The others run whole
+// batches of the block.
 bool ragged_batches(int fam, Mode mode) { return fam == 2 || fam == 6 || (fam == 1 && mode == Mode::Forward); }
 
 // Time of a ragged batch of n paths relative to a full one. GB300, one batch
-// per SM, one / two / three warps per scheduler: k_tps 0.113, 0.125, 0.156 ms
-// (0.150 in its whole-batch variant), the forward of the 80/40 pair 0.037,
-// 0.048, 0.059.
-double batch_cost(int fam, int n)
+// per SM, 80/40, one / two / three / four warps per scheduler: k_tpb
+// 0.092, 0.120, 0.150, 0.187 ms; the forward of the pair 0.037, 0.048, 0.059.
+double batch_cost(int fam, int n, int batch)
 {
-    const int wps = (n + 127) / 128;
-    if (fam == 6) return wps == 1 ? 0.75 : wps == 2 ? 0.84 : 1.04;
+    const int wps = (n + 127) / 128, full = batch / 128;
+    if (fam == 6) return full <= 1 ? 1.0 : 0.49 + 0.51 * (wps - 1) / (full - 1);
     if (fam == 1) return wps == 1 ? 0.63 : wps == 2 ? 0.82 : 1.0;
     return 1.0;
 }
@@ -249,7 +236,7 @@ cudaError_t launch_f32_family(int fam, const lmm::DevModel &m, Mode mode, const 
 {
     if (fam == 1) return lmm::launch_tpp_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
     if (fam == 5) return lmm::launch_tp2_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
-    if (fam == 6) return lmm::launch_tps_any(m, z, seed, path0, philox, w, tape, s);
+    if (fam == 6) return lmm::launch_tpb_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
     if (fam == 7) return lmm::launch_tpq_any(m, z, seed, path0, philox, w, tape, s);
     return lmm::launch_wpp_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
 }
@@ -267,7 +254,7 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
     if (family == 1) err = lmm::tpp_blocks_per_sm(mode, philox, &b);
     else if (family == 2) err = lmm::wpp_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 5) err = lmm::tp2_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
-    else if (family == 6) err = lmm::tps_blocks_per_sm(philox, &b);
+    else if (family == 6) err = lmm::tpb_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 7) err = lmm::tpq_blocks_per_sm(philox, &b);
     else return fail(LMM_ERR_UNSUPPORTED, "unknown kernel family");
     if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
@@ -279,20 +266,24 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
 
 // The family of a call of `paths` paths: the warp-per-path kernels for few
 // paths, family_for above. A thread-per-path kernel takes one path's latency
-// (80/40 fused 0.113 ms, 160/120 0.47 ms) for anything from one path to a
+// (80/40 fused 0.090 ms, 160/120 0.47 ms) for anything from one path to a
 // device full of single warps; a warp per path takes 0.04 ms (0.096) for one
 // path and its throughput beyond the device's resident warps (3,648 on GB300):
-// 80/40 fused, kernel alone, 3,001 / 4,864 / 9,728 paths 0.055 / 0.086 / 0.152
-// against 0.113 ms, 160/120 0.15 / 0.25 / 0.48 against 0.47-0.48 ms. The line
-// is two fills of the device, for every mode alike: the fused call and the
-// forward/backward pair of the same size must round alike.
+// 80/40 fused, kernel alone, 3,001 / 4,864 / 7,296 paths 0.049 / 0.079 / 0.105
+// against 0.090 ms, 160/120 at 3,001 / 4,864 / 9,728 paths 0.15 / 0.25 / 0.48
+// against 0.47-0.48 ms. The line is one and a half fills of the device for the
+// shapes whose fused call runs in rate blocks, two for the others, and the same
+// for every mode: the fused call and the forward/backward pair of the same size
+// must round alike.
 int family_at(lmm_engine *e, Mode mode, int64_t paths, int *fam)
 {
     *fam = family_for(e, mode);
     if (*fam == 0 || *fam == 2 || !lmm::f32_wpp_supports(e->nn, e->nmat)) return LMM_OK;
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, 2, Mode::Fused, false, &bps));
-    if (paths <= 2 * (int64_t)e->sms * bps * batch_paths(e, 2, Mode::Fused) / e->nscen) *fam = 2;
+    const int64_t fill = (int64_t)e->sms * bps * batch_paths(e, 2, Mode::Fused);
+    const int64_t line = family_for(e, Mode::Fused) == 6 ? fill + fill / 2 : 2 * fill;
+    if (paths <= line / e->nscen) *fam = 2;
     return LMM_OK;
 }
 
@@ -326,10 +317,10 @@ void plan_items(const lmm_engine *e, int64_t nvs, int64_t paths, int block, int 
 // partial one; one wave of blocks loops over the units, so a launch takes
 // ceil(units / blocks) times the longest unit. A ragged batch's time goes with
 // the warps on the busiest of an SM's four schedulers (batch_cost), hardly with
-// its paths. The plan is the cheapest split: 20,000 paths take every SM with
-// five warps (0.125 ms) where whole batches took 53 SMs with twelve (0.150),
-// and 131,072 paths two full batches and one of three warps on each of 147 SMs
-// where they took three full ones on 114 (0.440 -> 0.423 ms a call).
+// its paths. The plan is the cheapest split: 30,000 paths take every SM with
+// seven warps (0.117 ms) where whole batches took 59 SMs with sixteen (0.183),
+// and 131,072 paths a full batch and one of eleven warps on each SM where a
+// second full one took 0.352 ms (0.318).
 struct PathPlan {
     int64_t items = 1, ipaths = 1;
     int bpaths = 1;
@@ -346,41 +337,40 @@ PathPlan plan_paths(const lmm_engine *e, int fam, Mode mode, int64_t nvs, int64_
 {
     const int batch = batch_paths(e, fam, mode), gran = batch_gran(fam);
     const int64_t cap = std::max<int64_t>(1, (int64_t)e->sms * bps);
-    const bool ragged = ragged_batches(fam, mode), whole = !ragged || fam == 6;
+    const bool ragged = ragged_batches(fam, mode);
     const double unit = 0.015;     // a unit's own cost: accumulators cleared and written out
     PathPlan best;
     double best_cost = 1e300;
-    auto take = [&](double cost, const PathPlan &p) {
-        if (cost >= best_cost * (1.0 - 1e-9)) return;
+    // `it` units per scenario, in whole batches or in batches of at most bp paths
+    auto take = [&](int64_t it, int bp) {
+        int64_t per = ((paths + it - 1) / it + gran - 1) / gran * gran;
+        const int64_t nb = (per + batch - 1) / batch;
+        if (!ragged) per = nb * batch;
+        const int64_t n = (paths + per - 1) / per;
+        const double waves = (double)((nvs * n + cap - 1) / cap);
+        const double cost = !ragged ? waves * ((double)nb + unit)
+                                    : waves * ((double)(per / bp) * batch_cost(fam, bp, batch) +
+                                               (per % bp ? batch_cost(fam, (int)(per % bp), batch) : 0.0) + unit);
+        if (cost >= best_cost * (1.0 - 1e-9) || nb > INT32_MAX) return;
         best_cost = cost;
-        best = p;
+        best = PathPlan{n, per, bp, ragged ? 0 : (int)nb};
+    };
+    auto units = [&](int64_t it) {
+        it = std::min(std::max<int64_t>(1, it), (paths + gran - 1) / gran);
+        const int per = (int)std::min<int64_t>((paths + it - 1) / it, batch);
+        for (int bp = batch; bp >= 128 || bp == batch; bp -= 128) {
+            take(it, bp);
+            if (!ragged || bp <= 128 || bp - 128 < per / 4) break;
+        }
     };
     // Several scenarios: short units too, which end within a few batches of each
-    // other (256 curves of 43 batches on 152 SMs: 7 units of 11 batches on the
-    // busiest SM, or 73 of one; GB300 10.47 -> 10.07 ms).
-    if (whole && nvs > 1)
-        for (int64_t ppt = 1; ppt <= 64; ++ppt) {
-            const int64_t n = (paths + ppt * batch - 1) / (ppt * batch);
-            if (nvs * n <= 16384)
-                take((double)((nvs * n + cap - 1) / cap) * ((double)ppt + unit), PathPlan{n, ppt * batch, batch, (int)ppt});
-        }
-    // units per scenario: what fills 1 .. 16 waves of blocks
-    for (int w = 1; w <= 16; ++w) {
-        const int64_t it = std::min(std::max<int64_t>(1, w * cap / nvs), (paths + gran - 1) / gran);
-        const int64_t per = ((paths + it - 1) / it + gran - 1) / gran * gran;
-        auto waves = [&](int64_t n) { return (double)((nvs * n + cap - 1) / cap); };
-        if (whole) {
-            const int64_t ppt = (per + batch - 1) / batch, n = (paths + ppt * batch - 1) / (ppt * batch);
-            if (ppt <= INT32_MAX) take(waves(n) * ((double)ppt + unit), PathPlan{n, ppt * batch, batch, (int)ppt});
-        }
-        for (int bp = (int)std::min<int64_t>(batch, per); ragged; bp -= 128) {
-            const int64_t n = (paths + per - 1) / per;
-            take(waves(n) * ((double)(per / bp) * batch_cost(fam, bp) +
-                             (per % bp ? batch_cost(fam, (int)(per % bp)) : 0.0) + unit),
-                 PathPlan{n, per, bp, 0});
-            if (bp <= 128) break;
-        }
-    }
+    // other (256 curves of 16,384 paths in units of one batch on every SM where
+    // units of eleven left some SMs a unit more: GB300 10.47 -> 10.07 ms).
+    if (nvs > 1)
+        for (int64_t nb = 1; nb <= 64; ++nb)
+            if (nvs * ((paths + nb * batch - 1) / (nb * batch)) <= 16384) units((paths + nb * batch - 1) / (nb * batch));
+    // units per scenario that fill 1 .. 16 waves of blocks
+    for (int w = 1; w <= 16; ++w) units(w * cap / nvs);
     return best;
 }
 
@@ -468,13 +458,12 @@ int wpp_scratch(lmm_engine *e, int64_t blocks, float **out)
     return LMM_OK;
 }
 
-// Scratch of the fused split-reverse kernel (k_tps) for a grid of `blocks`
-// blocks: per block the drift sums at the half boundary, the suffix sums
-// handed from the upper to the lower half, the lower half's parked rates and
-// the upper half's deltas.
-int tps_scratch(lmm_engine *e, int64_t blocks, float **out)
+// Scratch of the rate-block kernel (k_tpb) for a grid of `blocks` blocks: what
+// waits between its passes and blocks, and the rate checkpoints.
+int tpb_scratch(lmm_engine *e, int64_t blocks, float **out)
 {
-    LMM_TRY(e->wscratch.ensure(sizeof(float) * (size_t)blocks * lmm::tps_scratch_floats_per_block(e->nn, e->nmat)));
+    LMM_TRY(e->wscratch.ensure(sizeof(float) * (size_t)blocks *
+                               lmm::tpb_scratch_floats_per_block(e->nn, e->nmat, e->dm.ckpt)));
     *out = e->wscratch.as<float>();
     return LMM_OK;
 }
@@ -522,7 +511,7 @@ int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t p
     LMM_TRY(plan(e, fam, mode, e->nscen, paths, bps, nout, &w));
     if (fam == 2) LMM_TRY(wpp_scratch(e, w.grid, &tape));
     if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &tape));
-    if (fam == 6) LMM_TRY(tps_scratch(e, w.grid, &tape));
+    if (fam == 6) LMM_TRY(tpb_scratch(e, w.grid, &tape));
     if (fam == 7) LMM_TRY(tpq_scratch(e, w.grid, &tape));
     LMM_TRY(next_stamp(e));
     mark(e, 0);
@@ -818,7 +807,7 @@ int lmm_engine_set_checkpoint_interval(lmm_engine *e, int32_t steps)
     if (fam == 0)
         return fail(LMM_ERR_UNSUPPORTED, "no FP32 kernel for nn=" + std::to_string(e->nn) +
                                              ", nmat=" + std::to_string(e->nmat));
-    if ((fam == 1 || fam == 6) && steps != 0)
+    if (lmm::f32_tpp_supports(e->nn, e->nmat) && steps != 0)
         return fail(LMM_ERR_UNSUPPORTED, "the nn=80, nmat=40 kernel keeps every step's drift sums on chip and "
                                          "takes no rate checkpoints: only 0 is accepted");
     if (fam == 5 && steps % 2 != 0)
@@ -1058,7 +1047,7 @@ int lmm_swaption_breakdown_f64_device(lmm_engine *e, const double *d_z, int64_t 
 // Each piece writes its own range of partial sums and one ordered k_finalize
 // covers them all. Single-scenario engines only.
 #ifndef LMM_HOST_SPLIT
-#define LMM_HOST_SPLIT 1, 2, 6, 18, 45
+#define LMM_HOST_SPLIT 1, 3, 8, 24, 36
 #endif
 constexpr int kHostSplit[] = {LMM_HOST_SPLIT};
 constexpr int kHostChunks = sizeof(kHostSplit) / sizeof(kHostSplit[0]);
@@ -1111,7 +1100,7 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
         // the pieces run one after another
         LMM_TRY(fam == 2 ? wpp_scratch(e, most, &wscr)
                          : fam == 5 ? tp2_scratch(e, most, &wscr)
-                                    : fam == 6 ? tps_scratch(e, most, &wscr) : tpq_scratch(e, most, &wscr));
+                                    : fam == 6 ? tpb_scratch(e, most, &wscr) : tpq_scratch(e, most, &wscr));
     }
     LMM_TRY(next_stamp(e));
     if (!e->copy_stream) LMM_CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));

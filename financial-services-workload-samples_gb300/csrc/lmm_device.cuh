@@ -118,9 +118,22 @@ __device__ __forceinline__ void box_muller_f64(uint32_t a, uint32_t b, double &z
     z1 = r * s;
 }
 
-// Barrier of the block's first n threads (n a multiple of 32), for the step
-// loops of batches that do not fill the block.
-__device__ __forceinline__ void sync_threads(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
+// 2^x to about an ulp, for what is not followed by another rounding of its size:
+// x = n + f and the exponential series for 2^f, |f| <= 1/2 (the term left out is
+// below 6e-9); beyond 2^+-125 the unit's.
+__device__ __forceinline__ float ex2_ulp(float x)
+{
+    const float n = rintf(x), f = (x - n) * 0.693147181f;
+    float p = 1.0f / 5040.0f;
+    p = fmaf(p, f, 1.0f / 720.0f);
+    p = fmaf(p, f, 1.0f / 120.0f);
+    p = fmaf(p, f, 1.0f / 24.0f);
+    p = fmaf(p, f, 1.0f / 6.0f);
+    p = fmaf(p, f, 0.5f);
+    p = fmaf(p, f, 1.0f);
+    p = fmaf(p, f, 1.0f);
+    return fabsf(x) < 125.0f ? p * __int_as_float((127 + (int)n) << 23) : ex2_approx(x);
+}
 
 __device__ __forceinline__ float warp_sum(float v)
 {
@@ -189,6 +202,39 @@ __device__ __forceinline__ void two_sum_acc(float &s, float &c, float x)
     const float v = __fsub_rn(t, s);
     c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, v)), __fsub_rn(x, v)));
     s = t;
+}
+
+// Two FP32 values in a register pair: one instruction for both, each rounded as
+// the scalar operation (PTX ISA: add/sub/fma.rn.f32x2).
+using P2 = unsigned long long;
+
+__device__ __forceinline__ P2 p2(float lo, float hi)
+{
+    P2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack(P2 x, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
+}
+__device__ __forceinline__ P2 add2(P2 a, P2 b)
+{
+    P2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ P2 sub2(P2 a, P2 b)
+{
+    P2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c)
+{
+    P2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 // The F2 nearest a double (host data staged once per block).

@@ -1,0 +1,634 @@
+// FP32 thread-per-path LMM kernel in rate blocks (k_tpb): the fused call for
+// NN=80, NMAT=40, and every mode of the shapes without a kernel of their own.
+//
+// One CUDA thread carries one Monte Carlo path through
+//   forward   path_calc_b1   (LiborMarketModel/liborSwaptionGreeks.cpp:34-82)
+//   payoff    portfolio_b    (:120-211), adjoint aliasing of :178/:181 fixed
+//   reverse   path_calc_b2   (:86-117) plus the vega adjoint (not in the reference)
+// The forward runs in passes of kFR = 40 rates (steps in skewed pairs, the two
+// cells of a step at rates 2m and 2m+1 on one reciprocal: fwd_pair_window_cap in
+// lmm_f32_tpp.cu, whose roundings these are), the reverse in blocks of kRR = 20
+// rates from the top (groups of four steps as a skewed wavefront, rebuilt from
+// the drift sums at the block's top rate: rev_block_window there). One copy of
+// either body serves every pass and block; what waits between them (per-step
+// drift and suffix sums at block boundaries, the rates, the log-adjoints, the
+// rate checkpoints) lies in the block's scratch in L2.
+//
+// What bounds it. The cells read about 140,000 register operands a path and the
+// register file delivers two 32-bit operands a clock and scheduler; issue slots
+// (68,000 a path) come next. Blocks of 20 rates leave 128 registers a thread,
+// so 16 warps cover the chains (ncu at 1,089,536 paths, 80/40: issue active 76%,
+// dispatch stalls 0.6 of an issue). GB300, 80/40, against the kernel that held
+// 40 rates and 12 warps: 256 curves x 16,384 paths 10.07 -> 9.19 ms, 16,777,216
+// Philox paths 40.57 -> 38.85 ms, 131,072 paths 0.422 -> 0.325 ms. Steps on the
+// way (Philox paths): constants read from shared memory (one 16-byte broadcast a
+// position) instead of the parameter bank 39.4 -> 38.4 ms; one barrier per batch
+// instead of one every second step group 40.4 -> 39.4 ms, none 58 ms (the warps
+// drift apart on the code: instruction cache); blocks of 40 / 10 / 8 rates 41.2 /
+// 42.3 / 45 ms; groups of 5 steps 41.4 ms; ragged batches 38.4 -> 39.7 ms; packed
+// column sums 39.7 -> 38.85 ms. Two paths a thread in packed FP32
+// (fma.rn.f32x2) reads as many operands for a path and ran 40.5 ms.
+//
+// Other shapes, against the kernel that gave a path two threads or a warp: 50,001
+// paths of 96/60 0.96 -> 0.405 ms.
+//
+// The reverse runs in units of sigma = lambda sqrt(delta): with X = 1/(delta L),
+// t = 1/(X + 1), y = (drift sum + normal term)/sqrt(delta) a cell is
+//   X *= 2^(a y + c), y -= sigma t, S += sigma Pb, Pb += sigma (1 - t) t S,
+//   vega_sigma += Pb (y - sigma) + t S        (a = sigma log2 e, c = -sigma a/2)
+// so one constant serves where lambda, delta lambda and delta^2 lambda stood;
+// vega_lambda = sqrt(delta) vega_sigma, applied to the block's sums.
+#pragma once
+
+#include "lmm_device.cuh"
+#include "lmm_f32_payoff.cuh"
+
+namespace lmm {
+namespace {
+
+constexpr int kFR = 40, kFC = 8;       // forward: rates per pass, and per chunk of its body
+constexpr int kRR = 20, kRG = 4;       // reverse: rates per block, steps per group
+constexpr float kPadIL = 1e15f;        // inverse rate of the padding above rate nn: t = 0 beside any sum
+
+// Sizes and offsets of one shape, in rows of B values where B counts threads.
+struct TpbLay {
+    int nn, nmat, M, nf, nr;           // nf forward passes, nr reverse blocks
+    int nout;
+    // shared memory, bytes
+    int kf, kr, il0, ost, okf, owf, okk, vg, acc, bytes;
+    // scratch, rows: drift sums at the top of every half pass [2 nf][nmat], suffix sums at the bottom of the
+    // reverse block last run [nmat], rates [kFR nf], log-adjoints, then deltas [kRR nr], annuity factors [M],
+    // normal terms [nmat], checkpoints [nck][kRR nr]
+    int s_v, s_s, s_x, s_d, s_b, s_q, s_ck;
+};
+
+__host__ __device__ constexpr int tpb_al(int x) { return (x + 15) & ~15; }
+
+__host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int B)
+{
+    TpbLay L{};
+    L.nn = nn;
+    L.nmat = nmat;
+    L.M = nn - nmat;
+    L.nf = (nn + kFR - 1) / kFR;
+    L.nr = (nn + kRR - 1) / kRR;
+    L.nout = mode == Mode::Fused ? 1 + 2 * nn : (mode == Mode::Forward ? 1 : 2 * nn);
+    const int kc = nmat + kFR * L.nf;                       // NMAT zero rows (k < 0), then k = 0 ..
+    L.kf = 0;
+    L.kr = L.kf + 16 * kc;
+    L.il0 = L.kr + 16 * kc;
+    L.ost = tpb_al(L.il0 + 4 * kFR * L.nf);
+    L.okf = tpb_al(L.ost + 4 * (L.M + 1));
+    L.owf = L.okf + 4 * kMaxNopt;
+    L.okk = L.owf + 4 * kMaxNopt;
+    L.vg = L.okk + 8 * kMaxNopt;
+    const int rows = kRG + kRR * L.nr;                      // kRG spare rows for k < 0
+    L.acc = L.vg + 4 * rows * B;
+    L.bytes = L.acc + 8 * (B / 32) * 2 * L.nout;
+    L.s_v = 0;
+    L.s_s = 2 * L.nf * nmat;
+    L.s_x = L.s_s + nmat;
+    L.s_d = L.s_x + kFR * L.nf;
+    L.s_b = L.s_d + kRR * L.nr;
+    L.s_q = L.s_b + L.M;
+    L.s_ck = L.s_q + nmat;
+    return L;
+}
+
+// What the forward holds of a rate: the inverse rate IL itself (80/40), or the
+// log2 of its fall since the start, D: IL = IL0 2^-D (LOGS, other shapes). A
+// product a step collects a rounding of IL each (4e-7 over 60 steps), and a drift
+// sum that starts from the normal term one of that term a rate; D stays below 1
+// or so, the normal term is added to the drift sum at each rate, and the payoff's
+// factors keep their rounding. Against the exact paths, 100 sets of normals, 96/60,
+// 50,001 paths: median error of the Greeks 2.8e-7 (the rates themselves, a warp a
+// path) -> 1.1e-7, and sets in which a swaption at the money paid on one side only
+// 17 -> 1; 150/100, 20,000 paths 5.7e-7 -> 8.1e-8 and 12 -> 0. It takes 0.405 ms
+// where products took 0.343 (96/60). 80/40 rounds as its pair of calls does.
+template <bool LOGS>
+__device__ __forceinline__ float inv_rate(float x, const float *il0)
+{
+    return LOGS ? *il0 * ex2_approx(-x) : x;
+}
+
+// One forward cell: drift sum, and the rate's update; the new inverse rate.
+template <bool LOGS>
+__device__ __forceinline__ float fwd_cell_b(float &x, float &V, float sq, float a, float c, float zc, float t, const float *il0)
+{
+    V = fmaf(zc, t, V);
+    if (!LOGS) return x *= ex2_approx(-fmaf(a, V, c));
+    x += fmaf(a, V + sq, c);
+    return inv_rate<true>(x, il0);
+}
+
+// Forward steps n and n+1 over the kFR rates LO .. LO+kFR-1 in R[]: cell (n, p)
+// next to cell (n+1, p-1). kcn points at step n's constants of local rate 0 (k =
+// LO-n-1; zero rows below k = 0 make inactive cells exact no-ops), nrel = n - LO <
+// kFR - 1. V0, V1 enter as the drift sums below the pass and leave as the sums at
+// its top; V0h, V1h are those at its middle rate kRR - 1. q0, q1 are the normal
+// terms (LOGS; in V0, V1 otherwise), il0 the pass's first inverse rates.
+template <bool LOGS>
+__device__ __forceinline__ void fwd_pair_block(float (&R)[kFR], const float4 *kcn, float delta, int nrel, float q0, float q1,
+                                               const float *il0, float &V0, float &V1, float &V0h, float &V1h)
+{
+    static_assert(kFC % 2 == 0 && kFR % kFC == 0 && kFR == 2 * kRR, "reciprocal pairs (2m, 2m+1) inside chunks");
+    float A[3], C[3], Z[3];
+    auto load = [&](int j) {
+        const float4 q = kcn[j];
+        A[(j + 3) % 3] = q.x;
+        C[(j + 3) % 3] = q.y;
+        Z[(j + 3) % 3] = q.z;
+    };
+    auto cell = [&](int p, float &V, float q, int j, float t) {
+        return fwd_cell_b<LOGS>(R[p], V, q, A[(j + 3) % 3], C[(j + 3) % 3], Z[(j + 3) % 3], t, il0 + p);
+    };
+    V0h = V0;
+    V1h = V1;
+    const int c0 = nrel + 1 > 0 ? (nrel + 1) / kFC : 0;
+    float t0n = 0.0f, t1n = 0.0f;       // the second reciprocals of the steps' pairs in flight
+    float even = 0.0f;                  // inverse rate p-1 after step n
+#pragma unroll
+    for (int c = 0; c * kFC < kFR; ++c) {
+        if (c >= c0) {
+            if (c == c0) {
+                if (c > 0) load(c * kFC - 2);
+                load(c * kFC - 1);
+                if (c > 0) {            // step n+1's pair below the chunk: rates inactive in step n, unchanged
+                    const int p = c > 0 ? c * kFC - 2 : 0;
+                    float ta;
+                    rcp_pair(inv_rate<LOGS>(R[p], il0 + p) + delta, inv_rate<LOGS>(R[p + 1], il0 + p + 1) + delta, ta, t1n);
+                }
+            }
+#pragma unroll
+            for (int p = c * kFC; p < (c + 1) * kFC; ++p) {
+                load(p);
+                float t;
+                if (p % 2 == 0)
+                    rcp_pair(inv_rate<LOGS>(R[p], il0 + p) + delta, inv_rate<LOGS>(R[p + 1], il0 + p + 1) + delta, t, t0n);
+                else
+                    t = t0n;
+                const float x = cell(p, V0, q0, p, t);
+                if (p % 2 == 1) {
+                    float ta;
+                    rcp_pair(even + delta, x + delta, ta, t1n);
+                    cell(p - 1, V1, q1, p - 2, ta);
+                } else {
+                    even = x;
+                    if (p >= 1) cell(p - 1, V1, q1, p - 2, t1n);
+                }
+                if (p == kRR - 1) V0h = V0;
+                if (p == kRR) V1h = V1;
+            }
+        }
+    }
+    cell(kFR - 1, V1, q1, kFR - 2, t1n);
+}
+
+// One forward step alone (the last of an odd number).
+template <bool LOGS>
+__device__ __forceinline__ void fwd_one_block(float (&R)[kFR], const float4 *kcn, float delta, float sq, const float *il0,
+                                              float &V, float &Vh)
+{
+#pragma unroll
+    for (int p = 0; p < kFR; p += 2) {
+        float t[2];
+        rcp_pair(inv_rate<LOGS>(R[p], il0 + p) + delta, inv_rate<LOGS>(R[p + 1], il0 + p + 1) + delta, t[0], t[1]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float4 q = kcn[p + e];
+            fwd_cell_b<LOGS>(R[p + e], V, sq, q.x, q.y, q.z, t[e], il0 + p + e);
+        }
+        if (p + 2 == kRR) Vh = V;
+    }
+}
+
+struct TpbStep {
+    float y, S;
+};
+
+// Reverse steps n .. n-G+1 over the rates LO .. LO+kRR-1 in X[], Pb[]: cell (n-g,
+// i+g) at position i. kr and vg point at step n's constants and vega rows of local
+// position 0. A vega row stays in registers from position j to j-2(G-1) and takes
+// one read-modify-write. When every step is active at the bottom rate (LO > n) the
+// body runs to its last position and flushes the rows still open; otherwise it is
+// left below the lowest active position (the open rows hold no-op cells of spare
+// rows). With CK, rates j > tl are replaced by rs[j*B] after their last cell.
+template <int B, int G, bool CK>
+__device__ __forceinline__ void rev_block(float (&X)[kRR], float (&Pb)[kRR], TpbStep (&st)[G], const float4 *kr, float *vg,
+                                          int n, int LO, const float *rs, int tl)
+{
+    constexpr int JMAX = kRR + G - 2, W = 2 * G - 1;
+    float A[W], C[W], Sg[W], acc[W];
+    auto load = [&](int j) {
+        const float4 q = kr[j];
+        A[j % W] = q.x;
+        C[j % W] = q.y;
+        Sg[j % W] = q.z;
+    };
+#pragma unroll
+    for (int j = kRR; j <= JMAX; ++j) {
+        load(j);
+        acc[j % W] = 0.0f;
+    }
+    const bool full = LO > n;
+    const int imin = n - 2 * G + 3 - LO;     // lowest local position with an active cell
+#pragma unroll
+    for (int i = kRR - 1; i >= -(G - 1); --i) {
+        if (!full && i < imin) return;
+        if (i >= 0) {
+            load(i);
+            acc[i % W] = 0.0f;
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (i + g >= 0 && i + g <= kRR - 1) {
+                const int j = (i + 2 * g) % W, x = i + g;
+                const float xn = X[x] * ex2_approx(fmaf(A[j], st[g].y, C[j]));
+                const float t = rcp_approx(xn + 1.0f);
+                const float h = st[g].y - Sg[j];
+                st[g].y = fmaf(-Sg[j], t, st[g].y);
+                st[g].S = fmaf(Sg[j], Pb[x], st[g].S);
+                const float tS = t * st[g].S;
+                acc[j] += fmaf(Pb[x], h, tS);
+                Pb[x] = fmaf(fmaf(-Sg[j], t, Sg[j]), tS, Pb[x]);
+                X[x] = xn;
+            }
+        }
+        const int jf = i + 2 * (G - 1);
+        if (jf >= 0 && jf <= JMAX) vg[jf * B] += acc[jf % W];
+        const int jr = i + G - 1;
+        if (CK && jr >= 0 && jr <= kRR - 1 && jr > tl) X[jr] = rs[jr * B];
+    }
+    if (full) {
+#pragma unroll
+        for (int j = 0; j < G - 1; ++j) vg[j * B] += acc[j % W];
+    }
+}
+
+// Normals of steps n and n+1 times sqrt(delta), for even n in ascending order,
+// in quads loaded four steps ahead (one 16-byte load where a row starts on such a
+// boundary: vec).
+template <bool PHILOX>
+struct TpbNormals {
+    const float *zp;
+    uint64_t seed, gpath;
+    int nmat;
+    bool vec;
+    float4 q, next;
+    __device__ __forceinline__ float4 quad(int i) const
+    {
+        if (PHILOX) {
+            float g[4];
+            normals_quad_f32(seed, gpath, (uint32_t)i, g);
+            return make_float4(g[0], g[1], g[2], g[3]);
+        }
+        if (vec) return __ldg(reinterpret_cast<const float4 *>(zp) + i);
+        auto at = [&](int n) { return n < nmat ? __ldg(zp + n) : 0.0f; };
+        return make_float4(at(4 * i), at(4 * i + 1), at(4 * i + 2), at(4 * i + 3));
+    }
+    __device__ __forceinline__ void start() { next = quad(0); }
+    __device__ __forceinline__ void pair(int n, float sqd, float &a, float &b)
+    {
+        if ((n & 3) == 0) {
+            q = next;
+            if (n + 4 < nmat) next = quad((n >> 2) + 1);
+        }
+        a = sqd * ((n & 2) ? q.z : q.x);
+        b = sqd * ((n & 2) ? q.w : q.y);
+    }
+};
+
+// Column sums of a warp's 32 paths: lane handles outputs k = lane, lane+32, ...,
+// rows t and t+16 in the halves of packed TwoSums (half the additions: 256 curves
+// x 16,384 paths 9.46 -> 9.19 ms); the (t+lane)&31 rotation keeps the lanes on 32
+// different banks. Adds sums and sums of squares into FP64 accumulators.
+template <int B>
+__device__ __forceinline__ void column_sums(int nn, const float *vg, int warp, int lane, double *acc, int nout, int off)
+{
+    for (int k = lane; k < nn; k += 32) {
+        const float *col = vg + k * B + warp * 32;
+        P2 a = 0, c = 0, a2 = 0;
+#pragma unroll 8
+        for (int t = 0; t < 16; ++t) {
+            const P2 x = p2(col[(t + lane) & 31], col[(t + 16 + lane) & 31]);
+            const P2 s = add2(a, x), v = sub2(s, a);
+            c = add2(c, add2(sub2(a, sub2(s, v)), sub2(x, v)));
+            a = s;
+            a2 = fma2(x, x, a2);
+        }
+        float s, s1, e, e1, q, q1;
+        unpack(a, s, s1);
+        unpack(c, e, e1);
+        unpack(a2, q, q1);
+        two_sum_acc(s, e, s1);
+        acc[off + k] += (double)s + (double)__fadd_rn(e, e1);
+        acc[nout + off + k] += (double)__fadd_rn(q, q1);
+    }
+}
+
+// NN, NMAT: the shape, or 0 for a shape at run time (any mode, `mode`; rate
+// checkpoints every m.ckpt steps, a multiple of kRG, or none).
+template <int NN, int NMAT, int B, bool PHILOX>
+__global__ void __launch_bounds__(B, 1)
+k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w, float *__restrict__ scr,
+      const double *__restrict__ vbar, int mode_arg)
+{
+    constexpr bool FIX = NN > 0;
+    constexpr int NW = B / 32;
+    const Mode mode = FIX ? Mode::Fused : (Mode)mode_arg;
+    const TpbLay Ly = FIX ? tpb_layout(NN, NMAT, Mode::Fused, B) : tpb_layout(m.nn, m.nmat, mode, B);
+    const int nn = Ly.nn, nmat = Ly.nmat, M = Ly.M, nout = Ly.nout;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float4 *kf_s = reinterpret_cast<float4 *>(smem + Ly.kf), *kr_s = reinterpret_cast<float4 *>(smem + Ly.kr);
+    float *il0_s = reinterpret_cast<float *>(smem + Ly.il0);
+    int *ost_s = reinterpret_cast<int *>(smem + Ly.ost);
+    float *okf_s = reinterpret_cast<float *>(smem + Ly.okf);
+    float *owf_s = reinterpret_cast<float *>(smem + Ly.owf);
+    F2 *okk_s = reinterpret_cast<F2 *>(smem + Ly.okk);
+    float *vg_s = reinterpret_cast<float *>(smem + Ly.vg);
+    double *acc_s = reinterpret_cast<double *>(smem + Ly.acc);
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < nmat + kFR * Ly.nf; i += B) {
+        const int k = i - nmat;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f), r = f;
+        if (k >= 0 && k < nn) {
+            const double sg = m.lamd[k] * m.sqdd, a = sg * 1.4426950408889634;
+            f = m.kc[k];
+            r = make_float4((float)a, (float)(-0.5 * a * sg), (float)sg, 0.f);
+        }
+        kf_s[i] = f;
+        kr_s[i] = r;
+    }
+    for (int i = tid; i <= M; i += B) ost_s[i] = m.opt_start[i];
+    for (int i = tid; i < m.nopt; i += B) {
+        okf_s[i] = m.optKf[i];
+        owf_s[i] = m.optWf[i];
+        okk_s[i] = f2_from(m.optKd[i] * m.deltad);
+    }
+    double *acc = acc_s + warp * 2 * nout;
+    const float delta = m.delta, sqd = m.sqd;
+    const float inv_d = (float)(1.0 / m.deltad), inv_sqd = (float)(1.0 / m.sqdd);
+    const float4 *kf = kf_s + nmat, *kr = kr_s + nmat;
+    float *vg0 = vg_s + kRG * B + tid;
+    const int ck = !FIX && m.ckpt > 0 ? m.ckpt : nmat, nck = (nmat - 1) / ck;
+    const int rows = Ly.s_ck + (FIX ? 0 : nck * kRR * Ly.nr);
+    float *sc = scr + (size_t)blockIdx.x * rows * B + tid;          // sc[row * B]
+    const bool vec = FIX ? NMAT % 4 == 0 : (nmat & 3) == 0;
+    const bool bsm = FIX ? 2 * (NN - NMAT) <= kRR * ((NN + kRR - 1) / kRR) : false;   // annuity factors in shared memory
+
+    const int units = m.nscen * w.items;
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const int scen = unit / w.items, item = unit % w.items;
+        __syncthreads();          // the previous unit's reads of il0/acc are done
+        for (int i = tid; i < kFR * Ly.nf; i += B) il0_s[i] = i < nn ? m.invL0f[scen * nn + i] : kPadIL;
+        for (int i = tid; i < NW * 2 * nout; i += B) acc_s[i] = 0.0;
+        const float vb = !FIX && mode == Mode::Backward ? (float)vbar[scen] : 1.0f;
+
+        for (int jb = 0; batch_left(w, item, jb) > 0; ++jb) {       // block-uniform
+            // one barrier per batch keeps the warps near each other in the code (instruction cache)
+            __syncthreads();
+            if ((tid & ~31) >= batch_left(w, item, jb)) continue;    // whole warps
+            const int64_t pc0 = (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths;
+            float V;
+            {
+                // ---- forward (path_calc_b1 :34-82) ----
+                const int64_t pc = tid < batch_left(w, item, jb) ? pc0 + tid : w.paths - 1;
+                const float *zp = PHILOX ? nullptr : z + pc * nmat;
+                F2 disc{1.0f, 0.0f};              // the discount product, rates 0 .. nmat-1 in order
+                float R[kFR];
+                float *sq = sc + (size_t)Ly.s_q * B;
+                float *Bst = bsm ? vg0 + M * B : sc + (size_t)Ly.s_b * B, *ILst = vg0;
+#pragma unroll 1
+                for (int ps = 0; ps < Ly.nf; ++ps) {
+                    const int LO = ps * kFR;
+                    const float *vin = sc + (size_t)(Ly.s_v + (2 * ps - 1) * nmat) * B;
+                    float *vo = sc + (size_t)(Ly.s_v + 2 * ps * nmat) * B;
+#pragma unroll
+                    for (int i = 0; i < kFR; ++i) R[i] = FIX ? il0_s[LO + i] : 0.0f;
+                    TpbNormals<PHILOX> zs{zp, seed, (uint64_t)(path0 + pc), nmat, vec};
+                    float nv0 = 0.0f, nv1 = 0.0f, nq0 = 0.0f, nq1 = 0.0f;
+                    if (ps == 0) {
+                        zs.start();
+                    } else {
+                        nv0 = vin[0];
+                        if (nmat > 1) nv1 = vin[B];
+                        if (!FIX) {
+                            nq0 = sq[0];
+                            if (nmat > 1) nq1 = sq[B];
+                        }
+                    }
+#pragma unroll 1
+                    for (int n = 0; n + 1 < nmat; n += 2) {
+                        float V0, V1, V0h, V1h, q0 = nq0, q1 = nq1;
+                        if (ps == 0) {
+                            zs.pair(n, sqd, q0, q1);
+                            V0 = FIX ? q0 : 0.0f;
+                            V1 = FIX ? q1 : 0.0f;
+                            if (!FIX) {
+                                sq[n * B] = q0;
+                                sq[(n + 1) * B] = q1;
+                            }
+                        } else {
+                            V0 = nv0;
+                            V1 = nv1;
+                            if (n + 2 < nmat) nv0 = vin[(n + 2) * B];
+                            if (n + 3 < nmat) nv1 = vin[(n + 3) * B];
+                            if (!FIX && n + 2 < nmat) nq0 = sq[(n + 2) * B];
+                            if (!FIX && n + 3 < nmat) nq1 = sq[(n + 3) * B];
+                        }
+                        if (n - LO < kFR - 1) {
+                            fwd_pair_block<!FIX>(R, kf - (n + 1) + LO, delta, n - LO, q0, q1, il0_s + LO, V0, V1, V0h, V1h);
+                        } else {                 // no rate of the pass moves
+                            V0h = V0;
+                            V1h = V1;
+                        }
+                        vo[n * B] = V0h;
+                        vo[(n + 1) * B] = V1h;
+                        vo[(nmat + n) * B] = V0;
+                        vo[(nmat + n + 1) * B] = V1;
+                        if (!FIX && nck > 0 && (n + 2) % ck == 0 && n + 2 < nmat) {
+                            // rates i <= n+2 are final from here on: only the others are saved
+                            float *cp = sc + (size_t)(Ly.s_ck + ((n + 2) / ck - 1) * kRR * Ly.nr + LO) * B;
+#pragma unroll
+                            for (int i = 0; i < kFR; ++i)
+                                if (LO + i > n + 2 && LO + i < kRR * Ly.nr) cp[i * B] = inv_rate<!FIX>(R[i], il0_s + LO + i) * inv_d;
+                        }
+                    }
+                    if (!FIX && (nmat & 1)) {
+                        const int n = nmat - 1;
+                        float V0 = nv0, V0h, q0 = nq0, q1;
+                        if (ps == 0) {
+                            zs.pair(n, sqd, q0, q1);
+                            sq[n * B] = q0;
+                        }
+                        V0h = V0;
+                        if (n - LO < kFR - 1) fwd_one_block<true>(R, kf - (n + 1) + LO, delta, q0, il0_s + LO, V0, V0h);
+                        vo[n * B] = V0h;
+                        vo[(nmat + n) * B] = V0;
+                    }
+#pragma unroll
+                    for (int i = 0; i < kFR; ++i) {
+                        const float il = FIX ? R[i] : il0_s[LO + i] * ex2_ulp(-R[i]);
+                        sc[(Ly.s_x + LO + i) * B] = il * inv_d;
+                        if (LO + i < nmat)
+                            disc = FIX ? f2_mul(disc, bond_ratio(il, delta)) : f2_mul(disc, bond_ratio2(il, delta));
+                        else if (LO + i < nn)
+                            ILst[(LO + i - nmat) * B] = il;
+                    }
+                }
+                // ---- payoff (portfolio_b :133-171, :186-197) and the annuity adjoint ----
+                unsigned long long mask;
+                float dsc;
+                V = payoff_forward_staged<B, !FIX>(M, disc, delta, ost_s, okk_s, owf_s, &dsc, Bst, ILst, &mask);
+                if (FIX || mode != Mode::Forward) {
+                    payoff_adjoint_stage<B>(M, vb, dsc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
+#pragma unroll 4
+                    for (int i = 0; i < M; ++i) sc[(Ly.s_d + nmat + i) * B] = ILst[i * B];
+                }
+            }
+            if (FIX || mode != Mode::Forward) {
+#pragma unroll 8
+                for (int k = 0; k < kRR * Ly.nr; ++k) vg0[k * B] = 0.0f;
+
+                // ---- reverse: the blocks from the top, each over the steps with an active cell in it ----
+                float *su = sc + (size_t)Ly.s_s * B;
+                const float *sq = sc + (size_t)Ly.s_q * B;
+                const float nvs = -vb * V;
+#pragma unroll 1
+                for (int b = Ly.nr - 1; b >= 0; --b) {
+                    const int LO = b * kRR;
+                    const bool top = b == Ly.nr - 1;
+                    const float *vt = sc + (size_t)(Ly.s_v + b * nmat) * B;
+                    float X[kRR], Pb[kRR];
+#pragma unroll
+                    for (int i = 0; i < kRR; ++i) X[i] = sc[(Ly.s_x + LO + i) * B];
+                    if (FIX && LO >= NMAT) {
+#pragma unroll
+                        for (int i = 0; i < kRR; ++i) Pb[i] = sc[(Ly.s_d + LO + i) * B];
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < kRR; ++i) {
+                            Pb[i] = nvs * rcp_approx(X[i] + 1.0f);
+                            if (!FIX && LO + i >= nmat) Pb[i] = LO + i < nn ? sc[(Ly.s_d + LO + i) * B] : 0.0f;
+                        }
+                    }
+                    // the steps above a whole number of groups, one at a time; then the groups of kRG
+                    auto back = [&](int t, const float *&rs, int &tl) {   // the rates to take back at time t
+                        rs = sc;
+                        tl = kRR;
+                        if (!FIX && nck > 0 && t % ck == 0 && t >= ck) {
+                            rs = sc + (size_t)(Ly.s_ck + (t / ck - 1) * kRR * Ly.nr + LO) * B;
+                            tl = t - LO;
+                        }
+                    };
+                    const float *rs;
+                    int tl, n = nmat - 1;
+                    if (!FIX) {
+#pragma unroll 1
+                        for (; (n + 1) % kRG != 0; --n) {
+                            if (LO + kRR - 1 <= n) continue;
+                            TpbStep s1[1] = {{(vt[n * B] + sq[n * B]) * inv_sqd, top ? 0.0f : su[n * B]}};
+                            back(n, rs, tl);
+                            rev_block<B, 1, true>(X, Pb, s1, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
+                            su[n * B] = s1[0].S;
+                        }
+                    }
+                    while (LO + kRR - 1 <= n - kRG + 1) n -= kRG;
+                    float nv[kRG], ns[kRG];       // the next group's restart sums, loaded a group ahead
+                    if (n > 0) {
+#pragma unroll
+                        for (int g = 0; g < kRG; ++g) {
+                            nv[g] = FIX ? vt[(n - g) * B] : vt[(n - g) * B] + sq[(n - g) * B];
+                            ns[g] = top ? 0.0f : su[(n - g) * B];
+                        }
+                    }
+#pragma unroll 1
+                    for (; n > 0; n -= kRG) {
+                        TpbStep st[kRG];
+#pragma unroll
+                        for (int g = 0; g < kRG; ++g) st[g] = {nv[g] * inv_sqd, ns[g]};
+                        if (n - kRG > 0) {
+#pragma unroll
+                            for (int g = 0; g < kRG; ++g) {
+                                nv[g] = FIX ? vt[(n - kRG - g) * B] : vt[(n - kRG - g) * B] + sq[(n - kRG - g) * B];
+                                ns[g] = top ? 0.0f : su[(n - kRG - g) * B];
+                            }
+                        }
+                        back(n - kRG + 1, rs, tl);
+                        rev_block<B, kRG, !FIX>(X, Pb, st, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
+                        if (b > 0) {
+#pragma unroll
+                            for (int g = 0; g < kRG; ++g) su[(n - g) * B] = st[g].S;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < kRR; ++i) sc[(Ly.s_d + LO + i) * B] = Pb[i] * il0_s[LO + i];
+                }
+            }
+
+            // ---- cross-path reduction of this batch ----
+            const bool active = tid < batch_left(w, item, jb);
+            if (FIX || mode != Mode::Backward) {
+                const float v = active ? V : 0.0f;
+                const float s1 = warp_sum(v), s2 = warp_sum(v * v);
+                if (lane == 0) {
+                    acc[0] += (double)s1;
+                    acc[nout] += (double)s2;
+                }
+            }
+            if (FIX || mode != Mode::Forward) {
+                const int off = FIX || mode == Mode::Fused ? 1 : 0;
+                float *vgw = vg_s + kRG * B;
+                if (!active) {
+#pragma unroll 1
+                    for (int k = 0; k < nn; ++k) vg0[k * B] = 0.0f;
+                }
+                __syncwarp();
+                column_sums<B>(nn, vgw, warp, lane, acc, nout, off + nn);
+                __syncwarp();
+#pragma unroll 16
+                for (int i = 0; i < nn; ++i) vg0[i * B] = active ? sc[(Ly.s_d + i) * B] : 0.0f;
+                __syncwarp();
+                column_sums<B>(nn, vgw, warp, lane, acc, nout, off);
+                __syncwarp();
+            }
+        }
+
+        __syncthreads();
+        const int voff = FIX || mode == Mode::Fused ? 1 + nn : nn;
+        for (int o = tid; o < 2 * nout; o += B) {
+            double s2 = 0.0;
+#pragma unroll
+            for (int q = 0; q < NW; ++q) s2 += acc_s[q * 2 * nout + o];
+            // vegas per lambda: sqrt(delta) times those per sigma, delta times their squares
+            if ((FIX || mode != Mode::Forward) && (o < nout ? o >= voff : o - nout >= voff)) s2 *= o < nout ? m.sqdd : m.deltad;
+            w.partial[(size_t)unit * 2 * nout + o] = s2;
+        }
+    }  // units
+}
+
+template <int NN, int NMAT, int B>
+cudaError_t launch_tpb(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox, const Work &w,
+                       float *scr, const double *vbar, cudaStream_t s)
+{
+    const int bytes = tpb_layout(m.nn, m.nmat, mode, B).bytes;
+    auto kern = philox ? k_tpb<NN, NMAT, B, true> : k_tpb<NN, NMAT, B, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    kern<<<(unsigned)w.grid, B, bytes, s>>>(m, z, seed, path0, w, scr, vbar, (int)mode);
+    return cudaGetLastError();
+}
+
+template <int NN, int NMAT, int B>
+cudaError_t occ_tpb(int nn, int nmat, Mode mode, bool philox, int *blocks)
+{
+    const int bytes = tpb_layout(nn, nmat, mode, B).bytes;
+    auto kern = philox ? k_tpb<NN, NMAT, B, true> : k_tpb<NN, NMAT, B, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, B, bytes);
+}
+
+}  // namespace
+}  // namespace lmm

@@ -49,6 +49,8 @@
 // fixed order, so results are bit-reproducible.
 #include "lmm_device.cuh"
 
+#include "lmm_f32_payoff.cuh"
+
 #include <cuda_bf16.h>
 
 // Threads per block of the fused kernel: 254 registers per thread leave room
@@ -194,20 +196,6 @@ struct TppLayout {
     static constexpr int acc = align16(vc + vc_bytes);               // double[NW][2*NOUT]
     static constexpr int bytes = acc + 8 * NW * 2 * NOUT;
 };
-
-// Paths of batch jb of an item (0 or less: there is none).
-__device__ __forceinline__ int batch_left(const Work &w, int item, int jb)
-{
-    const int64_t p0 = (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths;
-    const int64_t iend = min((int64_t)(item + 1) * w.ipaths, w.paths);
-    return (int)max(min(iend - p0, (int64_t)w.bpaths), (int64_t)0);
-}
-
-// A batch's paths, kept per warp in shared memory (batch_left): the step loops
-// have no register to spare for it. The batch runs in the first threads of the
-// block, whole warps.
-__device__ __forceinline__ int read_left(const int *left) { return *reinterpret_cast<const volatile int *>(left); }
-__device__ __forceinline__ void sync_batch(const int *left) { sync_threads((read_left(left) + 31) & ~31); }
 
 __device__ __forceinline__ float pick4(const float4 &q, int j)
 {
@@ -387,13 +375,9 @@ __device__ __forceinline__ void kahan_add_bf16c(float &s, unsigned short &cb, fl
 // 1: the reverse windows keep d = -delta*lambda_k beside each constant of
 // their ring (one multiply per position, shared by the G cells of the
 // position), and the cell forms lambda(1 - delta t) as one FMA,
-// fma(d, t, lambda), instead of an FMA and a multiply. Per kernel: k_tpp,
-// k_tps, k_tpq.
+// fma(d, t, lambda), instead of an FMA and a multiply. Per kernel: k_tpp, k_tpq.
 #ifndef LMM_TPP_DCONST
 #define LMM_TPP_DCONST 1
-#endif
-#ifndef LMM_TPS_DCONST
-#define LMM_TPS_DCONST 1
 #endif
 #ifndef LMM_TPQ_DCONST
 #define LMM_TPQ_DCONST 0
@@ -486,46 +470,6 @@ __device__ __forceinline__ void rev_group_window(float (&IL)[NN], float (&Pb)[NN
     }
 }
 
-// Portfolio value, portfolio_b :133-171 and :186-197, from the inverse rates.
-// The factors 1/(1+delta L) come from t = 1/(IL + delta) (MUFU reciprocal,
-// within 1 ulp) as 1 - delta t while delta L < 1 (within 0.5 + delta L ulp:
-// about 0.5 ulp for ordinary rates) and as IL t above (within 2.5 ulp). The
-// discount and annuity products, the annuity sum, the swap values and the
-// payoff sum are double-FP32 (F2, lmm_device.cuh): FP64-like products on
-// the FP32 pipe (FP64 products cost 10% of the fused kernel's time on
-// GB300). Returns the discounted value; *disc_out receives the discount
-// factor, *mask_out which swaptions (in grouped order) paid, and Bst[m*B] (if
-// given) the annuity factors B[m] of :139 rounded to FP32, for the adjoint.
-// payoff_forward_staged is its annuity part, from the discount product
-// `disc` and the M annuity rates staged in ILst[m*B].
-template <int M, int B>
-__device__ __forceinline__ float payoff_forward_staged(F2 disc, float delta, const int *ost, const F2 *oKd,
-                                                       const float *oWf, float *disc_out, float *Bst,
-                                                       const float *ILst, unsigned long long *mask_out)
-{
-    F2 b{1.0f, 0.0f}, sb{0.0f, 0.0f}, vs{0.0f, 0.0f};
-    unsigned long long mask = 0ull;
-#pragma unroll 1
-    for (int m = 0; m < M; ++m) {
-        b = f2_mul(b, bond_ratio(ILst[m * B], delta));
-        sb = f2_add(sb, b);                                   // annuity / delta
-        if (Bst) Bst[m * B] = b.hi;
-        const int o1 = ost[m + 1];
-#pragma unroll 1
-        for (int o = ost[m]; o < o1; ++o) {
-            const float sw = f2_swap_value(oKd[o], sb, b);
-            if (sw < 0.0f) {
-                vs = f2_add(vs, (-100.0f * sw) * oWf[o]);
-                mask |= 1ull << o;
-            }
-        }
-    }
-    *disc_out = disc.hi;
-    *mask_out = mask;
-    const F2 v = f2_mul(vs, disc);
-    return __fadd_rn(v.hi, v.lo);
-}
-
 template <int NN, int NMAT, int B>
 __device__ __forceinline__ float payoff_forward(const float (&IL)[NN], float delta, const int *ost,
                                                 const F2 *oKd, const float *oWf, float *disc_out,
@@ -540,42 +484,7 @@ __device__ __forceinline__ float payoff_forward(const float (&IL)[NN], float del
     // (instruction cache).
 #pragma unroll
     for (int m = 0; m < M; ++m) ILst[m * B] = IL[NMAT + m];
-    return payoff_forward_staged<M, B>(disc, delta, ost, oKd, oWf, disc_out, Bst, ILst, mask_out);
-}
-
-// Payoff adjoint, portfolio_b :173-184 (with the rate and its adjoint kept
-// apart) and :199-209, seeded with vbar = dOut/dV. Writes the log-adjoints
-// Pb[i] = L_i dOut/dL_i of the terminal rates. Bst[m*B] holds B[m] from the
-// forward: rebuilding B[m-1] = B[m](1 + delta L) backwards from the last,
-// smallest factor would underflow FP32 on paths whose rates grow large.
-template <int NN, int NMAT, int B>
-__device__ __forceinline__ void payoff_adjoint_stage(float vbar, float disc, const float *Bst, float *ILst,
-                                                     unsigned long long mask, float delta, const int *ost,
-                                                     const float *oKf, const float *oWf)
-{
-    constexpr int M = NN - NMAT;
-    const float scale = -vbar * disc * delta;
-    float Sb = 0.0f, Bb = 0.0f;
-    // Rolled over the rates staged by payoff_forward; each staged rate is
-    // replaced by its log-adjoint, copied into Pb[] afterwards.
-#pragma unroll 1
-    for (int m = M - 1; m >= 0; --m) {
-        const float il = ILst[m * B];
-        const float t = rcp_approx(il + delta);               // L/(1+delta L)
-        const float r = bond_ratio_t(il, delta, t);
-        const float Bm = Bst[m * B];
-        const int o1 = ost[m + 1];
-#pragma unroll 1
-        for (int o = ost[m]; o < o1; ++o) {
-            if ((mask >> o) & 1ull) {
-                Sb -= (100.0f * oKf[o]) * oWf[o];
-                Bb -= 100.0f * oWf[o];
-            }
-        }
-        Bb = fmaf(delta, Sb, Bb);
-        ILst[m * B] = scale * Bb * Bm * t;
-        Bb *= r;
-    }
+    return payoff_forward_staged<B>(M, disc, delta, ost, oKd, oWf, disc_out, Bst, ILst, mask_out);
 }
 
 template <int NN, int NMAT, int B>
@@ -585,7 +494,7 @@ __device__ __forceinline__ void payoff_adjoint(const float (&IL)[NN], float (&Pb
                                                const int *ost, const float *oKf, const float *oWf)
 {
     constexpr int M = NN - NMAT;
-    payoff_adjoint_stage<NN, NMAT, B>(vbar, disc, Bst, ILst, mask, delta, ost, oKf, oWf);
+    payoff_adjoint_stage<B>(M, vbar, disc, Bst, ILst, mask, delta, ost, oKf, oWf);
 #pragma unroll
     for (int m = 0; m < M; ++m) Pb[NMAT + m] = ILst[m * B];
     const float vs = -vbar * V * delta;
@@ -856,399 +765,6 @@ k_tpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             w.partial[(size_t)unit * 2 * NOUT + o] = s;
         }
     }  // units
-}
-
-// ---------------------------------------------------------------------------
-// k_tps: the fused kernel with the reverse sweep split over the two rate
-// halves, for more warps per SM.
-//
-// In k_tpp the reverse sweep holds all NN inverse rates and NN log-adjoints
-// in registers (232 per thread), which allows 8 warps per SM: two per
-// scheduler, too few to cover the cells' ex2 -> rcp dependency chains. The
-// forward needs only the NN rates. Here the reverse runs as two passes over
-// the halves of the rates, one after the other in the same thread:
-//   R1: rates H..NN-1 for every step, starting each step from the full drift
-//       sum (saved by the forward, shared memory) and an empty suffix sum;
-//       it leaves, per step, the suffix sum at rate H in the scratch;
-//   R2: rates 0..H-1 for every step, starting each step from the forward's
-//       drift sum at rate H-1 (scratch) and R1's suffix sum.
-// The lower half's terminal rates wait in the scratch during R1, the upper
-// half's deltas during R2, so at most H rates and H log-adjoints are live:
-// about 150 registers, 12 warps per SM (three per scheduler). The cells, the
-// step windows (G = 4 reverse steps per body, constants and vega partial sums
-// in rings), the payoff and the reductions are those of k_tpp; a vega row
-// takes read-modify-writes from both passes.
-// The scratch (per block of the wave, FP32, [row][B] so that a warp's 32
-// paths are contiguous): the drift sums at rate H-1 [NMAT], R1's suffix sums
-// at rate H [NMAT], the lower half's terminal inverse rates [H] and the upper
-// half's deltas [NN-H]. It is written and read back by the same thread within
-// one batch of B paths, and stays in L2 (about 37 MB per wave at NN = 80).
-// ---------------------------------------------------------------------------
-#ifndef LMM_TPS_BLOCK
-#define LMM_TPS_BLOCK 384
-#endif
-// Barriers in k_tps's step loops (0: none; they keep the warps of a block on
-// the same stretch of code; every array the loops touch is per thread).
-#ifndef LMM_TPS_SYNC
-#define LMM_TPS_SYNC LMM_TPP_SYNC
-#endif
-// 1: k_tps reads the per-maturity constants from the kernel-parameter bank;
-// 0: from shared memory.
-#ifndef LMM_TPS_KCPARAM
-#define LMM_TPS_KCPARAM 1
-#endif
-// Forward step pairs between block barriers, reverse chunk lengths and the
-// constant prefetch distance of k_tps, with normals from memory and with
-// Philox normals (the k_tpp kernels keep LMM_TPP_*). GB300, with the shared
-// forward reciprocals: 4,194,304 paths, a forward barrier every 2, 4, 8 pairs
-// or once per batch (20 pairs) 10.01, 9.88, 9.86, 9.83 ms; constants at the
-// position of use 9.98 against 9.88 (one ahead); 16.8M Philox paths, 42.35 ms
-// as LMM_TPP_*, 41.54 with 2-position reverse chunks and constants one ahead,
-// 41.33 / 41.24 / 41.15 / 40.81 with a forward barrier every 2 / 4 / 8 pairs /
-// once per batch. 256 curves x 262,144 paths with these settings: 163.5 ms
-// (166.2 before). Reverse chunks of one position (the body left right below
-// the lowest active position): 9.80 -> 9.78 ms, Philox 40.62 -> 40.58 ms.
-#ifndef LMM_TPS_FSYNC
-#define LMM_TPS_FSYNC 20
-#endif
-// Reverse step groups between block barriers. GB300: every group, every
-// second, fourth, tenth: 4,194,304 paths 9.84, 9.81, 9.83, 9.92 ms; 16.8M
-// Philox paths 40.84 / 40.62 ms (every group / every second).
-#ifndef LMM_TPS_RSYNC
-#define LMM_TPS_RSYNC 2
-#endif
-#ifndef LMM_TPS_FSYNC_PHILOX
-#define LMM_TPS_FSYNC_PHILOX 20
-#endif
-#ifndef LMM_TPS_RCHUNK
-#define LMM_TPS_RCHUNK 1
-#endif
-#ifndef LMM_TPS_RCHUNK_PHILOX
-#define LMM_TPS_RCHUNK_PHILOX 1
-#endif
-#ifndef LMM_TPS_PREF
-#define LMM_TPS_PREF LMM_TPP_PREF
-#endif
-#ifndef LMM_TPS_PREF_PHILOX
-#define LMM_TPS_PREF_PHILOX 1
-#endif
-
-template <int NN, int NMAT>
-struct TpsLayout {
-    static constexpr int B = LMM_TPS_BLOCK;
-    static constexpr int NW = B / 32;
-    static constexpr int H = NN / 2;
-    static constexpr int M = NN - NMAT;
-    static constexpr int VPAD = 4;
-    static constexpr int NOUT = 1 + 2 * NN;
-    static constexpr int il0 = 0;                                    // float[NN]
-    static constexpr int ost = align16(il0 + 4 * NN);                // int[M+1]
-    static constexpr int okf = align16(ost + 4 * (M + 1));           // float[kMaxNopt]
-    static constexpr int owf = align16(okf + 4 * kMaxNopt);          // float[kMaxNopt]
-    static constexpr int okk = align16(owf + 4 * kMaxNopt);          // F2[kMaxNopt]
-    static constexpr int vt = align16(okk + 8 * kMaxNopt);           // float[NMAT][B] full drift sums
-    static constexpr int vg = vt + 4 * NMAT * B;                     // float[VPAD+NN][B] vega rows
-    static constexpr int kc = align16(vg + 4 * (VPAD + NN) * B);     // float4[NMAT+NN] (!LMM_TPS_KCPARAM)
-    static constexpr int acc = align16(kc + (LMM_TPS_KCPARAM ? 0 : 16 * (NMAT + NN)));   // double[NW][2*NOUT]
-    static constexpr int bytes = acc + 8 * NW * 2 * NOUT;
-    // scratch rows per block
-    static constexpr int s_v = 0, s_s = NMAT, s_il = 2 * NMAT, s_d = 2 * NMAT + H, rows = 2 * NMAT + NN;
-    static_assert(NN % 2 == 0 && NMAT == H, "the upper half is the annuity rates");
-};
-
-
-// Reverse steps n .. n-G+1 over one half of the rates, rates LO .. LO+H-1 held
-// in X[], Pb[] at local positions 0 .. H-1: rev_group_window on a block of
-// rates. st[0].kc and st[0].vg point at step n's constants and vega rows of
-// the block's local position 0. The upper half (LO > 0) is active in every
-// step (n < NMAT <= LO), so its body runs to the last position and flushes
-// the vega slots of positions 0 .. G-2, which hold its cells' sums; the lower
-// half (LO = 0) leaves the body as rev_group_window does.
-template <int H, int LO, int B, int G, int CH, int P>
-__device__ __forceinline__ void rev_half_window(float (&X)[H], float (&Pb)[H], RevStep (&st)[G], float delta,
-                                                int n)
-{
-    constexpr int JMAX = H + G - 2;
-    constexpr int W = 2 * G - 1 + P;
-    const float4 *kc = st[0].kc;
-    float *vg = st[0].vg;
-    float4 C[W];
-    float D[W];
-    float A[W];
-#pragma unroll
-    for (int j = H - P; j <= JMAX; ++j) {
-        C[j % W] = kc[j];
-        D[j % W] = -delta * C[j % W].w;
-        if (j >= H) A[j % W] = 0.0f;
-    }
-    const int imin = n - 2 * G + 3 - LO;     // lowest local position with an active cell
-#pragma unroll
-    for (int q = 0; q * CH < H + G - 1; ++q) {
-        const int top = H - 1 - q * CH;
-        if (LO == 0 && top < imin) return;
-#pragma unroll
-        for (int i = top; i > top - CH && i >= -(G - 1); --i) {
-            if (i - P >= (LO > 0 ? 0 : 1)) {
-                C[(i - P) % W] = kc[i - P];
-                D[(i - P) % W] = -delta * C[(i - P) % W].w;
-            }
-            if (i >= (LO > 0 ? 0 : 1)) A[i % W] = 0.0f;
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                if (i + g >= (LO > 0 ? 0 : 1) && i + g <= H - 1) {
-                    const int j = i + 2 * g;
-                    rev_cell<H, LMM_TPS_DCONST != 0>(X, Pb, st[g], i + g, C[j % W], D[j % W], A[j % W], delta);
-                }
-            }
-            const int jf = i + 2 * (G - 1);
-            if (jf >= (LO > 0 ? 0 : 1) && jf <= JMAX) vg[jf * B] += A[jf % W];
-        }
-    }
-    if (LO > 0) {
-#pragma unroll
-        for (int j = 0; j < G - 1; ++j) vg[j * B] += A[j % W];
-    }
-}
-
-template <bool RAGGED>
-__device__ __forceinline__ void tps_sync(const int *left)
-{
-    if (RAGGED)
-        sync_batch(left);
-    else
-        __syncthreads();
-}
-
-// RAGGED: batches of w.bpaths paths and a last partial one per item, each run
-// by the warps that have paths. Otherwise whole batches of the block (w.ppt per
-// item), in which every warp runs: the ragged batches' bookkeeping costs 40
-// more bytes of spills and 4% of a full batch's time (curves 10.48 -> 10.94 ms),
-// so the plan takes it only where it saves more.
-template <int NN, int NMAT, bool PHILOX, bool RAGGED>
-__global__ void __launch_bounds__(LMM_TPS_BLOCK, 384 / LMM_TPS_BLOCK)
-k_tps(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w,
-      float *__restrict__ scr, const __grid_constant__ TppConst<NN, NMAT> kp)
-{
-    using Lay = TpsLayout<NN, NMAT>;
-    constexpr int B = Lay::B, H = Lay::H, M = Lay::M, NOUT = Lay::NOUT, PAD = NMAT;
-    constexpr int G = LMM_TPP_SKEW, RCH = PHILOX ? LMM_TPS_RCHUNK_PHILOX : LMM_TPS_RCHUNK;
-    constexpr int PF = PHILOX ? LMM_TPS_PREF_PHILOX : LMM_TPS_PREF;
-    static_assert(NMAT % 4 == 0 && NMAT % G == 0, "normals in quads, reverse steps in groups");
-    static_assert(RCH - 1 <= Lay::VPAD, "the windows' spare vega rows lie inside the table");
-    extern __shared__ __align__(16) unsigned char smem[];
-    float *il0_s = reinterpret_cast<float *>(smem + Lay::il0);
-    int *ost_s = reinterpret_cast<int *>(smem + Lay::ost);
-    float *okf_s = reinterpret_cast<float *>(smem + Lay::okf);
-    float *owf_s = reinterpret_cast<float *>(smem + Lay::owf);
-    F2 *okk_s = reinterpret_cast<F2 *>(smem + Lay::okk);
-    float *vt_s = reinterpret_cast<float *>(smem + Lay::vt);
-    float *vg_s = reinterpret_cast<float *>(smem + Lay::vg);
-    double *acc_s = reinterpret_cast<double *>(smem + Lay::acc);
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ int left_s[Lay::NW];
-    for (int i = tid; i <= M; i += B) ost_s[i] = m.opt_start[i];
-    for (int i = tid; i < m.nopt; i += B) {
-        okf_s[i] = m.optKf[i];
-        owf_s[i] = m.optWf[i];
-        okk_s[i] = f2_from(m.optKd[i] * m.deltad);
-    }
-    double *acc = acc_s + warp * 2 * NOUT;
-    const float delta = m.delta, sqd = m.sqd;
-    float4 *kc_s = reinterpret_cast<float4 *>(smem + Lay::kc);
-    if (!LMM_TPS_KCPARAM) {
-        for (int i = tid; i < PAD + NN; i += B) kc_s[i] = kp.v[i];
-    }
-    const float4 *kc0 = (LMM_TPS_KCPARAM ? kp.v : kc_s) + PAD;
-    float *vg0 = vg_s + Lay::VPAD * B + tid;
-    float *vt0 = vt_s + tid;
-    float *sc = scr + (size_t)blockIdx.x * Lay::rows * B + tid;    // sc[row * B]
-
-    const int units = m.nscen * w.items;
-    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
-        const int scen = unit / w.items, item = unit % w.items;
-        __syncthreads();          // the previous unit's reads of il0/acc are done
-        for (int i = tid; i < NN; i += B) il0_s[i] = m.invL0f[scen * NN + i];
-        for (int i = tid; i < Lay::NW * 2 * NOUT; i += B) acc_s[i] = 0.0;
-        __syncthreads();
-
-        for (int jb = 0; RAGGED || jb < w.ppt; ++jb) {
-            int64_t pl;
-            if (RAGGED) {
-                const int left = batch_left(w, item, jb);
-                if ((tid & ~31) >= left) break;      // whole warps; later batches are no larger
-                if (lane == 0) left_s[warp] = left;
-                __syncwarp();
-                pl = tid < left ? (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths + tid : w.paths;
-            } else {
-                const int64_t p0 = ((int64_t)item * w.ppt + jb) * B;
-                if (p0 >= w.paths) break;            // block-uniform
-                pl = p0 + tid;
-            }
-            const bool act = pl < w.paths;
-            const int64_t pc = act ? pl : w.paths - 1;
-            const float *zp = PHILOX ? nullptr : z + pc * NMAT;
-            const uint64_t gpath = (uint64_t)(path0 + pc);
-
-            float disc = 1.0f, V, vs;
-            float Xu[H], Pu[H];       // upper half: inverse rates and log-adjoints
-            unsigned long long mask = 0ull;
-            {
-                // ---- forward over all NN rates (path_calc_b1 :34-82) ----
-                float IL[NN];
-#pragma unroll
-                for (int i = 0; i < NN; ++i) IL[i] = il0_s[i];
-                float4 zq, zq_next = zquad<PHILOX, NMAT>(zp, seed, gpath, 0);
-                for (int n = 0; n < NMAT; n += 2) {
-                    if (LMM_TPS_SYNC && (n % (2 * (PHILOX ? LMM_TPS_FSYNC_PHILOX : LMM_TPS_FSYNC))) == 0)
-                        tps_sync<RAGGED>(left_s + warp);
-                    if ((n & 3) == 0) {
-                        zq = zq_next;
-                        if ((n >> 2) + 1 < NMAT / 4) zq_next = zquad<PHILOX, NMAT>(zp, seed, gpath, (n >> 2) + 1);
-                    }
-                    const float sqez0 = sqd * ((n & 2) ? zq.z : zq.x);
-                    const float sqez1 = sqd * ((n & 2) ? zq.w : zq.y);
-                    float V0, V1, V0c, V1c;
-                    fwd_pair_window_cap<NN, LMM_TPP_CHUNK, PF, H - 1>(IL, kc0 - (n + 1), sqez0, sqez1,
-                                                                                delta, n, V0, V1, V0c, V1c);
-                    vt0[n * B] = V0;
-                    vt0[(n + 1) * B] = V1;
-                    sc[(Lay::s_v + n) * B] = V0c;
-                    sc[(Lay::s_v + n + 1) * B] = V1c;
-                }
-                // ---- payoff (portfolio_b :133-171, :186-197) and the annuity adjoint ----
-                float *Bst = vg0;
-                float *ILst = vg0 + M * B;
-                V = payoff_forward<NN, NMAT, B>(IL, delta, ost_s, okk_s, owf_s, &disc, Bst, ILst, &mask);
-                payoff_adjoint_stage<NN, NMAT, B>(1.0f, disc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
-#pragma unroll
-                for (int i = 0; i < H; ++i) {
-                    Xu[i] = IL[H + i];
-                    Pu[i] = ILst[i * B];
-                    sc[(Lay::s_il + i) * B] = IL[i];     // the lower half waits in the scratch
-                }
-                vs = -V * delta;
-            }
-#pragma unroll
-            for (int k = 0; k < NN; ++k) vg0[k * B] = 0.0f;
-
-            // ---- R1: the upper half's reverse, every step ----
-            for (int n = NMAT - 1; n > 0; n -= G) {
-                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) tps_sync<RAGGED>(left_s + warp);
-                RevStep st[G];
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const int mm = n - g;
-                    st[g].sqez = 0.0f;
-                    st[g].V = vt0[mm * B];
-                    st[g].S = 0.0f;
-                    st[g].kc = kc0 - (mm + 1) + H;
-                    st[g].vg = vg0 + (H - mm - 1) * B;
-                }
-                rev_half_window<H, H, B, G, RCH, PF>(Xu, Pu, st, delta, n);
-#pragma unroll
-                for (int g = 0; g < G; ++g) sc[(Lay::s_s + n - g) * B] = st[g].S;
-            }
-#pragma unroll
-            for (int i = 0; i < H; ++i) sc[(Lay::s_d + i) * B] = Pu[i] * il0_s[H + i];
-
-            // ---- R2: the lower half's reverse ----
-            float Xl[H], Pl[H];
-#pragma unroll
-            for (int i = 0; i < H; ++i) {
-                Xl[i] = sc[(Lay::s_il + i) * B];
-                Pl[i] = vs * rcp_approx(Xl[i] + delta);
-            }
-            float nv[G], ns[G];       // the next group's restart sums, loaded a group ahead
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                nv[g] = sc[(Lay::s_v + NMAT - 1 - g) * B];
-                ns[g] = sc[(Lay::s_s + NMAT - 1 - g) * B];
-            }
-            for (int n = NMAT - 1; n > 0; n -= G) {
-                if (LMM_TPS_SYNC && ((NMAT - 1 - n) / G) % LMM_TPS_RSYNC == 0) tps_sync<RAGGED>(left_s + warp);
-                RevStep st[G];
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const int mm = n - g;
-                    st[g].sqez = 0.0f;
-                    st[g].V = nv[g];
-                    st[g].S = ns[g];
-                    st[g].kc = kc0 - (mm + 1);
-                    st[g].vg = vg0 - (mm + 1) * B;
-                }
-                if (n - G > 0) {
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        nv[g] = sc[(Lay::s_v + n - G - g) * B];
-                        ns[g] = sc[(Lay::s_s + n - G - g) * B];
-                    }
-                }
-                rev_half_window<H, 0, B, G, RCH, PF>(Xl, Pl, st, delta, n);
-            }
-
-            // ---- cross-path reduction of this batch of B paths ----
-            const bool active = RAGGED ? tid < read_left(left_s + warp) : act;
-            {
-                const float v = active ? V : 0.0f;
-                const float s1 = warp_sum(v), s2 = warp_sum(v * v);
-                if (lane == 0) {
-                    acc[0] += (double)s1;
-                    acc[NOUT] += (double)s2;
-                }
-            }
-            float *vgw = vg_s + Lay::VPAD * B;
-            if (!active) {
-#pragma unroll
-                for (int k = 0; k < NN; ++k) vg0[k * B] = 0.0f;
-            }
-            __syncwarp();
-            column_reduce<NN, B>(vgw, warp, lane, acc, NOUT, 1 + NN);
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < H; ++i) {
-                vg0[i * B] = active ? Pl[i] * il0_s[i] : 0.0f;
-                vg0[(H + i) * B] = active ? sc[(Lay::s_d + i) * B] : 0.0f;
-            }
-            __syncwarp();
-            column_reduce<NN, B>(vgw, warp, lane, acc, NOUT, 1);
-            __syncwarp();
-        }
-
-        __syncthreads();
-        for (int o = tid; o < 2 * NOUT; o += B) {
-            double s2 = 0.0;
-#pragma unroll
-            for (int q = 0; q < Lay::NW; ++q) s2 += acc_s[q * 2 * NOUT + o];
-            w.partial[(size_t)unit * 2 * NOUT + o] = s2;
-        }
-    }  // units
-}
-
-template <int NN, int NMAT, bool PHILOX, bool RAGGED>
-cudaError_t launch_tps(const DevModel &m, const float *z, uint64_t seed, int64_t path0, const Work &w,
-                       float *scr, cudaStream_t s)
-{
-    using Lay = TpsLayout<NN, NMAT>;
-    auto kern = k_tps<NN, NMAT, PHILOX, RAGGED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::bytes);
-    if (e != cudaSuccess) return e;
-    TppConst<NN, NMAT> kp;
-    for (int i = 0; i < NMAT + NN; ++i)
-        kp.v[i] = i < NMAT ? make_float4(0.f, 0.f, 0.f, 0.f) : m.kc_host[i - NMAT];
-    const unsigned grid = (unsigned)(w.grid > 0 ? w.grid : (int64_t)m.nscen * w.items);
-    kern<<<grid, Lay::B, Lay::bytes, s>>>(m, z, seed, path0, w, scr, kp);
-    return cudaGetLastError();
-}
-
-template <int NN, int NMAT, bool PHILOX, bool RAGGED>
-cudaError_t occ_tps(int *blocks)
-{
-    using Lay = TpsLayout<NN, NMAT>;
-    auto kern = k_tps<NN, NMAT, PHILOX, RAGGED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::bytes);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, Lay::B, Lay::bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -1622,8 +1138,8 @@ k_tpq(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 float *ILst = vg0 + M * B;
 #pragma unroll
                 for (int m2 = 0; m2 < M; ++m2) ILst[m2 * B] = IL[NMAT - HF + m2];
-                V = payoff_forward_staged<M, B>(dprod, delta, ost_s, okk_s, owf_s, &disc, Bst, ILst, &mask);
-                payoff_adjoint_stage<NN, NMAT, B>(1.0f, disc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
+                V = payoff_forward_staged<B>(M, dprod, delta, ost_s, okk_s, owf_s, &disc, Bst, ILst, &mask);
+                payoff_adjoint_stage<B>(M, 1.0f, disc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
 #pragma unroll
                 for (int i = 0; i < H; ++i) {
                     X[i] = IL[NN - HF - H + i];
@@ -1787,8 +1303,6 @@ cudaError_t occ_tpp(int *blocks)
 
 bool f32_tpp_supports(int nn, int nmat) { return nn == 80 && nmat == 40; }
 
-int tps_block_threads() { return LMM_TPS_BLOCK; }
-
 bool f32_tpq_supports(int nn, int nmat) { return nn == 160 && nmat == 120; }
 
 int tpq_block_threads() { return LMM_TPQ_BLOCK; }
@@ -1812,23 +1326,6 @@ cudaError_t launch_tpq_any(const DevModel &m, const float *z, uint64_t seed, int
                   : launch_tpq<160, 120, false>(m, z, seed, path0, w, scratch, s);
 }
 
-size_t tps_scratch_floats_per_block(int nn, int nmat) { return (size_t)(2 * nmat + nn) * LMM_TPS_BLOCK; }
-
-cudaError_t tps_blocks_per_sm(bool philox, int *blocks)
-{
-    return philox ? occ_tps<80, 40, true, false>(blocks) : occ_tps<80, 40, false, false>(blocks);
-}
-
-cudaError_t launch_tps_any(const DevModel &m, const float *z, uint64_t seed, int64_t path0, bool philox,
-                           const Work &w, float *scratch, cudaStream_t s)
-{
-    if (w.ppt > 0)
-        return philox ? launch_tps<80, 40, true, false>(m, z, seed, path0, w, scratch, s)
-                      : launch_tps<80, 40, false, false>(m, z, seed, path0, w, scratch, s);
-    return philox ? launch_tps<80, 40, true, true>(m, z, seed, path0, w, scratch, s)
-                  : launch_tps<80, 40, false, true>(m, z, seed, path0, w, scratch, s);
-}
-
 int tpp_block_threads(Mode mode)
 {
     return mode == Mode::Fused ? tpp_block<Mode::Fused>()
@@ -1839,7 +1336,7 @@ int tpp_block_threads(Mode mode)
     do {                                                                                     \
         if (philox) {                                                                        \
             switch (mode) {                                                                  \
-                case Mode::Fused: return FN<80, 40, true, Mode::Fused>(__VA_ARGS__);         \
+                case Mode::Fused: break;                                                     \
                 case Mode::Forward: return FN<80, 40, true, Mode::Forward>(__VA_ARGS__);     \
                 case Mode::Backward: return FN<80, 40, true, Mode::Backward>(__VA_ARGS__);   \
             }                                                                                \

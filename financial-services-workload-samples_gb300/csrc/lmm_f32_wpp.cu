@@ -23,7 +23,14 @@
 //   dV/dlambda_k += Pb_i (Y_i - delta lambda_k) + t S'_i.
 // The payoff (portfolio_b :120-211, aliasing fixed) runs with double-FP32
 // products and sums (F2, lmm_device.cuh): the discount product is a warp
-// product reduction, the annuity recursion runs on lane 0.
+// product reduction, the annuity recursion runs on lane 0, on factors that the
+// lanes have formed side by side.
+// The forward holds log2(L/L0), which stays below 1 or so, where a product a step
+// would collect a rounding of L each, and the payoff's factors 1/(1 + delta L)
+// keep their rounding: fewer swaptions at the money pay or not unlike the exact
+// path (100 sets of normals, 80/40, 3,001 paths, median error of the Greeks 2.3e-7 ->
+// 5.6e-8; 50/20, 1,500 paths 4.5e-7 -> 7.9e-8; the latter with 2 sets that differ in
+// a swaption before, none now). 3,001 paths of 80/40 0.054 -> 0.049 ms.
 #include "lmm_device.cuh"
 
 namespace lmm {
@@ -86,7 +93,7 @@ __host__ __device__ inline WppLay wpp_layout(int nn, int nmat, int S, Mode mode 
     size_t w = 0;
     L.vg = w; w = al16(w + 4 * (size_t)(32 * S + wpp_head(nmat)));   // head rows discard, then vegas
     L.lw = w; w = al16(w + 4 * (size_t)32 * S);           // payoff staging [32*S]
-    L.bw = w; w = al16(w + 4 * (size_t)32 * S);           // annuity factors B[m] [32*S]
+    L.bw = w; w = al16(w + 4 * (size_t)32 * S);           // low parts of 1/(1 + delta L), then annuity factors B[m] [32*S]
     L.acc = w; w = al16(w + 8 * (size_t)2 * L.nout);      // FP64 sums [2*nout]
     L.per_warp = w;
     L.bytes = o + kWppWarps * w;
@@ -134,11 +141,12 @@ __device__ __forceinline__ int wpp_row(const int (&base)[S], int s, int n)
     return LMM_WPP_PAD ? base[s] - n : max(base[s] - n, 0);
 }
 
-// One forward step n over the lane's slots; returns Y at the lane's top slot
-// (its drift sum plus sqrt(delta) z), from which the reverse restarts.
+// One forward step n over the lane's slots, on D = log2(L/L0) and the rates L that
+// follow from it; returns Y at the lane's top slot (its drift sum plus
+// sqrt(delta) z), from which the reverse restarts.
 template <int S>
-__device__ __forceinline__ float wpp_fwd_step(float (&L)[S], const int (&base)[S], int n, float sqez,
-                                              int lane, const float4 *kc, float delta)
+__device__ __forceinline__ float wpp_fwd_step(float (&L)[S], float (&D)[S], const float (&L0)[S], const int (&base)[S], int n,
+                                              float sqez, int lane, const float4 *kc, float delta)
 {
     float a[S];
     float4 kk[S];
@@ -152,7 +160,10 @@ __device__ __forceinline__ float wpp_fwd_step(float (&L)[S], const int (&base)[S
     }
     const float X = warp_excl_prefix(P, lane) + sqez;
 #pragma unroll
-    for (int s = 0; s < S; ++s) L[s] *= ex2_approx(fmaf(kk[s].x, X + a[s], kk[s].y));
+    for (int s = 0; s < S; ++s) {
+        D[s] += fmaf(kk[s].x, X + a[s], kk[s].y);
+        L[s] = L0[s] * ex2_approx(D[s]);
+    }
     return X + a[S - 1];
 }
 
@@ -190,6 +201,15 @@ __device__ __forceinline__ void wpp_rev_step(float (&L)[S], float (&Pb)[S], cons
     // The next step's vega rows overlap neighbouring lanes' rows of this
     // step: order the shared-memory read-modify-writes across the warp.
     __syncwarp();
+}
+
+// 1/(1 + delta L), with the rounding of the reciprocal and of the sum while
+// delta L < 1.
+__device__ __forceinline__ F2 wpp_ratio(float L, float delta)
+{
+    const float q = fmaf(delta, L, 1.0f), r = __frcp_rn(q);
+    const float e = __fmaf_rn(delta, L, __fsub_rn(1.0f, q));
+    return {r, q < 2.0f ? r * __fmaf_rn(-r, e, __fmaf_rn(-r, q, 1.0f)) : 0.0f};
 }
 
 template <bool PHILOX>
@@ -253,6 +273,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     float *yt = ytop + ((size_t)blockIdx.x * kWppWarps + warp) * wpp_scratch_floats(nmat, S, ckn) + lane;
     float *ck = yt + (size_t)32 * nmat;     // ck[(c*S + s)*32]: rate of slot s at step c*ckn
     float *vg_s = reinterpret_cast<float *>(wbase + Ly.vg);
+    float *rt_s = vg_s + wpp_head(nmat);    // the payoff's factors, in the vega rows before their use
     float *lw_s = reinterpret_cast<float *>(wbase + Ly.lw);
     float *bw_s = reinterpret_cast<float *>(wbase + Ly.bw);
     double *acc = reinterpret_cast<double *>(wbase + Ly.acc);
@@ -296,11 +317,12 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             const uint64_t gpath = (uint64_t)(path0 + p);
             ZChunk<PHILOX> zc;
 
-            float L[S], Pb[S];
+            float L[S], Pb[S], L0[S], D[S];
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int i = S * lane + s;
-                L[s] = i < nn ? l0_s[i] : 1.0f;
+                L[s] = L0[s] = i < nn ? l0_s[i] : 1.0f;
+                D[s] = 0.0f;
             }
             // ---- forward ----
             for (int n = 0; n < nmat; ++n) {
@@ -309,7 +331,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     for (int s = 0; s < S; ++s) ck[((n / ckn) * S + s) * 32] = L[s];
                 }
                 const float sqez = sqd * zc.get(n, zp, nmat, seed, gpath, lane);
-                const float y = wpp_fwd_step<S>(L, base, n, sqez, lane, kc_s, delta);
+                const float y = wpp_fwd_step<S>(L, D, L0, base, n, sqez, lane, kc_s, delta);
                 if (MODE != Mode::Forward) yt[n * 32] = y;
             }
             // ---- payoff (double-FP32 products) and its adjoint ----
@@ -317,8 +339,15 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int i = S * lane + s;
-                if (i < nmat) dprod = f2_mul(dprod, __frcp_rn(fmaf(delta, L[s], 1.0f)));
-                if (i < nn) lw_s[i] = L[s];
+                L[s] = L0[s] * ex2_ulp(D[s]);
+                const F2 r = wpp_ratio(L[s], delta);
+                if (i < nmat) {
+                    dprod = f2_mul(dprod, r);
+                } else if (i < nn) {
+                    lw_s[i] = L[s];
+                    rt_s[i - nmat] = r.hi;
+                    bw_s[i - nmat] = r.lo;
+                }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -332,7 +361,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 F2 bb{1.0f, 0.0f}, sb{0.0f, 0.0f}, vs{0.0f, 0.0f};
                 unsigned long long mask = 0ull;
                 for (int mm = 0; mm < M; ++mm) {
-                    bb = f2_mul(bb, __frcp_rn(fmaf(delta, lw_s[nmat + mm], 1.0f)));
+                    bb = f2_mul(bb, F2{rt_s[mm], bw_s[mm]});
                     sb = f2_add(sb, bb);                      // annuity / delta
                     bw_s[mm] = bb.hi;
                     for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
@@ -354,7 +383,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 float Sb = 0.0f, Bb = 0.0f;
                 for (int mm = M - 1; mm >= 0; --mm) {
                     const float Ln = lw_s[nmat + mm];
-                    const float r = __frcp_rn(fmaf(delta, Ln, 1.0f));
+                    const float r = rt_s[mm];
                     const float Bm = bw_s[mm];
                     for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
                         if ((mask >> o) & 1ull) {
@@ -368,6 +397,8 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 }
             }
             V = __shfl_sync(0xffffffffu, V, 0);
+            __syncwarp();
+            for (int mm = lane; mm < M; mm += 32) rt_s[mm] = 0.0f;
             __syncwarp();
             if (MODE == Mode::Forward) {
                 if (lane == 0) {

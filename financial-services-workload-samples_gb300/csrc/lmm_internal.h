@@ -38,13 +38,14 @@ struct DevModel {
 
 // Path partition of one launch: nscen * items units; unit u takes scenario
 // u / items and the path range [item*ipaths, (item+1)*ipaths) of it, item =
-// u % items, in batches of bpaths. FP64 kernels: ppt batches of a block each.
+// u % items, in batches of bpaths; or, in the kernels of whole batches, ppt
+// batches of the block.
 struct Work {
     int64_t paths;        // per scenario
     int items;            // items per scenario
-    int64_t ipaths = 0;   // FP32 kernels: paths per item
-    int bpaths = 0;       // FP32 kernels: paths per batch, at most the kernel's batch size
-    int ppt = 0;          // FP64 kernels, and k_tps where every batch is full: batches per item
+    int64_t ipaths = 0;   // paths per item
+    int bpaths = 0;       // paths per batch, at most the kernel's batch size
+    int ppt = 0;          // kernels of whole batches: batches per item
     double *partial;      // [nscen*items][2*nout]: per-item sums and sums of squares
     int nout;             // outputs per scenario reduced by this launch
     int grid = 0;         // FP32 kernels: blocks launched (0: one per unit); block b
@@ -66,14 +67,15 @@ cudaError_t tpp_blocks_per_sm(Mode mode, bool philox, int *blocks);
 cudaError_t launch_tpp_any(const DevModel &m, Mode mode, const float *z, uint64_t seed,
                            int64_t path0, bool philox, const Work &w, float *tape,
                            const double *vbar, cudaStream_t s);
-// The fused 80/40 kernel with the reverse sweep split over the rate halves
-// (lmm_f32_tpp.cu, k_tps): 12 warps per SM, a per-block scratch of
-// tps_scratch_floats_per_block floats.
-int tps_block_threads();
-size_t tps_scratch_floats_per_block(int nn, int nmat);
-cudaError_t tps_blocks_per_sm(bool philox, int *blocks);
-cudaError_t launch_tps_any(const DevModel &m, const float *z, uint64_t seed, int64_t path0, bool philox,
-                           const Work &w, float *scratch, cudaStream_t s);
+// FP32 thread-per-path kernels in rate blocks (lmm_f32_tpb.cuh, k_tpb): the
+// fused 80/40 call, and every mode of other shapes whose checkpoint interval is
+// a multiple of 4. A per-block scratch of tpb_scratch_floats_per_block floats.
+bool f32_tpb_supports(int nn, int nmat, int ckpt);
+int tpb_block_threads(int nn, int nmat);
+size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt);
+cudaError_t tpb_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks);
+cudaError_t launch_tpb_any(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
+                           const Work &w, float *scratch, const double *vbar, cudaStream_t s);
 // The fused 160/120 kernel with one thread per path and the reverse in passes
 // over blocks of 40 rates (lmm_f32_tpp.cu, k_tpq): a per-block scratch of
 // tpq_scratch_floats_per_block floats; checkpoint intervals multiples of 4.

@@ -1,5 +1,5 @@
-"""Path counts at the edges of the launch plan: the line between the
-warp-per-path and the thread-per-path kernels (two fills of the device), single
+"""Shapes and path counts at the edges of the launch plan: the line between the
+warp-per-path and the thread-per-path kernels (in fills of the device), single
 warps per SM, partly filled last batches, one path more than whole waves, and
 several scenarios in short units. FP32 results against the FP64 kernel on the
 same normals within the FP32 rule (1e-4 per Greek, Greeks below 1% of their
@@ -12,7 +12,7 @@ from conftest import cfgs, pkg
 
 pytestmark = pytest.mark.gpu
 
-FILL = 2 * 152 * 6 * 4       # the line at 80/40 and 160/120 on 152 SMs
+FILL = 2 * 152 * 6 * 4       # two fills on 152 SMs, the line at 160/120; one and a half at 80/40
 
 
 def _scaled(g, r, nn):
@@ -62,6 +62,11 @@ def test_80x40_counts(paths):
     _run(cfgs().workload(4, paths), paths, 70 + paths % 7, pair=True, philox=True)
 
 
+@pytest.mark.parametrize("paths", [FILL * 3 // 4, FILL * 3 // 4 + 1, 152 * 512, 152 * 512 + 1, 152 * 512 + 152 * 416 + 5])
+def test_80x40_counts_of_blocks_of_512(paths):
+    _run(cfgs().workload(4, paths), paths, 71 + paths % 5, pair=True, philox=True)
+
+
 @pytest.mark.parametrize("paths", [3, FILL, FILL + 1, 152 * 256 + 1])
 def test_160x120_counts(paths):
     _run(cfgs().workload(3, paths), paths, 80 + paths % 7, pair=True)
@@ -72,3 +77,39 @@ def test_scenarios(curves, paths):
     cfg = cfgs().workload(5, paths)
     cfg.L0 = np.ascontiguousarray(cfg.L0[:curves])
     _run(cfg, paths, 90 + curves)
+
+
+def _shape(nn, nmat, paths, seed, nopt=7, vol=(0.1, 0.2)):
+    rng = np.random.default_rng(seed)
+    return cfgs().LmmConfig("shape", nn, nmat, 0.25, rng.uniform(0.02, 0.07, nn), rng.uniform(*vol, nn),
+                            rng.integers(1, nn - nmat + 1, nopt).astype(np.int32), rng.uniform(0.03, 0.06, nopt), paths)
+
+
+# rate counts at the edges of the blocks of 20 and passes of 40, step counts with every remainder by 4, block sizes
+# of 512, 384, 256 and 128 threads
+SHAPES = [(2, 1), (3, 2), (19, 7), (20, 10), (21, 6), (33, 7), (40, 39), (41, 20), (61, 33), (79, 40), (96, 60), (100, 99),
+          (121, 62), (160, 80), (181, 45), (200, 100), (256, 40), (256, 131)]
+
+
+@pytest.mark.parametrize("nn,nmat", SHAPES, ids=lambda v: str(v))
+def test_shapes_beyond_the_line(nn, nmat):
+    """More paths than the warp-per-path kernels take, with a ragged end; the
+    vols keep the Euler paths of the long shapes tame."""
+    paths = 2 * 152 * 16 * 4 + 257
+    cfg = _shape(nn, nmat, paths, nn * 1000 + nmat, vol=(0.05, 0.12) if nmat > 90 else (0.1, 0.2))
+    _run(cfg, paths, nn + nmat, pair=True, philox=True)
+
+
+@pytest.mark.parametrize("ck", [0, 4, 6, 8, 12, 60])
+def test_checkpoint_intervals_beyond_the_line(ck):
+    """Intervals that are a multiple of 4 and one that is not (warp per path)."""
+    cfg = _shape(96, 60, 10007, 5)
+    cfg.ckpt_every = ck
+    _run(cfg, 10007, 6, pair=True)
+
+
+def test_scenarios_of_a_shape_beyond_the_line():
+    cfg = _shape(50, 22, 4001, 7)
+    rng = np.random.default_rng(1)
+    cfg.L0 = rng.uniform(0.02, 0.07, (5, 50))
+    _run(cfg, 4001, 8, pair=True)
