@@ -221,11 +221,13 @@ bool ragged_batches(int fam, Mode mode) { return fam == 2 || fam == 6 || (fam ==
 
 // Time of a ragged batch of n paths relative to a full one. GB300, one batch
 // per SM, 80/40, one / two / three / four warps per scheduler: k_tpb
-// 0.092, 0.120, 0.150, 0.187 ms; the forward of the pair 0.037, 0.048, 0.059.
+// 0.092, 0.120, 0.150, 0.187 ms (a linear fit; other shapes alike, 20,000 paths of
+// 128/100 in one batch 0.586 ms, in two 0.860); the forward of the pair 0.037,
+// 0.048, 0.059.
 double batch_cost(int fam, int n, int batch)
 {
     const int wps = (n + 127) / 128, full = batch / 128;
-    if (fam == 6) return full <= 1 ? 1.0 : 0.49 + 0.51 * (wps - 1) / (full - 1);
+    if (fam == 6) return (0.32 + 0.17 * wps) / (0.32 + 0.17 * full);
     if (fam == 1) return wps == 1 ? 0.63 : wps == 2 ? 0.82 : 1.0;
     return 1.0;
 }
@@ -264,26 +266,39 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
     return LMM_OK;
 }
 
-// The family of a call of `paths` paths: the warp-per-path kernels for few
-// paths, family_for above. A thread-per-path kernel takes one path's latency
-// (80/40 fused 0.090 ms, 160/120 0.47 ms) for anything from one path to a
-// device full of single warps; a warp per path takes 0.04 ms (0.096) for one
-// path and its throughput beyond the device's resident warps (3,648 on GB300):
-// 80/40 fused, kernel alone, 3,001 / 4,864 / 7,296 paths 0.049 / 0.079 / 0.105
-// against 0.090 ms, 160/120 at 3,001 / 4,864 / 9,728 paths 0.15 / 0.25 / 0.48
-// against 0.47-0.48 ms. The line is one and a half fills of the device for the
-// shapes whose fused call runs in rate blocks, two for the others, and the same
-// for every mode: the fused call and the forward/backward pair of the same size
-// must round alike.
+// Fills of the device up to which a warp per path is the faster one. A
+// thread-per-path kernel takes one path's latency for anything from one path to
+// a device full of single warps; a warp per path takes a short time for one path
+// and its throughput beyond the device's resident warps (3,648 on GB300; 3,040
+// above 160 rates). 160/120 fused, kernel alone, at 3,001 / 4,864 / 9,728 paths:
+// 0.15 / 0.25 / 0.48 against 0.47 ms, two fills. Shapes in rate blocks: the ratio
+// of the two estimates in us, fitted to whole calls of 13 shapes, of which a warp
+// per path / rate blocks took, at 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line
+// at 2.9 fills), 0.246 / 0.416 (128/100; 2.9), 0.109 / 0.160 (64/50; 2.4), 0.086 /
+// 0.113 (60/30; 2.2), 0.090 / 0.100 (80/40; 1.6), 0.055 / 0.057 (40/10; 1.4).
+// Above 160 rates a lane's eight rates collide on the banks: one fill (3,600
+// paths, 161/100 0.61 / 0.55, 256/40 0.42 / 0.44).
+double wpp_fills(int nn, int nmat, bool rate_blocks)
+{
+    if (!rate_blocks) return 2.0;
+    const int slots = lmm::wpp_slots(nn);
+    if (slots > 5) return 1.0;
+    const double blocks = 25.0 + (nn == 80 && nmat == 40 ? 0.011 : 0.0175) * lmm::tpb_cells(nn, nmat);
+    return std::min(4.0, std::max(1.0, blocks / (20.0 + nmat * (0.5 + 0.15 * slots))));
+}
+
+// The family of a call of `paths` paths: the warp-per-path kernels for few paths,
+// family_for above; alike for every mode, as the fused call and the
+// forward/backward pair of the same size must round alike.
 int family_at(lmm_engine *e, Mode mode, int64_t paths, int *fam)
 {
     *fam = family_for(e, mode);
     if (*fam == 0 || *fam == 2 || !lmm::f32_wpp_supports(e->nn, e->nmat)) return LMM_OK;
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, 2, Mode::Fused, false, &bps));
-    const int64_t fill = (int64_t)e->sms * bps * batch_paths(e, 2, Mode::Fused);
-    const int64_t line = family_for(e, Mode::Fused) == 6 ? fill + fill / 2 : 2 * fill;
-    if (paths <= line / e->nscen) *fam = 2;
+    const double fill = (double)e->sms * bps * batch_paths(e, 2, Mode::Fused);
+    const double line = fill * wpp_fills(e->nn, e->nmat, family_for(e, Mode::Fused) == 6);
+    if (paths * e->nscen <= (int64_t)line) *fam = 2;
     return LMM_OK;
 }
 

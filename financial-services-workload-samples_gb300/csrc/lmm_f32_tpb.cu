@@ -1,6 +1,8 @@
 // Instances and dispatch of the rate-block kernel (lmm_f32_tpb.cuh).
 #include "lmm_f32_tpb.cuh"
 
+#include <algorithm>
+
 namespace lmm {
 
 // Threads per block: registers allow 512, 384, 256 threads (16, 12, 8 warps an
@@ -19,6 +21,16 @@ size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt)
     const TpbLay L = tpb_layout(nn, nmat, Mode::Fused, B);
     const int nck = ckpt > 0 ? (nmat - 1) / ckpt : 0;
     return (size_t)(L.s_ck + nck * kRR * L.nr) * B;
+}
+
+// Cells that one path walks, no-ops of partly active passes and blocks among them:
+// a launch of few paths takes their latency.
+int tpb_cells(int nn, int nmat)
+{
+    int c = 0;
+    for (int lo = 0; lo < nn; lo += kFR) c += kFR * std::min(nmat, lo + kFR - 1);
+    for (int lo = 0; lo < nn; lo += kRR) c += kRR * std::min(nmat, lo + kRR - 1);
+    return c;
 }
 
 // Checkpoints are restored between groups of steps.

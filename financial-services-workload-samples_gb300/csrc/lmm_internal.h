@@ -72,6 +72,7 @@ cudaError_t launch_tpp_any(const DevModel &m, Mode mode, const float *z, uint64_
 // a multiple of 4. A per-block scratch of tpb_scratch_floats_per_block floats.
 bool f32_tpb_supports(int nn, int nmat, int ckpt);
 int tpb_block_threads(int nn, int nmat);
+int tpb_cells(int nn, int nmat);
 size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt);
 cudaError_t tpb_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks);
 cudaError_t launch_tpb_any(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,

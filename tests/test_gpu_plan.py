@@ -103,9 +103,9 @@ def test_shapes_beyond_the_line(nn, nmat):
 @pytest.mark.parametrize("ck", [0, 4, 6, 8, 12, 60])
 def test_checkpoint_intervals_beyond_the_line(ck):
     """Intervals that are a multiple of 4 and one that is not (warp per path)."""
-    cfg = _shape(96, 60, 10007, 5)
+    cfg = _shape(96, 60, 15007, 5)
     cfg.ckpt_every = ck
-    _run(cfg, 10007, 6, pair=True)
+    _run(cfg, 15007, 6, pair=True)
 
 
 def test_scenarios_of_a_shape_beyond_the_line():
