@@ -182,9 +182,8 @@ void mark(lmm_engine *e, int i)
 int variant_key(int family, Mode mode, bool philox) { return family * 16 + (int)mode * 2 + (philox ? 1 : 0); }
 
 // Kernel family of an FP32 call of many paths (family_at):
-//   6 thread per path in rate blocks (k_tpb): fused 80/40 calls, and every mode
-//     of the shapes below without a kernel of their own;
-//   1 thread per path (k_tpp): the 80/40 forward/backward pair, on a tape;
+//   6 thread per path in rate blocks (k_tpb): every mode of 80/40 (the pair on a
+//     tape) and of the shapes without a kernel of their own;
 //   7 thread per path in blocks of 40 rates (k_tpq): fused 160/120 calls (GB300,
 //     1,048,576 paths: 14.2 ms; thread pair 18.3);
 //   5 two threads per path (lmm_f32_tp2.cu): the 160/120 pair, on a tape;
@@ -196,15 +195,13 @@ int family_for(const lmm_engine *e, Mode mode)
 {
     if (lmm::f32_tp2_supports(e->nn, e->nmat))
         return LMM_USE_TPQ && mode == Mode::Fused && lmm::f32_tpq_supports(e->nn, e->nmat) ? 7 : 5;
-    if (lmm::f32_tpp_supports(e->nn, e->nmat) && mode != Mode::Fused) return 1;
     if (lmm::f32_tpb_supports(e->nn, e->nmat, e->dm.ckpt)) return 6;
     return lmm::f32_wpp_supports(e->nn, e->nmat) ? 2 : 0;
 }
 
 // Paths one block takes per batch.
-int batch_paths(const lmm_engine *e, int fam, Mode mode)
+int batch_paths(const lmm_engine *e, int fam)
 {
-    if (fam == 1) return lmm::tpp_block_threads(mode);
     if (fam == 5) return lmm::tp2_paths_per_block(e->nn);
     if (fam == 6) return lmm::tpb_block_threads(e->nn, e->nmat);
     if (fam == 7) return lmm::tpq_block_threads();
@@ -215,32 +212,28 @@ int batch_paths(const lmm_engine *e, int fam, Mode mode)
 int batch_gran(int fam) { return fam == 2 ? lmm::wpp_block_threads() / 32 : 32; }
 
 // Kernels whose batches may be ragged (run by the warps that have paths): rate
-// blocks, the 80/40 forward-only kernel, warp per path. The others run whole
-// batches of the block.
-bool ragged_batches(int fam, Mode mode) { return fam == 2 || fam == 6 || (fam == 1 && mode == Mode::Forward); }
+// blocks, warp per path. The others run whole batches of the block.
+bool ragged_batches(int fam) { return fam == 2 || fam == 6; }
 
 // Time of a ragged batch of n paths relative to a full one. GB300, one batch
 // per SM, 80/40, one / two / three / four warps per scheduler: k_tpb
 // 0.092, 0.120, 0.150, 0.187 ms (a linear fit; other shapes alike, 20,000 paths of
-// 128/100 in one batch 0.586 ms, in two 0.860); the forward of the pair 0.037,
-// 0.048, 0.059.
+// 128/100 in one batch 0.586 ms, in two 0.860).
 double batch_cost(int fam, int n, int batch)
 {
     const int wps = (n + 127) / 128, full = batch / 128;
     if (fam == 6) return (0.32 + 0.17 * wps) / (0.32 + 0.17 * full);
-    if (fam == 1) return wps == 1 ? 0.63 : wps == 2 ? 0.82 : 1.0;
     return 1.0;
 }
 
 cudaError_t launch_f32_family(int fam, const lmm::DevModel &m, Mode mode, const float *z, uint64_t seed,
-                              int64_t path0, bool philox, const Work &w, float *tape, const double *vbar,
-                              cudaStream_t s)
+                              int64_t path0, bool philox, const Work &w, float *scr, float *tape,
+                              const double *vbar, cudaStream_t s)
 {
-    if (fam == 1) return lmm::launch_tpp_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
-    if (fam == 5) return lmm::launch_tp2_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
-    if (fam == 6) return lmm::launch_tpb_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
-    if (fam == 7) return lmm::launch_tpq_any(m, z, seed, path0, philox, w, tape, s);
-    return lmm::launch_wpp_any(m, mode, z, seed, path0, philox, w, tape, vbar, s);
+    if (fam == 5) return lmm::launch_tp2_any(m, mode, z, seed, path0, philox, w, mode == Mode::Fused ? scr : tape, vbar, s);
+    if (fam == 6) return lmm::launch_tpb_any(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
+    if (fam == 7) return lmm::launch_tpq_any(m, z, seed, path0, philox, w, scr, s);
+    return lmm::launch_wpp_any(m, mode, z, seed, path0, philox, w, scr, vbar, s);
 }
 
 int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
@@ -253,8 +246,7 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
     }
     int b = 0;
     cudaError_t err;
-    if (family == 1) err = lmm::tpp_blocks_per_sm(mode, philox, &b);
-    else if (family == 2) err = lmm::wpp_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
+    if (family == 2) err = lmm::wpp_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 5) err = lmm::tp2_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 6) err = lmm::tpb_blocks_per_sm(e->nn, e->nmat, mode, philox, &b);
     else if (family == 7) err = lmm::tpq_blocks_per_sm(philox, &b);
@@ -270,20 +262,22 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
 // thread-per-path kernel takes one path's latency for anything from one path to
 // a device full of single warps; a warp per path takes a short time for one path
 // and its throughput beyond the device's resident warps (3,648 on GB300; 3,040
-// above 160 rates). 160/120 fused, kernel alone, at 3,001 / 4,864 / 9,728 paths:
-// 0.15 / 0.25 / 0.48 against 0.47 ms, two fills. Shapes in rate blocks: the ratio
-// of the two estimates in us, fitted to whole calls of 13 shapes, of which a warp
-// per path / rate blocks took, at 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line
-// at 2.9 fills), 0.246 / 0.416 (128/100; 2.9), 0.109 / 0.160 (64/50; 2.4), 0.086 /
-// 0.113 (60/30; 2.2), 0.090 / 0.100 (80/40; 1.6), 0.055 / 0.057 (40/10; 1.4).
+// above 160 rates). 160/120, whole calls at 3,600 / 4,800 / 5,600 paths: fused
+// 0.191 / 0.258 / 0.295 against 0.53 ms, the pair 0.274 / 0.373 / 0.426 against
+// 0.393; the pair, which has to go with the fused call, puts the line at 1.33
+// fills. Shapes in rate blocks: the ratio of the two estimates in us, fitted to
+// whole calls of 13 shapes, of which a warp per path / rate blocks took, at
+// 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line at 2.9 fills), 0.246 / 0.416
+// (128/100; 2.9), 0.109 / 0.160 (64/50; 2.4), 0.086 / 0.113 (60/30; 2.2), 0.098 /
+// 0.100 and for the pair 0.158 / 0.132 (80/40; 1.3), 0.055 / 0.057 (40/10; 1.4).
 // Above 160 rates a lane's eight rates collide on the banks: one fill (3,600
 // paths, 161/100 0.61 / 0.55, 256/40 0.42 / 0.44).
 double wpp_fills(int nn, int nmat, bool rate_blocks)
 {
-    if (!rate_blocks) return 2.0;
+    if (!rate_blocks) return 4.0 / 3.0;
     const int slots = lmm::wpp_slots(nn);
     if (slots > 5) return 1.0;
-    const double blocks = 25.0 + (nn == 80 && nmat == 40 ? 0.011 : 0.0175) * lmm::tpb_cells(nn, nmat);
+    const double blocks = 25.0 + (nn == 80 && nmat == 40 ? 0.0088 : 0.0175) * lmm::tpb_cells(nn, nmat);
     return std::min(4.0, std::max(1.0, blocks / (20.0 + nmat * (0.5 + 0.15 * slots))));
 }
 
@@ -296,7 +290,7 @@ int family_at(lmm_engine *e, Mode mode, int64_t paths, int *fam)
     if (*fam == 0 || *fam == 2 || !lmm::f32_wpp_supports(e->nn, e->nmat)) return LMM_OK;
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, 2, Mode::Fused, false, &bps));
-    const double fill = (double)e->sms * bps * batch_paths(e, 2, Mode::Fused);
+    const double fill = (double)e->sms * bps * batch_paths(e, 2);
     const double line = fill * wpp_fills(e->nn, e->nmat, family_for(e, Mode::Fused) == 6);
     if (paths * e->nscen <= (int64_t)line) *fam = 2;
     return LMM_OK;
@@ -350,9 +344,9 @@ struct PathPlan {
 };
 PathPlan plan_paths(const lmm_engine *e, int fam, Mode mode, int64_t nvs, int64_t paths, int bps)
 {
-    const int batch = batch_paths(e, fam, mode), gran = batch_gran(fam);
+    const int batch = batch_paths(e, fam), gran = batch_gran(fam);
     const int64_t cap = std::max<int64_t>(1, (int64_t)e->sms * bps);
-    const bool ragged = ragged_batches(fam, mode);
+    const bool ragged = ragged_batches(fam);
     const double unit = 0.015;     // a unit's own cost: accumulators cleared and written out
     PathPlan best;
     double best_cost = 1e300;
@@ -524,13 +518,14 @@ int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t p
     const int nout = mode == Mode::Fused ? 1 + 2 * e->nn : (mode == Mode::Forward ? 1 : 2 * e->nn);
     Work w{};
     LMM_TRY(plan(e, fam, mode, e->nscen, paths, bps, nout, &w));
-    if (fam == 2) LMM_TRY(wpp_scratch(e, w.grid, &tape));
-    if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &tape));
-    if (fam == 6) LMM_TRY(tpb_scratch(e, w.grid, &tape));
-    if (fam == 7) LMM_TRY(tpq_scratch(e, w.grid, &tape));
+    float *scr = nullptr;
+    if (fam == 2) LMM_TRY(wpp_scratch(e, w.grid, &scr));
+    if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &scr));
+    if (fam == 6) LMM_TRY(tpb_scratch(e, w.grid, &scr));
+    if (fam == 7) LMM_TRY(tpq_scratch(e, w.grid, &scr));
     LMM_TRY(next_stamp(e));
     mark(e, 0);
-    cudaError_t err = launch_f32_family(fam, e->dm, mode, d_z, seed, path0, philox, w, tape, d_vbar, e->stream);
+    cudaError_t err = launch_f32_family(fam, e->dm, mode, d_z, seed, path0, philox, w, scr, tape, d_vbar, e->stream);
     if (err != cudaSuccess) return cuda_fail(err, "FP32 LMM kernel launch");
     mark(e, 1);
     LMM_CK(lmm::launch_finalize(w.partial, e->nscen, w.items, nout, paths, d_mean, d_se,
@@ -1076,7 +1071,7 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
     if (fam == 0) return fail(LMM_ERR_UNSUPPORTED, "no FP32 kernel for this shape");
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, fam, Mode::Fused, false, &bps));
-    const int per_batch = batch_paths(e, fam, Mode::Fused);
+    const int per_batch = batch_paths(e, fam);
     const int nout = 1 + 2 * e->nn;
     int64_t cpaths[kHostChunks], cfirst[kHostChunks];
     PathPlan cplan[kHostChunks];
@@ -1142,7 +1137,7 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
         w.grid = (int)std::min<int64_t>(cplan[c].items, (int64_t)e->sms * bps);
         w.partial = part;
         const float *zc = dz + (size_t)cfirst[c] * e->nmat;
-        cudaError_t err = launch_f32_family(fam, e->dm, Mode::Fused, zc, 0, 0, false, w, wscr, nullptr, e->stream);
+        cudaError_t err = launch_f32_family(fam, e->dm, Mode::Fused, zc, 0, 0, false, w, wscr, nullptr, nullptr, e->stream);
         if (err != cudaSuccess) return cuda_fail(err, "FP32 LMM kernel launch");
         part += (size_t)cplan[c].items * 2 * nout;
     }
@@ -1202,17 +1197,14 @@ int lmm_tape_create(lmm_engine *e, int64_t paths, lmm_tape **out)
     std::unique_ptr<lmm_tape> t(new lmm_tape());
     t->e = e;
     t->paths = paths;
-    // The thread-per-path (nn=80, nmat=40) and thread-pair (nn=160, nmat=120)
-    // kernels keep the terminal rates and the per-step drift sums; the
-    // warp-per-path backward recomputes its forward from the same normals and
-    // needs no tape.
+    // The rate-block (nn=80, nmat=40) and thread-pair (nn=160, nmat=120) pairs
+    // keep the terminal rates and the per-step drift sums, the thread pair also
+    // those at the half boundary; the others' backward recomputes its forward
+    // from the same normals and needs no tape.
     int fam = 0;
     LMM_TRY(family_at(e, Mode::Forward, paths, &fam));
-    if (fam == 1 || fam == 5) {
-        // thread pair: also the drift sums at the half boundary
-        const size_t rows = (size_t)e->nn + (size_t)e->nmat * (fam == 5 ? 2 : 1);
-        LMM_TRY(t->buf.ensure(sizeof(float) * rows * e->nscen * (size_t)paths));
-    }
+    const size_t rows = fam == 5 ? (size_t)e->nn + 2 * (size_t)e->nmat : fam == 6 ? (size_t)lmm::tpb_tape_rows(e->nn, e->nmat) : 0;
+    if (rows) LMM_TRY(t->buf.ensure(sizeof(float) * rows * e->nscen * (size_t)paths));
     *out = t.release();
     return LMM_OK;
 }

@@ -5,6 +5,10 @@
 
 namespace lmm {
 
+// The shape whose forward/backward pair runs on a tape (k_tpb): rows of it; 0:
+// the backward runs the forward again.
+int tpb_tape_rows(int nn, int nmat) { return nn == 80 && nmat == 40 ? nn + nmat : 0; }
+
 // Threads per block: registers allow 512, 384, 256 threads (16, 12, 8 warps an
 // SM), the vega rows of a block's paths have to fit in shared memory. 0: no
 // block fits.
@@ -17,10 +21,9 @@ int tpb_block_threads(int nn, int nmat)
 
 size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt)
 {
-    const int B = tpb_block_threads(nn, nmat);
-    const TpbLay L = tpb_layout(nn, nmat, Mode::Fused, B);
+    const TpbLay L = tpb_layout(nn, nmat, Mode::Fused, 32);      // rows
     const int nck = ckpt > 0 ? (nmat - 1) / ckpt : 0;
-    return (size_t)(L.s_ck + nck * kRR * L.nr) * B;
+    return (size_t)(L.s_ck + nck * kRR * L.nr) * tpb_block_threads(nn, nmat);
 }
 
 // Cells that one path walks, no-ops of partly active passes and blocks among them:
@@ -46,15 +49,26 @@ cudaError_t occ_tpb_narrow(int B, int nn, int nmat, Mode mode, bool philox, int 
 
 cudaError_t tpb_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks)
 {
-    if (nn == 80 && nmat == 40) return occ_tpb<80, 40, 512>(nn, nmat, mode, philox, blocks);
+    if (nn == 80 && nmat == 40) {
+        if (mode == Mode::Forward) return occ_tpb<80, 40, 512, Mode::Forward>(nn, nmat, mode, philox, blocks);
+        if (mode == Mode::Backward) return occ_tpb<80, 40, 512, Mode::Backward>(nn, nmat, mode, philox, blocks);
+        return occ_tpb<80, 40, 512>(nn, nmat, mode, philox, blocks);
+    }
     const int B = tpb_block_threads(nn, nmat);
     return B >= 384 ? occ_tpb_wide(B, nn, nmat, mode, philox, blocks) : occ_tpb_narrow(B, nn, nmat, mode, philox, blocks);
 }
 
 cudaError_t launch_tpb_any(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
-                           const Work &w, float *scr, const double *vbar, cudaStream_t s)
+                           const Work &w, float *scr, float *tape, const double *vbar, cudaStream_t s)
 {
-    if (m.nn == 80 && m.nmat == 40) return launch_tpb<80, 40, 512>(m, mode, z, seed, path0, philox, w, scr, vbar, s);
+    if (m.nn == 80 && m.nmat == 40) {
+        if (mode != Mode::Fused && !tape) return cudaErrorInvalidValue;
+        if (mode == Mode::Forward)
+            return launch_tpb<80, 40, 512, Mode::Forward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
+        if (mode == Mode::Backward)
+            return launch_tpb<80, 40, 512, Mode::Backward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
+        return launch_tpb<80, 40, 512>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s);
+    }
     const int B = tpb_block_threads(m.nn, m.nmat);
     return B >= 384 ? launch_tpb_wide(B, m, mode, z, seed, path0, philox, w, scr, vbar, s)
                     : launch_tpb_narrow(B, m, mode, z, seed, path0, philox, w, scr, vbar, s);

@@ -1,5 +1,6 @@
-// FP32 thread-per-path LMM kernel in rate blocks (k_tpb): the fused call for
-// NN=80, NMAT=40, and every mode of the shapes without a kernel of their own.
+// FP32 thread-per-path LMM kernel in rate blocks (k_tpb): the fused call and the
+// forward/backward pair for NN=80, NMAT=40, and every mode of the shapes without a
+// kernel of their own.
 //
 // One CUDA thread carries one Monte Carlo path through
 //   forward   path_calc_b1   (LiborMarketModel/liborSwaptionGreeks.cpp:34-82)
@@ -29,8 +30,12 @@
 // column sums 39.7 -> 38.85 ms. Two paths a thread in packed FP32
 // (fma.rn.f32x2) reads as many operands for a path and ran 40.5 ms.
 //
+// The 80/40 pair, 300,001 paths, against 80 rates and as many adjoints a thread
+// (12 and 8 warps an SM): 1.030 -> 0.808 ms, of which the forward 0.286; it ran 6%
+// slower with 20 warps of 96 registers.
+//
 // Other shapes, against the kernel that gave a path two threads or a warp: 50,001
-// paths of 96/60 0.96 -> 0.405 ms.
+// paths of 96/60 0.96 -> 0.393 ms.
 //
 // The reverse runs in units of sigma = lambda sqrt(delta): with X = 1/(delta L),
 // t = 1/(X + 1), y = (drift sum + normal term)/sqrt(delta) a cell is
@@ -58,8 +63,8 @@ struct TpbLay {
     int kf, kr, il0, ost, okf, owf, okk, vg, acc, bytes;
     // scratch, rows: drift sums at the top of every half pass [2 nf][nmat], suffix sums at the bottom of the
     // reverse block last run [nmat], rates [kFR nf], log-adjoints, then deltas [kRR nr], annuity factors [M],
-    // normal terms [nmat], checkpoints [nck][kRR nr]
-    int s_v, s_s, s_x, s_d, s_b, s_q, s_ck;
+    // drift sums without the normal terms at the top of the pass last run [nmat], normal terms [nmat], checkpoints [nck][kRR nr]
+    int s_v, s_s, s_x, s_d, s_b, s_p, s_q, s_ck;
 };
 
 __host__ __device__ constexpr int tpb_al(int x) { return (x + 15) & ~15; }
@@ -90,7 +95,8 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
     L.s_x = L.s_s + nmat;
     L.s_d = L.s_x + kFR * L.nf;
     L.s_b = L.s_d + kRR * L.nr;
-    L.s_q = L.s_b + L.M;
+    L.s_p = L.s_b + L.M;
+    L.s_q = L.s_p + nmat;
     L.s_ck = L.s_q + nmat;
     return L;
 }
@@ -103,7 +109,7 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
 // factors keep their rounding. Against the exact paths, 100 sets of normals, 96/60,
 // 50,001 paths: median error of the Greeks 2.8e-7 (the rates themselves, a warp a
 // path) -> 1.1e-7, and sets in which a swaption at the money paid on one side only
-// 17 -> 1; 150/100, 20,000 paths 5.7e-7 -> 8.1e-8 and 12 -> 0. It takes 0.405 ms
+// 17 -> 1; 150/100, 20,000 paths 5.7e-7 -> 8.1e-8 and 12 -> 0. It takes 0.393 ms
 // where products took 0.343 (96/60). 80/40 rounds as its pair of calls does.
 template <bool LOGS>
 __device__ __forceinline__ float inv_rate(float x, const float *il0)
@@ -326,17 +332,22 @@ __device__ __forceinline__ void column_sums(int nn, const float *vg, int warp, i
     }
 }
 
-// NN, NMAT: the shape, or 0 for a shape at run time (any mode, `mode`; rate
-// checkpoints every m.ckpt steps, a multiple of kRG, or none).
-template <int NN, int NMAT, int B, bool PHILOX>
+// NN, NMAT, MODE: the shape and mode, or 0 for a shape at run time (any mode,
+// `mode_arg`; rate checkpoints every m.ckpt steps, a multiple of kRG, or none).
+// The forward of a fixed shape writes the tape, [NN][total] terminal inverse rates
+// and [NMAT][total] drift sums at the top rate, and its backward reads it: what the
+// reverse of one block has for the drift sums at its bottom is where the block
+// below starts.
+template <int NN, int NMAT, int B, bool PHILOX, Mode MODE>
 __global__ void __launch_bounds__(B, 1)
 k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w, float *__restrict__ scr,
-      const double *__restrict__ vbar, int mode_arg)
+      float *__restrict__ tape, const double *__restrict__ vbar, int mode_arg)
 {
     constexpr bool FIX = NN > 0;
+    constexpr bool TAPED = FIX && MODE == Mode::Backward;
     constexpr int NW = B / 32;
-    const Mode mode = FIX ? Mode::Fused : (Mode)mode_arg;
-    const TpbLay Ly = FIX ? tpb_layout(NN, NMAT, Mode::Fused, B) : tpb_layout(m.nn, m.nmat, mode, B);
+    const Mode mode = FIX ? MODE : (Mode)mode_arg;
+    const TpbLay Ly = FIX ? tpb_layout(NN, NMAT, MODE, B) : tpb_layout(m.nn, m.nmat, mode, B);
     const int nn = Ly.nn, nmat = Ly.nmat, M = Ly.M, nout = Ly.nout;
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *kf_s = reinterpret_cast<float4 *>(smem + Ly.kf), *kr_s = reinterpret_cast<float4 *>(smem + Ly.kr);
@@ -383,26 +394,39 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
         __syncthreads();          // the previous unit's reads of il0/acc are done
         for (int i = tid; i < kFR * Ly.nf; i += B) il0_s[i] = i < nn ? m.invL0f[scen * nn + i] : kPadIL;
         for (int i = tid; i < NW * 2 * nout; i += B) acc_s[i] = 0.0;
-        const float vb = !FIX && mode == Mode::Backward ? (float)vbar[scen] : 1.0f;
+        const float vb = mode == Mode::Backward ? (float)vbar[scen] : 1.0f;
 
         for (int jb = 0; batch_left(w, item, jb) > 0; ++jb) {       // block-uniform
             // one barrier per batch keeps the warps near each other in the code (instruction cache)
             __syncthreads();
             if ((tid & ~31) >= batch_left(w, item, jb)) continue;    // whole warps
             const int64_t pc0 = (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths;
+            const int64_t pc = tid < batch_left(w, item, jb) ? pc0 + tid : w.paths - 1;
+            const int64_t total = (int64_t)m.nscen * w.paths;         // the tape's row
+            float *tp = FIX && MODE != Mode::Fused ? tape + (int64_t)scen * w.paths + pc : nullptr;
+            const bool own = FIX && MODE == Mode::Forward && pc == pc0 + tid;       // a path to put on the tape
             float V;
             {
                 // ---- forward (path_calc_b1 :34-82) ----
-                const int64_t pc = tid < batch_left(w, item, jb) ? pc0 + tid : w.paths - 1;
-                const float *zp = PHILOX ? nullptr : z + pc * nmat;
+                const float *zp = PHILOX || TAPED ? nullptr : z + pc * nmat;
                 F2 disc{1.0f, 0.0f};              // the discount product, rates 0 .. nmat-1 in order
                 float R[kFR];
                 float *sq = sc + (size_t)Ly.s_q * B;
-                float *Bst = bsm ? vg0 + M * B : sc + (size_t)Ly.s_b * B, *ILst = vg0;
+                float *Bst = mode == Mode::Forward ? nullptr : bsm ? vg0 + M * B : sc + (size_t)Ly.s_b * B, *ILst = vg0;
+                if (TAPED) {
+#pragma unroll 8
+                    for (int i = 0; i < nn; ++i) {
+                        const float il = tp[i * total];
+                        if (i < nmat)
+                            disc = f2_mul(disc, bond_ratio(il, delta));
+                        else
+                            ILst[(i - nmat) * B] = il;
+                    }
+                }
 #pragma unroll 1
-                for (int ps = 0; ps < Ly.nf; ++ps) {
+                for (int ps = 0; ps < (TAPED ? 0 : Ly.nf); ++ps) {
                     const int LO = ps * kFR;
-                    const float *vin = sc + (size_t)(Ly.s_v + (2 * ps - 1) * nmat) * B;
+                    float *vin = sc + (size_t)(FIX ? Ly.s_v + (2 * ps - 1) * nmat : Ly.s_p) * B;
                     float *vo = sc + (size_t)(Ly.s_v + 2 * ps * nmat) * B;
 #pragma unroll
                     for (int i = 0; i < kFR; ++i) R[i] = FIX ? il0_s[LO + i] : 0.0f;
@@ -443,10 +467,25 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             V0h = V0;
                             V1h = V1;
                         }
-                        vo[n * B] = V0h;
-                        vo[(n + 1) * B] = V1h;
-                        vo[(nmat + n) * B] = V0;
-                        vo[(nmat + n + 1) * B] = V1;
+                        if (!FIX) {
+                            vin[n * B] = V0;
+                            vin[(n + 1) * B] = V1;
+                            V0 += q0;
+                            V1 += q1;
+                            V0h += q0;
+                            V1h += q1;
+                        }
+                        if (!FIX || MODE == Mode::Fused) {
+                            vo[n * B] = V0h;
+                            vo[(n + 1) * B] = V1h;
+                        }
+                        if (!FIX || MODE == Mode::Fused || ps + 1 < Ly.nf) {
+                            vo[(nmat + n) * B] = V0;
+                            vo[(nmat + n + 1) * B] = V1;
+                        } else if (own) {
+                            tp[(NN + n) * total] = V0;
+                            tp[(NN + n + 1) * total] = V1;
+                        }
                         if (!FIX && nck > 0 && (n + 2) % ck == 0 && n + 2 < nmat) {
                             // rates i <= n+2 are final from here on: only the others are saved
                             float *cp = sc + (size_t)(Ly.s_ck + ((n + 2) / ck - 1) * kRR * Ly.nr + LO) * B;
@@ -464,13 +503,17 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                         }
                         V0h = V0;
                         if (n - LO < kFR - 1) fwd_one_block<true>(R, kf - (n + 1) + LO, delta, q0, il0_s + LO, V0, V0h);
-                        vo[n * B] = V0h;
-                        vo[(nmat + n) * B] = V0;
+                        vin[n * B] = V0;
+                        vo[n * B] = V0h + q0;
+                        vo[(nmat + n) * B] = V0 + q0;
                     }
 #pragma unroll
                     for (int i = 0; i < kFR; ++i) {
                         const float il = FIX ? R[i] : il0_s[LO + i] * ex2_ulp(-R[i]);
-                        sc[(Ly.s_x + LO + i) * B] = il * inv_d;
+                        if (!FIX || MODE == Mode::Fused)
+                            sc[(Ly.s_x + LO + i) * B] = il * inv_d;
+                        else if (own)
+                            tp[(LO + i) * total] = il;
                         if (LO + i < nmat)
                             disc = FIX ? f2_mul(disc, bond_ratio(il, delta)) : f2_mul(disc, bond_ratio2(il, delta));
                         else if (LO + i < nn)
@@ -481,28 +524,30 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 unsigned long long mask;
                 float dsc;
                 V = payoff_forward_staged<B, !FIX>(M, disc, delta, ost_s, okk_s, owf_s, &dsc, Bst, ILst, &mask);
-                if (FIX || mode != Mode::Forward) {
+                if (mode != Mode::Forward) {
                     payoff_adjoint_stage<B>(M, vb, dsc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
 #pragma unroll 4
                     for (int i = 0; i < M; ++i) sc[(Ly.s_d + nmat + i) * B] = ILst[i * B];
                 }
             }
-            if (FIX || mode != Mode::Forward) {
+            if (mode != Mode::Forward) {
 #pragma unroll 8
                 for (int k = 0; k < kRR * Ly.nr; ++k) vg0[k * B] = 0.0f;
 
                 // ---- reverse: the blocks from the top, each over the steps with an active cell in it ----
                 float *su = sc + (size_t)Ly.s_s * B;
-                const float *sq = sc + (size_t)Ly.s_q * B;
                 const float nvs = -vb * V;
 #pragma unroll 1
                 for (int b = Ly.nr - 1; b >= 0; --b) {
                     const int LO = b * kRR;
                     const bool top = b == Ly.nr - 1;
-                    const float *vt = sc + (size_t)(Ly.s_v + b * nmat) * B;
+                    const float *vt = sc + (size_t)(Ly.s_v + (TAPED ? 0 : b * nmat)) * B;
+                    float *vn = sc + (size_t)Ly.s_v * B;       // TAPED: the drift sums / sqrt(delta) at the block's bottom
+                    const float vsc = TAPED && !top ? 1.0f : inv_sqd;
+                    auto drift = [&](int n) { return TAPED && top ? tp[(NN + n) * total] : vt[n * B]; };
                     float X[kRR], Pb[kRR];
 #pragma unroll
-                    for (int i = 0; i < kRR; ++i) X[i] = sc[(Ly.s_x + LO + i) * B];
+                    for (int i = 0; i < kRR; ++i) X[i] = TAPED ? tp[(LO + i) * total] * inv_d : sc[(Ly.s_x + LO + i) * B];
                     if (FIX && LO >= NMAT) {
 #pragma unroll
                         for (int i = 0; i < kRR; ++i) Pb[i] = sc[(Ly.s_d + LO + i) * B];
@@ -528,7 +573,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll 1
                         for (; (n + 1) % kRG != 0; --n) {
                             if (LO + kRR - 1 <= n) continue;
-                            TpbStep s1[1] = {{(vt[n * B] + sq[n * B]) * inv_sqd, top ? 0.0f : su[n * B]}};
+                            TpbStep s1[1] = {{drift(n) * vsc, top ? 0.0f : su[n * B]}};
                             back(n, rs, tl);
                             rev_block<B, 1, true>(X, Pb, s1, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
                             su[n * B] = s1[0].S;
@@ -539,7 +584,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     if (n > 0) {
 #pragma unroll
                         for (int g = 0; g < kRG; ++g) {
-                            nv[g] = FIX ? vt[(n - g) * B] : vt[(n - g) * B] + sq[(n - g) * B];
+                            nv[g] = drift(n - g);
                             ns[g] = top ? 0.0f : su[(n - g) * B];
                         }
                     }
@@ -547,11 +592,11 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     for (; n > 0; n -= kRG) {
                         TpbStep st[kRG];
 #pragma unroll
-                        for (int g = 0; g < kRG; ++g) st[g] = {nv[g] * inv_sqd, ns[g]};
+                        for (int g = 0; g < kRG; ++g) st[g] = {nv[g] * vsc, ns[g]};
                         if (n - kRG > 0) {
 #pragma unroll
                             for (int g = 0; g < kRG; ++g) {
-                                nv[g] = FIX ? vt[(n - kRG - g) * B] : vt[(n - kRG - g) * B] + sq[(n - kRG - g) * B];
+                                nv[g] = drift(n - kRG - g);
                                 ns[g] = top ? 0.0f : su[(n - kRG - g) * B];
                             }
                         }
@@ -559,7 +604,10 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                         rev_block<B, kRG, !FIX>(X, Pb, st, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
                         if (b > 0) {
 #pragma unroll
-                            for (int g = 0; g < kRG; ++g) su[(n - g) * B] = st[g].S;
+                            for (int g = 0; g < kRG; ++g) {
+                                su[(n - g) * B] = st[g].S;
+                                if (TAPED) vn[(n - g) * B] = st[g].y;
+                            }
                         }
                     }
 #pragma unroll
@@ -569,7 +617,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 
             // ---- cross-path reduction of this batch ----
             const bool active = tid < batch_left(w, item, jb);
-            if (FIX || mode != Mode::Backward) {
+            if (mode != Mode::Backward) {
                 const float v = active ? V : 0.0f;
                 const float s1 = warp_sum(v), s2 = warp_sum(v * v);
                 if (lane == 0) {
@@ -577,8 +625,8 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     acc[nout] += (double)s2;
                 }
             }
-            if (FIX || mode != Mode::Forward) {
-                const int off = FIX || mode == Mode::Fused ? 1 : 0;
+            if (mode != Mode::Forward) {
+                const int off = mode == Mode::Fused ? 1 : 0;
                 float *vgw = vg_s + kRG * B;
                 if (!active) {
 #pragma unroll 1
@@ -596,35 +644,39 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
         }
 
         __syncthreads();
-        const int voff = FIX || mode == Mode::Fused ? 1 + nn : nn;
+        const int voff = mode == Mode::Fused ? 1 + nn : nn;
         for (int o = tid; o < 2 * nout; o += B) {
             double s2 = 0.0;
 #pragma unroll
             for (int q = 0; q < NW; ++q) s2 += acc_s[q * 2 * nout + o];
             // vegas per lambda: sqrt(delta) times those per sigma, delta times their squares
-            if ((FIX || mode != Mode::Forward) && (o < nout ? o >= voff : o - nout >= voff)) s2 *= o < nout ? m.sqdd : m.deltad;
+            if (mode != Mode::Forward && (o < nout ? o >= voff : o - nout >= voff)) s2 *= o < nout ? m.sqdd : m.deltad;
             w.partial[(size_t)unit * 2 * nout + o] = s2;
         }
     }  // units
 }
 
-template <int NN, int NMAT, int B>
+template <int NN, int NMAT, int B, Mode MODE = Mode::Fused>
 cudaError_t launch_tpb(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox, const Work &w,
-                       float *scr, const double *vbar, cudaStream_t s)
+                       float *scr, float *tape, const double *vbar, cudaStream_t s)
 {
     const int bytes = tpb_layout(m.nn, m.nmat, mode, B).bytes;
-    auto kern = philox ? k_tpb<NN, NMAT, B, true> : k_tpb<NN, NMAT, B, false>;
+    auto kern = k_tpb<NN, NMAT, B, false, MODE>;
+    if constexpr (MODE == Mode::Fused)
+        if (philox) kern = k_tpb<NN, NMAT, B, true, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)w.grid, B, bytes, s>>>(m, z, seed, path0, w, scr, vbar, (int)mode);
+    kern<<<(unsigned)w.grid, B, bytes, s>>>(m, z, seed, path0, w, scr, tape, vbar, (int)mode);
     return cudaGetLastError();
 }
 
-template <int NN, int NMAT, int B>
+template <int NN, int NMAT, int B, Mode MODE = Mode::Fused>
 cudaError_t occ_tpb(int nn, int nmat, Mode mode, bool philox, int *blocks)
 {
     const int bytes = tpb_layout(nn, nmat, mode, B).bytes;
-    auto kern = philox ? k_tpb<NN, NMAT, B, true> : k_tpb<NN, NMAT, B, false>;
+    auto kern = k_tpb<NN, NMAT, B, false, MODE>;
+    if constexpr (MODE == Mode::Fused)
+        if (philox) kern = k_tpb<NN, NMAT, B, true, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, B, bytes);

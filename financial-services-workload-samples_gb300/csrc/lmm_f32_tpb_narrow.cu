@@ -6,8 +6,8 @@ namespace lmm {
 cudaError_t launch_tpb_narrow(int B, const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
                           const Work &w, float *scr, const double *vbar, cudaStream_t s)
 {
-    return B == 256 ? launch_tpb<0, 0, 256>(m, mode, z, seed, path0, philox, w, scr, vbar, s)
-                    : launch_tpb<0, 0, 128>(m, mode, z, seed, path0, philox, w, scr, vbar, s);
+    return B == 256 ? launch_tpb<0, 0, 256>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s)
+                    : launch_tpb<0, 0, 128>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s);
 }
 
 cudaError_t occ_tpb_narrow(int B, int nn, int nmat, Mode mode, bool philox, int *blocks)

@@ -1326,40 +1326,13 @@ cudaError_t launch_tpq_any(const DevModel &m, const float *z, uint64_t seed, int
                   : launch_tpq<160, 120, false>(m, z, seed, path0, w, scratch, s);
 }
 
-int tpp_block_threads(Mode mode)
-{
-    return mode == Mode::Fused ? tpp_block<Mode::Fused>()
-                               : (mode == Mode::Forward ? tpp_block<Mode::Forward>() : tpp_block<Mode::Backward>());
-}
+int tpp_block_threads() { return tpp_block<Mode::Fused>(); }
 
-#define LMM_TPP_DISPATCH(FN, ...)                                                            \
-    do {                                                                                     \
-        if (philox) {                                                                        \
-            switch (mode) {                                                                  \
-                case Mode::Fused: break;                                                     \
-                case Mode::Forward: return FN<80, 40, true, Mode::Forward>(__VA_ARGS__);     \
-                case Mode::Backward: return FN<80, 40, true, Mode::Backward>(__VA_ARGS__);   \
-            }                                                                                \
-        } else {                                                                             \
-            switch (mode) {                                                                  \
-                case Mode::Fused: return FN<80, 40, false, Mode::Fused>(__VA_ARGS__);        \
-                case Mode::Forward: return FN<80, 40, false, Mode::Forward>(__VA_ARGS__);    \
-                case Mode::Backward: return FN<80, 40, false, Mode::Backward>(__VA_ARGS__);  \
-            }                                                                                \
-        }                                                                                    \
-        return cudaErrorInvalidValue;                                                        \
-    } while (0)
+cudaError_t tpp_blocks_per_sm(int *blocks) { return occ_tpp<80, 40, false, Mode::Fused>(blocks); }
 
-cudaError_t tpp_blocks_per_sm(Mode mode, bool philox, int *blocks)
+cudaError_t launch_tpp_any(const DevModel &m, const float *z, const Work &w, cudaStream_t s)
 {
-    LMM_TPP_DISPATCH(occ_tpp, blocks);
-}
-
-cudaError_t launch_tpp_any(const DevModel &m, Mode mode, const float *z, uint64_t seed,
-                           int64_t path0, bool philox, const Work &w, float *tape,
-                           const double *vbar, cudaStream_t s)
-{
-    LMM_TPP_DISPATCH(launch_tpp, m, z, seed, path0, w, tape, vbar, s);
+    return launch_tpp<80, 40, false, Mode::Fused>(m, z, 0, 0, w, nullptr, nullptr, s);
 }
 
 }  // namespace lmm

@@ -60,23 +60,23 @@ enum class Mode : int { Fused = 0, Forward = 1, Backward = 2 };
 int record_error(int status, const char *what);
 int record_cuda_error(cudaError_t e, const char *what);
 
-// FP32 thread-per-path kernels (lmm_f32_tpp.cu, NN=80, NMAT=40).
+// FP32 thread-per-path kernel without scratch (lmm_f32_tpp.cu, NN=80, NMAT=40):
+// the no-allocation call.
 bool f32_tpp_supports(int nn, int nmat);
-int tpp_block_threads(Mode mode);     // threads per block = paths per batch
-cudaError_t tpp_blocks_per_sm(Mode mode, bool philox, int *blocks);
-cudaError_t launch_tpp_any(const DevModel &m, Mode mode, const float *z, uint64_t seed,
-                           int64_t path0, bool philox, const Work &w, float *tape,
-                           const double *vbar, cudaStream_t s);
-// FP32 thread-per-path kernels in rate blocks (lmm_f32_tpb.cuh, k_tpb): the
-// fused 80/40 call, and every mode of other shapes whose checkpoint interval is
-// a multiple of 4. A per-block scratch of tpb_scratch_floats_per_block floats.
+int tpp_block_threads();              // threads per block = paths per batch
+cudaError_t tpp_blocks_per_sm(int *blocks);
+cudaError_t launch_tpp_any(const DevModel &m, const float *z, const Work &w, cudaStream_t s);
+// FP32 thread-per-path kernels in rate blocks (lmm_f32_tpb.cuh, k_tpb): every
+// mode of 80/40 (the pair on a tape) and of other shapes whose checkpoint interval
+// is a multiple of 4. A per-block scratch of tpb_scratch_floats_per_block floats.
 bool f32_tpb_supports(int nn, int nmat, int ckpt);
 int tpb_block_threads(int nn, int nmat);
 int tpb_cells(int nn, int nmat);
+int tpb_tape_rows(int nn, int nmat);
 size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt);
 cudaError_t tpb_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks);
 cudaError_t launch_tpb_any(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
-                           const Work &w, float *scratch, const double *vbar, cudaStream_t s);
+                           const Work &w, float *scratch, float *tape, const double *vbar, cudaStream_t s);
 // The fused 160/120 kernel with one thread per path and the reverse in passes
 // over blocks of 40 rates (lmm_f32_tpp.cu, k_tpq): a per-block scratch of
 // tpq_scratch_floats_per_block floats; checkpoint intervals multiples of 4.

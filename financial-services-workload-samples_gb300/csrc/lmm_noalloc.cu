@@ -132,7 +132,7 @@ int setup_device(int dev, DeviceSetup *out)
         int sms = 0, bps = 0;
         ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "cudaDeviceGetAttribute");
-        ce = lmm::tpp_blocks_per_sm(lmm::Mode::Fused, false, &bps);
+        ce = lmm::tpp_blocks_per_sm(&bps);
         if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "occupancy query");
         if (bps < 1) return lmm::record_error(LMM_ERR_UNSUPPORTED, "the fused kernel does not fit on this device");
         s.scratch = static_cast<unsigned char *>(ptr);
@@ -196,7 +196,7 @@ extern "C" int lmm_greeks_f32_device_noalloc(const lmm_params *p, const float *d
     }
 
     // About two waves of the device, capped by the partial-sum space.
-    const int64_t block = lmm::tpp_block_threads(lmm::Mode::Fused);
+    const int64_t block = lmm::tpp_block_threads();
     const int64_t nscen = p->nscen;
     int64_t items = (2 * (int64_t)ds.sms * ds.bps + nscen - 1) / nscen;
     if (items * nscen > kMaxItems) items = kMaxItems / nscen;
@@ -241,7 +241,7 @@ extern "C" int lmm_greeks_f32_device_noalloc(const lmm_params *p, const float *d
     w.partial = partial;
     w.nout = kNout;
 
-    ce = lmm::launch_tpp_any(m, lmm::Mode::Fused, d_z, 0, 0, false, w, nullptr, nullptr, st);
+    ce = lmm::launch_tpp_any(m, d_z, w, st);
     if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "FP32 LMM kernel launch");
     ce = lmm::launch_finalize(partial, p->nscen, w.items, kNout, paths, d_out, d_se, flag, 1, st);
     if (ce != cudaSuccess) return lmm::record_cuda_error(ce, "finalize launch");
