@@ -217,8 +217,7 @@ bool ragged_batches(int fam) { return fam == 2 || fam == 6; }
 
 // Time of a ragged batch of n paths relative to a full one. GB300, one batch
 // per SM, 80/40, one / two / three / four warps per scheduler: k_tpb
-// 0.092, 0.120, 0.150, 0.187 ms (a linear fit; other shapes alike, 20,000 paths of
-// 128/100 in one batch 0.586 ms, in two 0.860).
+// 0.092, 0.120, 0.150, 0.187 ms (a linear fit, which serves the other shapes too).
 double batch_cost(int fam, int n, int batch)
 {
     const int wps = (n + 127) / 128, full = batch / 128;
@@ -267,18 +266,19 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
 // 0.393; the pair, which has to go with the fused call, puts the line at 1.33
 // fills. Shapes in rate blocks: the ratio of the two estimates in us, fitted to
 // whole calls of 13 shapes, of which a warp per path / rate blocks took, at
-// 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line at 2.9 fills), 0.246 / 0.416
-// (128/100; 2.9), 0.109 / 0.160 (64/50; 2.4), 0.086 / 0.113 (60/30; 2.2), 0.098 /
-// 0.100 and for the pair 0.158 / 0.132 (80/40; 1.3), 0.055 / 0.057 (40/10; 1.4).
-// Above 160 rates a lane's eight rates collide on the banks: one fill (3,600
-// paths, 161/100 0.61 / 0.55, 256/40 0.42 / 0.44).
+// 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line at 2.9 fills), 0.109 / 0.160
+// (64/50; 2.4), 0.086 / 0.113 (60/30; 2.2), 0.098 / 0.100 and for the pair 0.158 /
+// 0.132 (80/40; 1.3), 0.055 / 0.057 (40/10; 1.4), and with a window of vega rows, at
+// 11,000, 0.454 / 0.592 (128/100; 4). Above 160 rates a lane's eight rates collide on
+// the banks: two fills (5,600 paths, 161/100 0.94 / 0.76, 256/40 0.82 / 0.64; 3,600,
+// 256/119 1.04 / 1.37).
 double wpp_fills(int nn, int nmat, bool rate_blocks)
 {
     if (!rate_blocks) return 4.0 / 3.0;
     const int slots = lmm::wpp_slots(nn);
-    if (slots > 5) return 1.0;
-    const double blocks = 25.0 + (nn == 80 && nmat == 40 ? 0.0088 : 0.0175) * lmm::tpb_cells(nn, nmat);
-    return std::min(4.0, std::max(1.0, blocks / (20.0 + nmat * (0.5 + 0.15 * slots))));
+    if (slots > 5) return 2.0;
+    const double cell = nn == 80 && nmat == 40 ? 0.0088 : lmm::tpb_windowed(nn, nmat) ? 0.025 : 0.0175;
+    return std::min(4.0, std::max(1.0, (25.0 + cell * lmm::tpb_cells(nn, nmat)) / (20.0 + nmat * (0.5 + 0.15 * slots))));
 }
 
 // The family of a call of `paths` paths: the warp-per-path kernels for few paths,

@@ -1,29 +1,41 @@
-// Instances and dispatch of the rate-block kernel (lmm_f32_tpb.cuh).
+// Instances and dispatch of the rate-block kernel (lmm_f32_tpb.cuh): 80/40, whose
+// forward rounds as the no-allocation call's.
 #include "lmm_f32_tpb.cuh"
 
 #include <algorithm>
 
 namespace lmm {
 
+namespace {
+
+bool is_tape_shape(int nn, int nmat) { return nn == 80 && nmat == 40; }
+
+bool fits(int nn, int nmat, int B, bool win) { return tpb_layout(nn, nmat, Mode::Fused, B, win).bytes <= 227 * 1024; }
+
+}  // namespace
+
 // The shape whose forward/backward pair runs on a tape (k_tpb): rows of it; 0:
 // the backward runs the forward again.
-int tpb_tape_rows(int nn, int nmat) { return nn == 80 && nmat == 40 ? nn + nmat : 0; }
+int tpb_tape_rows(int nn, int nmat) { return is_tape_shape(nn, nmat) ? nn + nmat : 0; }
 
-// Threads per block: registers allow 512, 384, 256 threads (16, 12, 8 warps an
-// SM), the vega rows of a block's paths have to fit in shared memory. 0: no
-// block fits.
-int tpb_block_threads(int nn, int nmat)
-{
-    for (int B : {512, 384, 256, 128})
-        if (tpb_layout(nn, nmat, Mode::Fused, B).bytes <= 227 * 1024) return B;
-    return 0;
-}
+// Registers allow 512 threads a block (16 warps an SM). Where the vega rows of 512
+// paths and the warps' sums do not fit in shared memory, 384 threads where theirs
+// do, and else 512 with the rows in a window. GB300, 50,001 paths of 96/60: 0.393 ms
+// with 384 threads, 0.498 in a window; 20,000 / 65,000 paths, 256 threads (128 above
+// 156 rates) against the window: 128/100 0.586 / 1.790 against 0.740 / 1.129 ms,
+// 161/100 1.157 / 2.464 against 0.982 / 1.500, 256/119 2.13 / 4.60 against 1.91 /
+// 2.71. The window costs its rows' way from and to the scratch, which is latency
+// where the warps are few.
+bool tpb_windowed(int nn, int nmat) { return !fits(nn, nmat, 512, false) && !fits(nn, nmat, 384, false); }
+
+int tpb_block_threads(int nn, int nmat) { return fits(nn, nmat, 512, false) || tpb_windowed(nn, nmat) ? 512 : 384; }
 
 size_t tpb_scratch_floats_per_block(int nn, int nmat, int ckpt)
 {
-    const TpbLay L = tpb_layout(nn, nmat, Mode::Fused, 32);      // rows
+    const int B = tpb_block_threads(nn, nmat);
+    const TpbLay L = tpb_layout(nn, nmat, Mode::Fused, B, tpb_windowed(nn, nmat));
     const int nck = ckpt > 0 ? (nmat - 1) / ckpt : 0;
-    return (size_t)(L.s_ck + nck * kRR * L.nr) * tpb_block_threads(nn, nmat);
+    return (size_t)(L.s_ck + nck * kRR * L.nr) * B;
 }
 
 // Cells that one path walks, no-ops of partly active passes and blocks among them:
@@ -37,41 +49,44 @@ int tpb_cells(int nn, int nmat)
 }
 
 // Checkpoints are restored between groups of steps.
-bool f32_tpb_supports(int nn, int nmat, int ckpt) { return tpb_block_threads(nn, nmat) > 0 && ckpt % kRG == 0; }
+bool f32_tpb_supports(int nn, int nmat, int ckpt)
+{
+    return fits(nn, nmat, tpb_block_threads(nn, nmat), tpb_windowed(nn, nmat)) && ckpt % kRG == 0;
+}
 
-// The instances for shapes at run time (lmm_f32_tpb_wide.cu, lmm_f32_tpb_narrow.cu).
-cudaError_t launch_tpb_wide(int B, const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
-                            const Work &w, float *scr, const double *vbar, cudaStream_t s);
-cudaError_t launch_tpb_narrow(int B, const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
+// The instances for shapes at run time (lmm_f32_tpb_shape.cu, lmm_f32_tpb_window.cu).
+cudaError_t launch_tpb_shape(int B, const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
+                             const Work &w, float *scr, const double *vbar, cudaStream_t s);
+cudaError_t launch_tpb_window(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
                               const Work &w, float *scr, const double *vbar, cudaStream_t s);
-cudaError_t occ_tpb_wide(int B, int nn, int nmat, Mode mode, bool philox, int *blocks);
-cudaError_t occ_tpb_narrow(int B, int nn, int nmat, Mode mode, bool philox, int *blocks);
+cudaError_t occ_tpb_shape(int B, int nn, int nmat, Mode mode, bool philox, int *blocks);
+cudaError_t occ_tpb_window(int nn, int nmat, Mode mode, bool philox, int *blocks);
 
 cudaError_t tpb_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks)
 {
-    if (nn == 80 && nmat == 40) {
-        if (mode == Mode::Forward) return occ_tpb<80, 40, 512, Mode::Forward>(nn, nmat, mode, philox, blocks);
-        if (mode == Mode::Backward) return occ_tpb<80, 40, 512, Mode::Backward>(nn, nmat, mode, philox, blocks);
-        return occ_tpb<80, 40, 512>(nn, nmat, mode, philox, blocks);
+    if (is_tape_shape(nn, nmat)) {
+        if (mode == Mode::Forward) return occ_tpb<80, 40, 512, false, Mode::Forward>(nn, nmat, mode, philox, blocks);
+        if (mode == Mode::Backward) return occ_tpb<80, 40, 512, false, Mode::Backward>(nn, nmat, mode, philox, blocks);
+        return occ_tpb<80, 40, 512, false>(nn, nmat, mode, philox, blocks);
     }
-    const int B = tpb_block_threads(nn, nmat);
-    return B >= 384 ? occ_tpb_wide(B, nn, nmat, mode, philox, blocks) : occ_tpb_narrow(B, nn, nmat, mode, philox, blocks);
+    return tpb_windowed(nn, nmat) ? occ_tpb_window(nn, nmat, mode, philox, blocks)
+                                  : occ_tpb_shape(tpb_block_threads(nn, nmat), nn, nmat, mode, philox, blocks);
 }
 
 cudaError_t launch_tpb_any(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
                            const Work &w, float *scr, float *tape, const double *vbar, cudaStream_t s)
 {
-    if (m.nn == 80 && m.nmat == 40) {
+    if (is_tape_shape(m.nn, m.nmat)) {
         if (mode != Mode::Fused && !tape) return cudaErrorInvalidValue;
         if (mode == Mode::Forward)
-            return launch_tpb<80, 40, 512, Mode::Forward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
+            return launch_tpb<80, 40, 512, false, Mode::Forward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
         if (mode == Mode::Backward)
-            return launch_tpb<80, 40, 512, Mode::Backward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
-        return launch_tpb<80, 40, 512>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s);
+            return launch_tpb<80, 40, 512, false, Mode::Backward>(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
+        return launch_tpb<80, 40, 512, false>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s);
     }
-    const int B = tpb_block_threads(m.nn, m.nmat);
-    return B >= 384 ? launch_tpb_wide(B, m, mode, z, seed, path0, philox, w, scr, vbar, s)
-                    : launch_tpb_narrow(B, m, mode, z, seed, path0, philox, w, scr, vbar, s);
+    return tpb_windowed(m.nn, m.nmat)
+               ? launch_tpb_window(m, mode, z, seed, path0, philox, w, scr, vbar, s)
+               : launch_tpb_shape(tpb_block_threads(m.nn, m.nmat), m, mode, z, seed, path0, philox, w, scr, vbar, s);
 }
 
 }  // namespace lmm

@@ -35,7 +35,11 @@
 // slower with 20 warps of 96 registers.
 //
 // Other shapes, against the kernel that gave a path two threads or a warp: 50,001
-// paths of 96/60 0.96 -> 0.393 ms.
+// paths of 96/60 0.96 -> 0.393 ms; 65,000 paths of 161/100 (vega rows in a window)
+// 10.1 -> 1.51 ms, with blocks of 128 threads instead of the window 2.46. 160/120 in
+// this kernel, with its rate checkpoints, ran 1,048,576 paths in 15.0 ms (k_tpq
+// 14.2): the scratch of 512 paths an SM does not stay in L2 (ncu: 2.3 TB/s from
+// DRAM, a fifth of the warps' time waiting for it).
 //
 // The reverse runs in units of sigma = lambda sqrt(delta): with X = 1/(delta L),
 // t = 1/(X + 1), y = (drift sum + normal term)/sqrt(delta) a cell is
@@ -53,23 +57,28 @@ namespace {
 
 constexpr int kFR = 40, kFC = 8;       // forward: rates per pass, and per chunk of its body
 constexpr int kRR = 20, kRG = 4;       // reverse: rates per block, steps per group
+constexpr int kSeg = 64;               // most steps that a window of vega rows spans, a multiple of kRG
 constexpr float kPadIL = 1e15f;        // inverse rate of the padding above rate nn: t = 0 beside any sum
 
 // Sizes and offsets of one shape, in rows of B values where B counts threads.
 struct TpbLay {
     int nn, nmat, M, nf, nr;           // nf forward passes, nr reverse blocks
-    int nout;
+    int nout, seg;                     // seg: steps that the window of vega rows spans (WIN)
     // shared memory, bytes
     int kf, kr, il0, ost, okf, owf, okk, vg, acc, bytes;
     // scratch, rows: drift sums at the top of every half pass [2 nf][nmat], suffix sums at the bottom of the
     // reverse block last run [nmat], rates [kFR nf], log-adjoints, then deltas [kRR nr], annuity factors [M],
-    // drift sums without the normal terms at the top of the pass last run [nmat], normal terms [nmat], checkpoints [nck][kRR nr]
-    int s_v, s_s, s_x, s_d, s_b, s_p, s_q, s_ck;
+    // drift sums without the normal terms at the top of the pass last run [nmat], normal terms [nmat], vegas [kRR nr]
+    // and sums (WIN), checkpoints [nck][kRR nr]
+    int s_v, s_s, s_x, s_d, s_b, s_p, s_q, s_g, s_a, s_ck;
 };
 
 __host__ __device__ constexpr int tpb_al(int x) { return (x + 15) & ~15; }
 
-__host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int B)
+// Rows of a window that spans seg steps.
+__host__ __device__ constexpr int tpb_win(int seg) { return seg + kRR - 1; }
+
+__host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int B, bool win)
 {
     TpbLay L{};
     L.nn = nn;
@@ -78,6 +87,8 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
     L.nf = (nn + kFR - 1) / kFR;
     L.nr = (nn + kRR - 1) / kRR;
     L.nout = mode == Mode::Fused ? 1 + 2 * nn : (mode == Mode::Forward ? 1 : 2 * nn);
+    const int nseg = (nmat + kSeg - 1) / kSeg;
+    L.seg = ((nmat + nseg - 1) / nseg + kRG - 1) / kRG * kRG;
     const int kc = nmat + kFR * L.nf;                       // NMAT zero rows (k < 0), then k = 0 ..
     L.kf = 0;
     L.kr = L.kf + 16 * kc;
@@ -87,9 +98,9 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
     L.owf = L.okf + 4 * kMaxNopt;
     L.okk = L.owf + 4 * kMaxNopt;
     L.vg = L.okk + 8 * kMaxNopt;
-    const int rows = kRG + kRR * L.nr;                      // kRG spare rows for k < 0
+    const int rows = win ? tpb_win(L.seg) : kRG + kRR * L.nr;           // kRG spare rows for k < 0
     L.acc = L.vg + 4 * rows * B;
-    L.bytes = L.acc + 8 * (B / 32) * 2 * L.nout;
+    L.bytes = L.acc + (win ? 0 : 8 * (B / 32) * 2 * L.nout);
     L.s_v = 0;
     L.s_s = 2 * L.nf * nmat;
     L.s_x = L.s_s + nmat;
@@ -97,7 +108,9 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
     L.s_b = L.s_d + kRR * L.nr;
     L.s_p = L.s_b + L.M;
     L.s_q = L.s_p + nmat;
-    L.s_ck = L.s_q + nmat;
+    L.s_g = L.s_q + nmat;
+    L.s_a = L.s_g + (win ? kRR * L.nr : 0);
+    L.s_ck = L.s_a + (win ? (1 + 2 * nn + 7) / 8 : 0);      // 2 nout doubles a warp
     return L;
 }
 
@@ -333,21 +346,26 @@ __device__ __forceinline__ void column_sums(int nn, const float *vg, int warp, i
 }
 
 // NN, NMAT, MODE: the shape and mode, or 0 for a shape at run time (any mode,
-// `mode_arg`; rate checkpoints every m.ckpt steps, a multiple of kRG, or none).
-// The forward of a fixed shape writes the tape, [NN][total] terminal inverse rates
-// and [NMAT][total] drift sums at the top rate, and its backward reads it: what the
-// reverse of one block has for the drift sums at its bottom is where the block
-// below starts.
-template <int NN, int NMAT, int B, bool PHILOX, Mode MODE>
+// `mode_arg`).
+// WIN: the vega rows of B paths don't fit in shared memory. They wait in the
+// scratch, and the reverse brings those that up to kSeg steps of a block touch into
+// a window and takes them back; the warps' sums lie in the scratch too.
+// Without WIN, the forward of a fixed shape writes the tape, [NN][total] terminal
+// inverse rates and [NMAT][total] drift sums at the top rate, and its backward reads
+// it: what the reverse of one block has for the drift sums at its bottom is where
+// the block below starts. All others restore rates every m.ckpt steps (a multiple of
+// kRG, or 0: never).
+template <int NN, int NMAT, int B, bool WIN, bool PHILOX, Mode MODE>
 __global__ void __launch_bounds__(B, 1)
 k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w, float *__restrict__ scr,
       float *__restrict__ tape, const double *__restrict__ vbar, int mode_arg)
 {
     constexpr bool FIX = NN > 0;
-    constexpr bool TAPED = FIX && MODE == Mode::Backward;
+    constexpr bool LOGS = !FIX, CK = !FIX || WIN;
+    constexpr bool TAPED = !CK && MODE == Mode::Backward;
     constexpr int NW = B / 32;
     const Mode mode = FIX ? MODE : (Mode)mode_arg;
-    const TpbLay Ly = FIX ? tpb_layout(NN, NMAT, MODE, B) : tpb_layout(m.nn, m.nmat, mode, B);
+    const TpbLay Ly = FIX ? tpb_layout(NN, NMAT, MODE, B, WIN) : tpb_layout(m.nn, m.nmat, mode, B, WIN);
     const int nn = Ly.nn, nmat = Ly.nmat, M = Ly.M, nout = Ly.nout;
     extern __shared__ __align__(16) unsigned char smem[];
     float4 *kf_s = reinterpret_cast<float4 *>(smem + Ly.kf), *kr_s = reinterpret_cast<float4 *>(smem + Ly.kr);
@@ -357,7 +375,10 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     float *owf_s = reinterpret_cast<float *>(smem + Ly.owf);
     F2 *okk_s = reinterpret_cast<F2 *>(smem + Ly.okk);
     float *vg_s = reinterpret_cast<float *>(smem + Ly.vg);
-    double *acc_s = reinterpret_cast<double *>(smem + Ly.acc);
+    const int ck = CK && m.ckpt > 0 ? m.ckpt : Ly.nmat, nck = CK ? (Ly.nmat - 1) / ck : 0;
+    const int rows = Ly.s_ck + nck * kRR * Ly.nr;
+    float *sb = scr + (size_t)blockIdx.x * rows * B;
+    double *acc_s = WIN ? reinterpret_cast<double *>(sb + (size_t)Ly.s_a * B) : reinterpret_cast<double *>(smem + Ly.acc);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < nmat + kFR * Ly.nf; i += B) {
@@ -381,12 +402,10 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     const float delta = m.delta, sqd = m.sqd;
     const float inv_d = (float)(1.0 / m.deltad), inv_sqd = (float)(1.0 / m.sqdd);
     const float4 *kf = kf_s + nmat, *kr = kr_s + nmat;
-    float *vg0 = vg_s + kRG * B + tid;
-    const int ck = !FIX && m.ckpt > 0 ? m.ckpt : nmat, nck = (nmat - 1) / ck;
-    const int rows = Ly.s_ck + (FIX ? 0 : nck * kRR * Ly.nr);
-    float *sc = scr + (size_t)blockIdx.x * rows * B + tid;          // sc[row * B]
+    float *vg0 = vg_s + (WIN ? 0 : kRG * B) + tid;
+    float *sc = sb + tid;                                            // sc[row * B]
     const bool vec = FIX ? NMAT % 4 == 0 : (nmat & 3) == 0;
-    const bool bsm = FIX ? 2 * (NN - NMAT) <= kRR * ((NN + kRR - 1) / kRR) : false;   // annuity factors in shared memory
+    const bool bsm = FIX ? 2 * (NN - NMAT) <= (WIN ? tpb_win(Ly.seg) : kRR * ((NN + kRR - 1) / kRR)) : false;   // annuity factors in shared memory
 
     const int units = m.nscen * w.items;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
@@ -403,8 +422,8 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             const int64_t pc0 = (int64_t)item * w.ipaths + (int64_t)jb * w.bpaths;
             const int64_t pc = tid < batch_left(w, item, jb) ? pc0 + tid : w.paths - 1;
             const int64_t total = (int64_t)m.nscen * w.paths;         // the tape's row
-            float *tp = FIX && MODE != Mode::Fused ? tape + (int64_t)scen * w.paths + pc : nullptr;
-            const bool own = FIX && MODE == Mode::Forward && pc == pc0 + tid;       // a path to put on the tape
+            float *tp = !CK && MODE != Mode::Fused ? tape + (int64_t)scen * w.paths + pc : nullptr;
+            const bool own = !CK && MODE == Mode::Forward && pc == pc0 + tid;       // a path to put on the tape
             float V;
             {
                 // ---- forward (path_calc_b1 :34-82) ----
@@ -412,7 +431,9 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 F2 disc{1.0f, 0.0f};              // the discount product, rates 0 .. nmat-1 in order
                 float R[kFR];
                 float *sq = sc + (size_t)Ly.s_q * B;
-                float *Bst = mode == Mode::Forward ? nullptr : bsm ? vg0 + M * B : sc + (size_t)Ly.s_b * B, *ILst = vg0;
+                float *Bst = mode == Mode::Forward ? nullptr : bsm ? vg0 + M * B : sc + (size_t)Ly.s_b * B;
+                const bool ilsm = !WIN || M <= tpb_win(Ly.seg);
+                float *ILst = ilsm ? vg0 : sc + (size_t)(Ly.s_d + nmat) * B;
                 if (TAPED) {
 #pragma unroll 8
                     for (int i = 0; i < nn; ++i) {
@@ -426,10 +447,10 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll 1
                 for (int ps = 0; ps < (TAPED ? 0 : Ly.nf); ++ps) {
                     const int LO = ps * kFR;
-                    float *vin = sc + (size_t)(FIX ? Ly.s_v + (2 * ps - 1) * nmat : Ly.s_p) * B;
+                    float *vin = sc + (size_t)(LOGS ? Ly.s_p : Ly.s_v + (2 * ps - 1) * nmat) * B;
                     float *vo = sc + (size_t)(Ly.s_v + 2 * ps * nmat) * B;
 #pragma unroll
-                    for (int i = 0; i < kFR; ++i) R[i] = FIX ? il0_s[LO + i] : 0.0f;
+                    for (int i = 0; i < kFR; ++i) R[i] = LOGS ? 0.0f : il0_s[LO + i];
                     TpbNormals<PHILOX> zs{zp, seed, (uint64_t)(path0 + pc), nmat, vec};
                     float nv0 = 0.0f, nv1 = 0.0f, nq0 = 0.0f, nq1 = 0.0f;
                     if (ps == 0) {
@@ -437,7 +458,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     } else {
                         nv0 = vin[0];
                         if (nmat > 1) nv1 = vin[B];
-                        if (!FIX) {
+                        if (LOGS) {
                             nq0 = sq[0];
                             if (nmat > 1) nq1 = sq[B];
                         }
@@ -447,9 +468,9 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                         float V0, V1, V0h, V1h, q0 = nq0, q1 = nq1;
                         if (ps == 0) {
                             zs.pair(n, sqd, q0, q1);
-                            V0 = FIX ? q0 : 0.0f;
-                            V1 = FIX ? q1 : 0.0f;
-                            if (!FIX) {
+                            V0 = LOGS ? 0.0f : q0;
+                            V1 = LOGS ? 0.0f : q1;
+                            if (LOGS) {
                                 sq[n * B] = q0;
                                 sq[(n + 1) * B] = q1;
                             }
@@ -458,16 +479,16 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             V1 = nv1;
                             if (n + 2 < nmat) nv0 = vin[(n + 2) * B];
                             if (n + 3 < nmat) nv1 = vin[(n + 3) * B];
-                            if (!FIX && n + 2 < nmat) nq0 = sq[(n + 2) * B];
-                            if (!FIX && n + 3 < nmat) nq1 = sq[(n + 3) * B];
+                            if (LOGS && n + 2 < nmat) nq0 = sq[(n + 2) * B];
+                            if (LOGS && n + 3 < nmat) nq1 = sq[(n + 3) * B];
                         }
                         if (n - LO < kFR - 1) {
-                            fwd_pair_block<!FIX>(R, kf - (n + 1) + LO, delta, n - LO, q0, q1, il0_s + LO, V0, V1, V0h, V1h);
+                            fwd_pair_block<LOGS>(R, kf - (n + 1) + LO, delta, n - LO, q0, q1, il0_s + LO, V0, V1, V0h, V1h);
                         } else {                 // no rate of the pass moves
                             V0h = V0;
                             V1h = V1;
                         }
-                        if (!FIX) {
+                        if (LOGS) {
                             vin[n * B] = V0;
                             vin[(n + 1) * B] = V1;
                             V0 += q0;
@@ -475,23 +496,23 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             V0h += q0;
                             V1h += q1;
                         }
-                        if (!FIX || MODE == Mode::Fused) {
+                        if (CK || MODE == Mode::Fused) {
                             vo[n * B] = V0h;
                             vo[(n + 1) * B] = V1h;
                         }
-                        if (!FIX || MODE == Mode::Fused || ps + 1 < Ly.nf) {
+                        if (CK || MODE == Mode::Fused || ps + 1 < Ly.nf) {
                             vo[(nmat + n) * B] = V0;
                             vo[(nmat + n + 1) * B] = V1;
                         } else if (own) {
                             tp[(NN + n) * total] = V0;
                             tp[(NN + n + 1) * total] = V1;
                         }
-                        if (!FIX && nck > 0 && (n + 2) % ck == 0 && n + 2 < nmat) {
+                        if (CK && nck > 0 && (n + 2) % ck == 0 && n + 2 < nmat) {
                             // rates i <= n+2 are final from here on: only the others are saved
                             float *cp = sc + (size_t)(Ly.s_ck + ((n + 2) / ck - 1) * kRR * Ly.nr + LO) * B;
 #pragma unroll
                             for (int i = 0; i < kFR; ++i)
-                                if (LO + i > n + 2 && LO + i < kRR * Ly.nr) cp[i * B] = inv_rate<!FIX>(R[i], il0_s + LO + i) * inv_d;
+                                if (LO + i > n + 2 && LO + i < kRR * Ly.nr) cp[i * B] = inv_rate<LOGS>(R[i], il0_s + LO + i) * inv_d;
                         }
                     }
                     if (!FIX && (nmat & 1)) {
@@ -509,13 +530,13 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     }
 #pragma unroll
                     for (int i = 0; i < kFR; ++i) {
-                        const float il = FIX ? R[i] : il0_s[LO + i] * ex2_ulp(-R[i]);
-                        if (!FIX || MODE == Mode::Fused)
+                        const float il = LOGS ? il0_s[LO + i] * ex2_ulp(-R[i]) : R[i];
+                        if (CK || MODE == Mode::Fused)
                             sc[(Ly.s_x + LO + i) * B] = il * inv_d;
                         else if (own)
                             tp[(LO + i) * total] = il;
                         if (LO + i < nmat)
-                            disc = FIX ? f2_mul(disc, bond_ratio(il, delta)) : f2_mul(disc, bond_ratio2(il, delta));
+                            disc = LOGS ? f2_mul(disc, bond_ratio2(il, delta)) : f2_mul(disc, bond_ratio(il, delta));
                         else if (LO + i < nn)
                             ILst[(LO + i - nmat) * B] = il;
                     }
@@ -523,16 +544,18 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 // ---- payoff (portfolio_b :133-171, :186-197) and the annuity adjoint ----
                 unsigned long long mask;
                 float dsc;
-                V = payoff_forward_staged<B, !FIX>(M, disc, delta, ost_s, okk_s, owf_s, &dsc, Bst, ILst, &mask);
+                V = payoff_forward_staged<B, LOGS>(M, disc, delta, ost_s, okk_s, owf_s, &dsc, Bst, ILst, &mask);
                 if (mode != Mode::Forward) {
                     payoff_adjoint_stage<B>(M, vb, dsc, Bst, ILst, mask, delta, ost_s, okf_s, owf_s);
+                    if (ilsm) {
 #pragma unroll 4
-                    for (int i = 0; i < M; ++i) sc[(Ly.s_d + nmat + i) * B] = ILst[i * B];
+                        for (int i = 0; i < M; ++i) sc[(Ly.s_d + nmat + i) * B] = ILst[i * B];
+                    }
                 }
             }
             if (mode != Mode::Forward) {
 #pragma unroll 8
-                for (int k = 0; k < kRR * Ly.nr; ++k) vg0[k * B] = 0.0f;
+                for (int k = 0; k < kRR * Ly.nr; ++k) (WIN ? sc + (size_t)Ly.s_g * B : vg0)[k * B] = 0.0f;
 
                 // ---- reverse: the blocks from the top, each over the steps with an active cell in it ----
                 float *su = sc + (size_t)Ly.s_s * B;
@@ -562,10 +585,28 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     auto back = [&](int t, const float *&rs, int &tl) {   // the rates to take back at time t
                         rs = sc;
                         tl = kRR;
-                        if (!FIX && nck > 0 && t % ck == 0 && t >= ck) {
+                        if (CK && nck > 0 && t % ck == 0 && t >= ck) {
                             rs = sc + (size_t)(Ly.s_ck + (t / ck - 1) * kRR * Ly.nr + LO) * B;
                             tl = t - LO;
                         }
+                    };
+                    // the vega rows that steps n .. nlo touch, k = kb .. LO - nlo + kRR - 2
+                    float *sg = sc + (size_t)Ly.s_g * B;
+                    int nlo = nmat, kb = 0;
+                    auto keep = [&]() {
+#pragma unroll 8
+                        for (int k = max(kb, 0); k < LO - nlo + kRR - 1; ++k) sg[k * B] = vg0[(k - kb) * B];
+                    };
+                    auto rows_of = [&](int n) {           // the rows of step n
+                        if (!WIN) return vg0 + (LO - n - 1) * B;
+                        if (n < nlo) {
+                            if (nlo < nmat) keep();
+                            nlo = max((n - Ly.seg + kRG) / kRG * kRG, 0);
+                            kb = LO - n - 1;
+#pragma unroll 16
+                            for (int k = max(kb, 0); k < LO - nlo + kRR - 1; ++k) vg0[(k - kb) * B] = sg[k * B];
+                        }
+                        return vg0 + (LO - n - 1 - kb) * B;
                     };
                     const float *rs;
                     int tl, n = nmat - 1;
@@ -575,7 +616,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             if (LO + kRR - 1 <= n) continue;
                             TpbStep s1[1] = {{drift(n) * vsc, top ? 0.0f : su[n * B]}};
                             back(n, rs, tl);
-                            rev_block<B, 1, true>(X, Pb, s1, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
+                            rev_block<B, 1, true>(X, Pb, s1, kr - (n + 1) + LO, rows_of(n), n, LO, rs, tl);
                             su[n * B] = s1[0].S;
                         }
                     }
@@ -601,7 +642,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             }
                         }
                         back(n - kRG + 1, rs, tl);
-                        rev_block<B, kRG, !FIX>(X, Pb, st, kr - (n + 1) + LO, vg0 + (LO - n - 1) * B, n, LO, rs, tl);
+                        rev_block<B, kRG, CK>(X, Pb, st, kr - (n + 1) + LO, rows_of(n), n, LO, rs, tl);
                         if (b > 0) {
 #pragma unroll
                             for (int g = 0; g < kRG; ++g) {
@@ -610,6 +651,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                             }
                         }
                     }
+                    if (WIN && nlo < nmat) keep();
 #pragma unroll
                     for (int i = 0; i < kRR; ++i) sc[(Ly.s_d + LO + i) * B] = Pb[i] * il0_s[LO + i];
                 }
@@ -627,19 +669,36 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             }
             if (mode != Mode::Forward) {
                 const int off = mode == Mode::Fused ? 1 : 0;
-                float *vgw = vg_s + kRG * B;
-                if (!active) {
+                float *vgw = vg0 - tid;
+                if (WIN) {
+                    const int R = tpb_win(Ly.seg);        // rows at a time
 #pragma unroll 1
-                    for (int k = 0; k < nn; ++k) vg0[k * B] = 0.0f;
-                }
-                __syncwarp();
-                column_sums<B>(nn, vgw, warp, lane, acc, nout, off + nn);
-                __syncwarp();
+                    for (int q = 0; q < 2; ++q) {         // vegas, deltas
+                        const float *sr = sc + (size_t)(q ? Ly.s_d : Ly.s_g) * B;
+#pragma unroll 1
+                        for (int k0 = 0; k0 < nn; k0 += R) {
+                            const int c = min(R, nn - k0);
 #pragma unroll 16
-                for (int i = 0; i < nn; ++i) vg0[i * B] = active ? sc[(Ly.s_d + i) * B] : 0.0f;
-                __syncwarp();
-                column_sums<B>(nn, vgw, warp, lane, acc, nout, off);
-                __syncwarp();
+                            for (int i = 0; i < c; ++i) vg0[i * B] = active ? sr[(k0 + i) * B] : 0.0f;
+                            __syncwarp();
+                            column_sums<B>(c, vgw, warp, lane, acc, nout, off + (q ? 0 : nn) + k0);
+                            __syncwarp();
+                        }
+                    }
+                } else {
+                    if (!active) {
+#pragma unroll 1
+                        for (int k = 0; k < nn; ++k) vg0[k * B] = 0.0f;
+                    }
+                    __syncwarp();
+                    column_sums<B>(nn, vgw, warp, lane, acc, nout, off + nn);
+                    __syncwarp();
+#pragma unroll 16
+                    for (int i = 0; i < nn; ++i) vg0[i * B] = active ? sc[(Ly.s_d + i) * B] : 0.0f;
+                    __syncwarp();
+                    column_sums<B>(nn, vgw, warp, lane, acc, nout, off);
+                    __syncwarp();
+                }
             }
         }
 
@@ -656,27 +715,27 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     }  // units
 }
 
-template <int NN, int NMAT, int B, Mode MODE = Mode::Fused>
+template <int NN, int NMAT, int B, bool WIN, Mode MODE = Mode::Fused>
 cudaError_t launch_tpb(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox, const Work &w,
                        float *scr, float *tape, const double *vbar, cudaStream_t s)
 {
-    const int bytes = tpb_layout(m.nn, m.nmat, mode, B).bytes;
-    auto kern = k_tpb<NN, NMAT, B, false, MODE>;
+    const int bytes = tpb_layout(m.nn, m.nmat, mode, B, WIN).bytes;
+    auto kern = k_tpb<NN, NMAT, B, WIN, false, MODE>;
     if constexpr (MODE == Mode::Fused)
-        if (philox) kern = k_tpb<NN, NMAT, B, true, MODE>;
+        if (philox) kern = k_tpb<NN, NMAT, B, WIN, true, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)w.grid, B, bytes, s>>>(m, z, seed, path0, w, scr, tape, vbar, (int)mode);
     return cudaGetLastError();
 }
 
-template <int NN, int NMAT, int B, Mode MODE = Mode::Fused>
+template <int NN, int NMAT, int B, bool WIN, Mode MODE = Mode::Fused>
 cudaError_t occ_tpb(int nn, int nmat, Mode mode, bool philox, int *blocks)
 {
-    const int bytes = tpb_layout(nn, nmat, mode, B).bytes;
-    auto kern = k_tpb<NN, NMAT, B, false, MODE>;
+    const int bytes = tpb_layout(nn, nmat, mode, B, WIN).bytes;
+    auto kern = k_tpb<NN, NMAT, B, WIN, false, MODE>;
     if constexpr (MODE == Mode::Fused)
-        if (philox) kern = k_tpb<NN, NMAT, B, true, MODE>;
+        if (philox) kern = k_tpb<NN, NMAT, B, WIN, true, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, B, bytes);

@@ -1,0 +1,17 @@
+// The rate-block kernel (lmm_f32_tpb.cuh) for shapes at run time, vega rows in a window.
+#include "lmm_f32_tpb.cuh"
+
+namespace lmm {
+
+cudaError_t launch_tpb_window(const DevModel &m, Mode mode, const float *z, uint64_t seed, int64_t path0, bool philox,
+                             const Work &w, float *scr, const double *vbar, cudaStream_t s)
+{
+    return launch_tpb<0, 0, 512, true>(m, mode, z, seed, path0, philox, w, scr, nullptr, vbar, s);
+}
+
+cudaError_t occ_tpb_window(int nn, int nmat, Mode mode, bool philox, int *blocks)
+{
+    return occ_tpb<0, 0, 512, true>(nn, nmat, mode, philox, blocks);
+}
+
+}  // namespace lmm

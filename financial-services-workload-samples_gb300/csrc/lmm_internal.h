@@ -70,6 +70,7 @@ cudaError_t launch_tpp_any(const DevModel &m, const float *z, const Work &w, cud
 // mode of 80/40 (the pair on a tape) and of other shapes whose checkpoint interval
 // is a multiple of 4. A per-block scratch of tpb_scratch_floats_per_block floats.
 bool f32_tpb_supports(int nn, int nmat, int ckpt);
+bool tpb_windowed(int nn, int nmat);
 int tpb_block_threads(int nn, int nmat);
 int tpb_cells(int nn, int nmat);
 int tpb_tape_rows(int nn, int nmat);
