@@ -28,6 +28,7 @@ k_finalize(const double *__restrict__ partial, int items, int nout, int64_t path
     const int scen = blockIdx.x / nchunk, o0 = (blockIdx.x % nchunk) * X;
     const int x = threadIdx.x % X, y = threadIdx.x / X, o = o0 + x;
     double a[kFinU] = {}, b[kFinU] = {};
+    wait_for_predecessor();
     if (o < nout) {
         const double *p0 = partial + (size_t)scen * items * 2 * nout + o;
         int it = y;
@@ -89,8 +90,7 @@ cudaError_t finalize(const double *partial, int nscen, int items, int nout, int6
 {
     const int64_t blocks = (int64_t)nscen * ((nout + X - 1) / X);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    k_finalize<X><<<(unsigned)blocks, kFinThreads, 0, s>>>(partial, items, nout, paths, mean, se, flag, stamp);
-    return cudaGetLastError();
+    return launch_early(k_finalize<X>, (unsigned)blocks, kFinThreads, 0, s, partial, items, nout, paths, mean, se, flag, stamp);
 }
 
 __global__ void k_bump_diff(double *mean, double *se, int nscen, int nout, double h)

@@ -204,6 +204,28 @@ __device__ __forceinline__ void two_sum_acc(float &s, float &c, float x)
     s = t;
 }
 
+// Launches a kernel that starts with wait_for_predecessor(): its blocks are placed
+// while the stream's kernel before it drains, and wait for the end of that one and
+// its writes. GB300, calls of 3,001 paths of 80/40 one after the other: 60.0 us ->
+// 57.4 with the sums' kernel launched so, 55.3 with the paths' kernel too.
+template <class... P, class... A>
+cudaError_t launch_early(void (*kern)(P...), unsigned grid, int block, int smem, cudaStream_t s, const A &...a)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = s;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, a...);
+}
+
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Two FP32 values in a register pair: one instruction for both, each rounded as
 // the scalar operation (PTX ISA: add/sub/fma.rn.f32x2).
 using P2 = unsigned long long;

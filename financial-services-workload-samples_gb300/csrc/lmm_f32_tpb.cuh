@@ -381,6 +381,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     double *acc_s = WIN ? reinterpret_cast<double *>(sb + (size_t)Ly.s_a * B) : reinterpret_cast<double *>(smem + Ly.acc);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    wait_for_predecessor();
     for (int i = tid; i < nmat + kFR * Ly.nf; i += B) {
         const int k = i - nmat;
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f), r = f;
@@ -725,8 +726,7 @@ cudaError_t launch_tpb(const DevModel &m, Mode mode, const float *z, uint64_t se
         if (philox) kern = k_tpb<NN, NMAT, B, WIN, true, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)w.grid, B, bytes, s>>>(m, z, seed, path0, w, scr, tape, vbar, (int)mode);
-    return cudaGetLastError();
+    return launch_early(kern, (unsigned)w.grid, B, bytes, s, m, z, seed, path0, w, scr, tape, vbar, (int)mode);
 }
 
 template <int NN, int NMAT, int B, bool WIN, Mode MODE = Mode::Fused>

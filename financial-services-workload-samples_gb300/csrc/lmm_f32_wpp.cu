@@ -279,6 +279,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     double *acc = reinterpret_cast<double *>(wbase + Ly.acc);
 
     const int head = wpp_head(nmat);
+    wait_for_predecessor();
     for (int i = tid; i < nn + head; i += kWppBlock)
         kc_s[i] = i < head ? make_float4(0.f, 0.f, 0.f, 0.f) : m.kc[i - head];
     for (int i = tid; i <= M; i += kWppBlock) ost_s[i] = m.opt_start[i];
@@ -468,8 +469,7 @@ cudaError_t wpp_launch_s(const DevModel &m, const float *z, uint64_t seed, int64
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)(w.grid > 0 ? w.grid : (int64_t)m.nscen * w.items);
-    kern<<<grid, kWppBlock, bytes, st>>>(m, z, seed, path0, w, vbar, ytop);
-    return cudaGetLastError();
+    return launch_early(kern, grid, kWppBlock, bytes, st, m, z, seed, path0, w, vbar, ytop);
 }
 
 template <int S, bool PHILOX, Mode MODE>
