@@ -261,23 +261,22 @@ int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
 // thread-per-path kernel takes one path's latency for anything from one path to
 // a device full of single warps; a warp per path takes a short time for one path
 // and its throughput beyond the device's resident warps (3,648 on GB300; 3,040
-// above 160 rates). 160/120, whole calls at 3,600 / 4,800 / 5,600 paths: fused
-// 0.191 / 0.258 / 0.295 against 0.53 ms, the pair 0.274 / 0.373 / 0.426 against
-// 0.393; the pair, which has to go with the fused call, puts the line at 1.33
-// fills. Shapes in rate blocks: the ratio of the two estimates in us, fitted to
-// whole calls of 13 shapes, of which a warp per path / rate blocks took, at
-// 5,400-5,600 paths, 0.133 / 0.236 ms (96/60; line at 2.9 fills), 0.109 / 0.160
-// (64/50; 2.4), 0.086 / 0.113 (60/30; 2.2), 0.098 / 0.100 and for the pair 0.158 /
-// 0.132 (80/40; 1.3), 0.055 / 0.057 (40/10; 1.4), and with a window of vega rows, at
-// 11,000, 0.454 / 0.592 (128/100; 4). Above 160 rates a lane's eight rates collide on
-// the banks: two fills (5,600 paths, 161/100 0.94 / 0.76, 256/40 0.82 / 0.64; 3,600,
-// 256/119 1.04 / 1.37).
+// above 160 rates). 160/120, whole calls at 3,600 / 4,800 paths: fused 0.183 / 0.246
+// against 0.52 ms, the pair 0.257 / 0.350 against 0.365; the pair, which has to go
+// with the fused call, puts the line at 1.33 fills. Shapes in rate blocks: the ratio
+// of the two estimates in us, fitted to whole calls of 13 shapes; a warp per path /
+// rate blocks took, at 5,400-5,600 paths, 0.121 / 0.236 ms (96/60; line at 2.9
+// fills), 0.103 / 0.150 (64/50; 2.4), 0.074 / 0.113 (60/30; 2.2), 0.081 / 0.096 and
+// for the pair 0.125 / 0.125 (80/40; 1.6), 0.050 / 0.053 (40/10; 1.4), and with a
+// window of vega rows, at 11,000, 0.456 / 0.592 (128/100; 4). Above 160 rates a
+// lane's eight rates collide on the banks: two fills (5,600 paths, 161/100 0.93 /
+// 0.76, 256/40 0.80 / 0.64; 3,600, 256/119 1.00 / 1.37).
 double wpp_fills(int nn, int nmat, bool rate_blocks)
 {
     if (!rate_blocks) return 4.0 / 3.0;
     const int slots = lmm::wpp_slots(nn);
     if (slots > 5) return 2.0;
-    const double cell = nn == 80 && nmat == 40 ? 0.0088 : lmm::tpb_windowed(nn, nmat) ? 0.025 : 0.0175;
+    const double cell = nn == 80 && nmat == 40 ? 0.011 : lmm::tpb_windowed(nn, nmat) ? 0.025 : 0.0175;
     return std::min(4.0, std::max(1.0, (25.0 + cell * lmm::tpb_cells(nn, nmat)) / (20.0 + nmat * (0.5 + 0.15 * slots))));
 }
 

@@ -23,8 +23,9 @@
 //   dV/dlambda_k += Pb_i (Y_i - delta lambda_k) + t S'_i.
 // The payoff (portfolio_b :120-211, aliasing fixed) runs with double-FP32
 // products and sums (F2, lmm_device.cuh): the discount product is a warp
-// product reduction, the annuity recursion runs on lane 0, on factors that the
-// lanes have formed side by side.
+// reduction, the annuity factors and sums and their adjoints are warp scans over
+// the maturities (on one lane they took a third of the instructions: 3,001 paths of
+// 80/40 55.3 -> 49.2 us a call).
 // The forward holds log2(L/L0), which stays below 1 or so, where a product a step
 // would collect a rounding of L each, and the payoff's factors 1/(1 + delta L)
 // keep their rounding: fewer swaptions at the money pay or not unlike the exact
@@ -125,6 +126,19 @@ __device__ __forceinline__ float warp_excl_suffix(float x, int lane)
     }
     const float ex = __shfl_down_sync(0xffffffffu, inc, 1);
     return lane == 31 ? 0.0f : ex;
+}
+
+// The same of double-FP32 values under an associative operation.
+template <class Op>
+__device__ __forceinline__ F2 warp_excl_prefix(F2 x, F2 one, int lane, Op op)
+{
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const F2 y{__shfl_up_sync(0xffffffffu, x.hi, d), __shfl_up_sync(0xffffffffu, x.lo, d)};
+        if (lane >= d) x = op(y, x);
+    }
+    const F2 ex{__shfl_up_sync(0xffffffffu, x.hi, 1), __shfl_up_sync(0xffffffffu, x.lo, 1)};
+    return lane == 0 ? one : ex;
 }
 
 // Constants and vega row of slot s at step n. The tables hold k at row
@@ -355,46 +369,63 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 const F2 other{__shfl_xor_sync(0xffffffffu, dprod.hi, o), __shfl_xor_sync(0xffffffffu, dprod.lo, o)};
                 dprod = f2_mul(dprod, other);
             }
-            const float disc = dprod.hi;
+            dprod = {__shfl_sync(0xffffffffu, dprod.hi, 0), __shfl_sync(0xffffffffu, dprod.lo, 0)};
             __syncwarp();
-            float V = 0.0f;
-            if (lane == 0) {
-                F2 bb{1.0f, 0.0f}, sb{0.0f, 0.0f}, vs{0.0f, 0.0f};
-                unsigned long long mask = 0ull;
-                for (int mm = 0; mm < M; ++mm) {
-                    bb = f2_mul(bb, F2{rt_s[mm], bw_s[mm]});
-                    sb = f2_add(sb, bb);                      // annuity / delta
-                    bw_s[mm] = bb.hi;
-                    for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
-                        const float sw = f2_swap_value(okk_s[o], sb, bb);
-                        if (sw < 0.0f) {
-                            vs = f2_add(vs, (-100.0f * sw) * owf_s[o]);
-                            mask |= 1ull << o;
-                        }
+            // Lane l takes the maturities m0 .. m1-1: annuity factors B[m] from the product of the lanes
+            // below, the annuity sum from their sums.
+            const int per = (M + 31) >> 5, m0 = min(per * lane, M), m1 = min(m0 + per, M);
+            F2 bb{1.0f, 0.0f}, sb{0.0f, 0.0f}, vs{0.0f, 0.0f};
+            for (int mm = m0; mm < m1; ++mm) bb = f2_mul(bb, F2{rt_s[mm], bw_s[mm]});
+            bb = warp_excl_prefix(bb, F2{1.0f, 0.0f}, lane, [](F2 x, F2 y) { return f2_mul(x, y); });
+            F2 b1 = bb;
+            for (int mm = m0; mm < m1; ++mm) {
+                b1 = f2_mul(b1, F2{rt_s[mm], bw_s[mm]});
+                sb = f2_add(sb, b1);
+            }
+            sb = warp_excl_prefix(sb, F2{0.0f, 0.0f}, lane, [](F2 x, F2 y) { return f2_add(x, y); });
+            unsigned long long mask = 0ull;
+            float Sb = 0.0f;
+            for (int mm = m0; mm < m1; ++mm) {
+                bb = f2_mul(bb, F2{rt_s[mm], bw_s[mm]});
+                sb = f2_add(sb, bb);                          // annuity / delta
+                bw_s[mm] = bb.hi;
+                for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
+                    const float sw = f2_swap_value(okk_s[o], sb, bb);
+                    if (sw < 0.0f) {
+                        vs = f2_add(vs, (-100.0f * sw) * owf_s[o]);
+                        Sb -= (100.0f * okf_s[o]) * owf_s[o];
+                        mask |= 1ull << o;
                     }
                 }
-                const F2 v = f2_mul(vs, dprod);
-                V = __fadd_rn(v.hi, v.lo);
-                if (MODE == Mode::Forward) mask = 0ull;     // no adjoint
-                // :173-184 with the rate kept apart from its adjoint; lw_s[i] becomes
-                // the log-adjoint of rate i >= nmat. B[m] comes from the forward
-                // (bw_s): rebuilding it backwards from the last, smallest factor
-                // would underflow FP32 on paths whose rates grow large.
-                const float scale = -vb * disc * delta;
-                float Sb = 0.0f, Bb = 0.0f;
-                for (int mm = M - 1; mm >= 0; --mm) {
-                    const float Ln = lw_s[nmat + mm];
-                    const float r = rt_s[mm];
-                    const float Bm = bw_s[mm];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                vs = f2_add(vs, F2{__shfl_xor_sync(0xffffffffu, vs.hi, o), __shfl_xor_sync(0xffffffffu, vs.lo, o)});
+            const F2 v = f2_mul(vs, dprod);
+            float V = __fadd_rn(v.hi, v.lo);
+            if (MODE != Mode::Forward) {
+                // :173-184 with the rate kept apart from its adjoint: what reaches rate nmat+m is the sum
+                // over j >= m of (Bb[j] + delta Sb[j]) B[j], where Bb[j] are the payoffs on B[j] and Sb[j]
+                // those on the annuities from j on; lw_s[i] becomes the log-adjoint of rate i >= nmat.
+                Sb = warp_excl_suffix(Sb, lane);
+                float W = 0.0f;
+                for (int mm = m1 - 1; mm >= m0; --mm) {
+                    float Bb = 0.0f;
                     for (int o = ost_s[mm]; o < ost_s[mm + 1]; ++o) {
                         if ((mask >> o) & 1ull) {
                             Sb -= (100.0f * okf_s[o]) * owf_s[o];
                             Bb -= 100.0f * owf_s[o];
                         }
                     }
-                    Bb = fmaf(delta, Sb, Bb);
-                    lw_s[nmat + mm] = scale * Bb * Bm * (Ln * r);
-                    Bb *= r;
+                    const float x = fmaf(delta, Sb, Bb) * bw_s[mm];
+                    bw_s[mm] = x;
+                    W += x;
+                }
+                W = warp_excl_suffix(W, lane);
+                const float scale = -vb * dprod.hi * delta;
+                for (int mm = m1 - 1; mm >= m0; --mm) {
+                    W += bw_s[mm];
+                    lw_s[nmat + mm] = scale * W * (lw_s[nmat + mm] * rt_s[mm]);
                 }
             }
             V = __shfl_sync(0xffffffffu, V, 0);
