@@ -150,10 +150,10 @@ cudaError_t launch_dfma_peak(int blocks, int iters, double a, double b, float *s
 // kind 0: ex2.approx, 1: rcp.approx, 2: both alternately; 16 per thread per iteration
 cudaError_t launch_mufu_peak(int kind, int blocks, int iters, float *sink, cudaStream_t s);
 
-// MRG32k3a jump tables (lmm_mrg.cu): A1^(2^k), A2^(2^k) for k < 64 and the
-// per-lane offsets A1^(l*span), A2^(l*span) for l < 32, entries mod m1/m2.
+// MRG32k3a jump tables (lmm_mrg.cu): A1^(2^k), A2^(2^k) for k < 64, entries mod
+// m1/m2.
 struct MrgTables {
-    uint32_t p1[64][9], p2[64][9], l1[32][9], l2[32][9];
+    uint32_t p1[64][9], p2[64][9];
 };
 // kind 0: uniforms (double), 1: normals (double, PPND16), 2: normals (float, PPND7)
 cudaError_t launch_mrg32k3a(int kind, uint32_t seed, int64_t first, int64_t count, double mean, double sd,

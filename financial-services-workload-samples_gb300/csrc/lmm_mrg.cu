@@ -13,12 +13,11 @@
 //   path has no FP64 operation).
 // Seeding from one 32-bit seed s: x state (s mod m1, 1, 1), y state (1,1,1).
 //
-// Work layout. Each warp owns a chunk of 32*kSpan consecutive stream
-// elements; lane l generates elements [l*kSpan, (l+1)*kSpan) of the chunk
-// with the plain recurrence after two jumps: the warp's chunk start
-// (A^(2^k) table, the same entries for every lane) and the lane's offset
-// (A^(l*kSpan) table). Generated values go through a 32x33 shared-memory tile
-// per warp so that each store instruction writes 32 consecutive elements.
+// Work layout. Each warp owns a chunk of 32*span consecutive stream elements;
+// lane l generates elements [l*span, (l+1)*span) of the chunk with the plain
+// recurrence after a jump to its start, by the powers A^(2^k). Generated values
+// go through a shared-memory tile per warp so that each store instruction writes
+// 16 or 32 consecutive elements.
 //
 // Arithmetic order: the central branch of the inversion and mean + sd*x use
 // explicitly rounded multiplies and adds (no contraction), as the C
@@ -34,7 +33,7 @@ namespace {
 
 constexpr uint64_t kM1 = 4294967087ULL;
 constexpr uint64_t kM2 = 4294944443ULL;
-constexpr int kSpan = 512;        // elements per lane per chunk (multiple of 32)
+constexpr int kSpan = 512;        // most elements per lane
 constexpr int64_t kHalfM1p1 = 2147483544;            // (m1 + 1) / 2
 constexpr float kNormF = (float)(1.0 / 4294967088.0); // 1 / (m1 + 1), rounded to FP32
 constexpr int kWarps = 4;         // warps per block
@@ -42,21 +41,6 @@ constexpr int kWarps = 4;         // warps per block
 // 32 columns and 5 blocks (shared memory) 8.97 ms, 16 columns and 6 / 7 / 8 / 10
 // blocks 8.81 / 8.71 / 8.63 / 8.63 ms.
 constexpr int kCols64 = 16, kBlocks64 = 8;
-
-__device__ __forceinline__ void jump(const uint32_t *m, uint64_t v[3], uint64_t mod)
-{
-    uint64_t r[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        uint64_t s = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) s = (s + ((uint64_t)m[3 * i + k] * v[k]) % mod) % mod;
-        r[i] = s;
-    }
-    v[0] = r[0];
-    v[1] = r[1];
-    v[2] = r[2];
-}
 
 // v mod m1 and v mod m2 for v < 2^54: 2^32 is 209 mod m1 and 22853 mod m2, so
 // the high word folds into the low one.
@@ -73,6 +57,28 @@ __device__ __forceinline__ uint32_t mod_m2(uint64_t v)
     const uint64_t x = (uint64_t)(uint32_t)(w >> 32) * 22853u + (uint32_t)w;  // < 2^32 + 2^20
     const uint32_t r = (uint32_t)x + 22853u * (uint32_t)(x >> 32);
     return r >= (uint32_t)kM2 ? r - (uint32_t)kM2 : r;
+}
+
+// A smaller value with the remainder of v mod 2^32 - c.
+__device__ __forceinline__ uint64_t fold(uint64_t v, uint32_t c) { return (v >> 32) * c + (uint32_t)v; }
+
+// v := M v mod 2^32 - c, entries of M and v below 2^32. A product folds to below
+// 2^47.5 (c < 2^14.5), the sum of three to below 2^33, then to below 2^32 + 2^16.
+__device__ __forceinline__ void jump(const uint32_t *m, uint32_t v[3], uint32_t c)
+{
+    uint32_t r[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        uint64_t s = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s += fold((uint64_t)m[3 * i + k] * v[k], c);
+        s = fold(fold(s, c), c);
+        const uint64_t mod = (1ULL << 32) - c;
+        r[i] = (uint32_t)(s >= mod ? s - mod : s);
+    }
+    v[0] = r[0];
+    v[1] = r[1];
+    v[2] = r[2];
 }
 
 // One step of both recurrences; returns z in [1, m1].
@@ -160,7 +166,7 @@ __device__ float ppnd7(float q, float pt)
 // ms; FP32 normals, by the recurrences' folded remainders, 1.11 -> 0.85 ms.
 template <int KIND>  // 0: uniforms (double), 1: normals (double), 2: normals (float)
 __global__ void __launch_bounds__(32 * kWarps, KIND == 1 ? kBlocks64 : 1)
-k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, double mean, double sd, void *out)
+k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, int span, double mean, double sd, void *out)
 {
     using T = typename std::conditional<KIND == 2, float, double>::type;
     constexpr int C = KIND == 1 ? kCols64 : 32;       // columns: elements per lane between stores
@@ -168,31 +174,23 @@ k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, doubl
     __shared__ uint16_t queue[KIND == 1 ? kWarps : 1][KIND == 1 ? 32 * C : 1];   // the tile's tails, row * (C + 1) + column
     constexpr int kUnroll = KIND == 1 ? 1 : 4;         // GB300, FP64 normals: 2 elements a body 11.5 ms, 1 8.6 (instruction cache)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t chunk = ((int64_t)blockIdx.x * kWarps + w) * (32 * (int64_t)kSpan);
+    const int64_t chunk = ((int64_t)blockIdx.x * kWarps + w) * (32 * (int64_t)span);
     if (chunk >= count) return;  // warp-uniform
 
-    uint64_t x64[3] = {seed % kM1, 1, 1}, y64[3] = {1, 1, 1};
-    const uint64_t e0 = (uint64_t)(first + chunk);
-    for (int k = 0; k < 64; ++k) {
-        if ((e0 >> k) & 1ULL) {  // the same k for every lane: broadcast reads
-            jump(J.p1[k], x64, kM1);
-            jump(J.p2[k], y64, kM2);
+    uint32_t x[3] = {seed >= (uint32_t)kM1 ? seed - (uint32_t)kM1 : seed, 1, 1}, y[3] = {1, 1, 1};
+    const uint64_t e0 = (uint64_t)first + (uint64_t)(chunk + (int64_t)lane * span);
+    for (int k = 0; k < 64 && (e0 >> k) != 0; ++k) {
+        if ((e0 >> k) & 1ULL) {
+            jump(J.p1[k], x, 209u);
+            jump(J.p2[k], y, 22853u);
         }
-    }
-    jump(J.l1[lane], x64, kM1);
-    jump(J.l2[lane], y64, kM2);
-    uint32_t x[3], y[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        x[i] = (uint32_t)x64[i];
-        y[i] = (uint32_t)y64[i];
     }
 
     T *o = static_cast<T *>(out);
     const float fmean = (float)mean, fsd = (float)sd;
     auto scaled = [&](double v) { return __dadd_rn(mean, __dmul_rn(sd, v)); };
     const bool plain = mean == 0.0 && sd == 1.0;      // mean + sd v = v for every v but -0, which does not occur
-    for (int t = 0; t < kSpan / C; ++t) {
+    for (int t = 0; t < span / C; ++t) {
         int queued = 0;                               // warp-uniform
 #pragma unroll kUnroll
         for (int i = 0; i < C; ++i) {
@@ -226,7 +224,7 @@ k_mrg32k3a(const MrgTables J, uint32_t seed, int64_t first, int64_t count, doubl
         }
 #pragma unroll 4
         for (int r = lane / C; r < 32; r += 32 / C) {
-            const int64_t e = chunk + (int64_t)r * kSpan + t * C + lane % C;
+            const int64_t e = chunk + (int64_t)r * span + t * C + lane % C;
             if (e < count) o[e] = tile[w][r][lane % C];
         }
         __syncwarp();
@@ -250,17 +248,6 @@ Mat mat_mul(const Mat &x, const Mat &y, uint64_t m)
     return r;
 }
 
-Mat mat_pow(Mat a, uint64_t e, uint64_t m)
-{
-    Mat r{{1, 0, 0, 0, 1, 0, 0, 0, 1}};
-    while (e) {
-        if (e & 1) r = mat_mul(r, a, m);
-        a = mat_mul(a, a, m);
-        e >>= 1;
-    }
-    return r;
-}
-
 void store(uint32_t dst[9], const Mat &m)
 {
     for (int i = 0; i < 9; ++i) dst[i] = (uint32_t)m.a[i];
@@ -278,14 +265,6 @@ MrgTables make_tables()
         p1 = mat_mul(p1, p1, kM1);
         p2 = mat_mul(p2, p2, kM2);
     }
-    const Mat s1 = mat_pow(A1, kSpan, kM1), s2 = mat_pow(A2, kSpan, kM2);
-    Mat l1{{1, 0, 0, 0, 1, 0, 0, 0, 1}}, l2 = l1;
-    for (int l = 0; l < 32; ++l) {
-        store(t.l1[l], l1);
-        store(t.l2[l], l2);
-        l1 = mat_mul(l1, s1, kM1);
-        l2 = mat_mul(l2, s2, kM2);
-    }
     return t;
 }
 
@@ -301,15 +280,27 @@ cudaError_t launch_mrg32k3a(int kind, uint32_t seed, int64_t first, int64_t coun
                             void *out, cudaStream_t s)
 {
     if (count <= 0) return cudaSuccess;
-    const int64_t per_block = (int64_t)kWarps * 32 * kSpan;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    // Elements per lane, a power of two: a lane takes as long as its elements, and the jump to its start as
+    // long as about three FP64 normals. FP64 normals: 8 fills of the SMs' 32 warps, which even out the last one
+    // (GB300, 167,772,160: 1 / 2 / 4 / 8 / 16 fills 8.62 / 8.62 / 8.42 / 8.37 / 8.39 ms); the others, cheaper next
+    // to the jump, 2 (FP32, 0.853 / 0.853 / 0.868 / 0.932 / 1.09 ms; 83,886,080 0.478 / 0.449 / 0.474 / 0.547 /
+    // 0.692). With 512 throughout, 655,360 normals took 1.17 ms (FP64) and 0.18 (FP32), now 0.076 and 0.019.
+    const int fills = kind == 1 ? 8 : 2, least = kind == 1 ? kCols64 : 32;
+    int span = kSpan;
+    while (span > least && count < (int64_t)fills * sms * 32 * 32 * span) span /= 2;
+    const int64_t per_block = (int64_t)kWarps * 32 * span;
     const int64_t blocks = (count + per_block - 1) / per_block;
     if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
     const MrgTables &t = mrg_tables();
     const dim3 grid((unsigned)blocks), block(32 * kWarps);
     switch (kind) {
-        case 0: k_mrg32k3a<0><<<grid, block, 0, s>>>(t, seed, first, count, mean, sd, out); break;
-        case 1: k_mrg32k3a<1><<<grid, block, 0, s>>>(t, seed, first, count, mean, sd, out); break;
-        case 2: k_mrg32k3a<2><<<grid, block, 0, s>>>(t, seed, first, count, mean, sd, out); break;
+        case 0: k_mrg32k3a<0><<<grid, block, 0, s>>>(t, seed, first, count, span, mean, sd, out); break;
+        case 1: k_mrg32k3a<1><<<grid, block, 0, s>>>(t, seed, first, count, span, mean, sd, out); break;
+        case 2: k_mrg32k3a<2><<<grid, block, 0, s>>>(t, seed, first, count, span, mean, sd, out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
