@@ -232,7 +232,7 @@ cudaError_t launch_f32_family(int fam, const lmm::DevModel &m, Mode mode, const 
     if (fam == 5) return lmm::launch_tp2_any(m, mode, z, seed, path0, philox, w, mode == Mode::Fused ? scr : tape, vbar, s);
     if (fam == 6) return lmm::launch_tpb_any(m, mode, z, seed, path0, philox, w, scr, tape, vbar, s);
     if (fam == 7) return lmm::launch_tpq_any(m, z, seed, path0, philox, w, scr, s);
-    return lmm::launch_wpp_any(m, mode, z, seed, path0, philox, w, scr, vbar, s);
+    return lmm::launch_wpp_any(m, mode, z, seed, path0, philox, w, mode == Mode::Forward ? tape : scr, vbar, s);
 }
 
 int blocks_per_sm(lmm_engine *e, int family, Mode mode, bool philox, int *out)
@@ -497,6 +497,15 @@ int tp2_scratch(lmm_engine *e, int64_t blocks, float **out)
     return LMM_OK;
 }
 
+int family_scratch(lmm_engine *e, int fam, Mode mode, int64_t blocks, float **out)
+{
+    *out = nullptr;
+    if (fam == 2) return mode != Mode::Forward ? wpp_scratch(e, blocks, out) : LMM_OK;
+    if (fam == 5) return mode == Mode::Fused ? tp2_scratch(e, blocks, out) : LMM_OK;
+    if (fam == 6) return tpb_scratch(e, blocks, out);
+    return tpq_scratch(e, blocks, out);
+}
+
 int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t path0, bool philox,
             int64_t paths, float *tape, const double *d_vbar, double *d_mean, double *d_se)
 {
@@ -512,16 +521,24 @@ int run_f32(lmm_engine *e, Mode mode, const float *d_z, uint64_t seed, int64_t p
                                              ", nmat=" + std::to_string(e->nmat));
     if (philox && mode != Mode::Fused)
         return fail(LMM_ERR_UNSUPPORTED, "the forward/backward pair reads its normals from memory");
+    if (fam == 2 && mode == Mode::Backward && tape) d_z = tape;     // kept by the forward
     int bps = 0;
     LMM_TRY(blocks_per_sm(e, fam, mode, philox, &bps));
     const int nout = mode == Mode::Fused ? 1 + 2 * e->nn : (mode == Mode::Forward ? 1 : 2 * e->nn);
     Work w{};
     LMM_TRY(plan(e, fam, mode, e->nscen, paths, bps, nout, &w));
     float *scr = nullptr;
-    if (fam == 2) LMM_TRY(wpp_scratch(e, w.grid, &scr));
-    if (fam == 5 && mode == Mode::Fused) LMM_TRY(tp2_scratch(e, w.grid, &scr));
-    if (fam == 6) LMM_TRY(tpb_scratch(e, w.grid, &scr));
-    if (fam == 7) LMM_TRY(tpq_scratch(e, w.grid, &scr));
+    int rc = family_scratch(e, fam, mode, w.grid, &scr);
+    if (rc == LMM_ERR_OUT_OF_MEMORY && fam == 6 && lmm::f32_wpp_supports(e->nn, e->nmat) &&
+        (mode == Mode::Fused || !lmm::tpb_tape_rows(e->nn, e->nmat))) {
+        // rate blocks ask for up to 20 MB an SM, a warp per path for a tenth of it
+        cudaGetLastError();
+        fam = 2;
+        LMM_TRY(blocks_per_sm(e, fam, mode, philox, &bps));
+        LMM_TRY(plan(e, fam, mode, e->nscen, paths, bps, nout, &w));
+        rc = family_scratch(e, fam, mode, w.grid, &scr);
+    }
+    LMM_TRY(rc);
     LMM_TRY(next_stamp(e));
     mark(e, 0);
     cudaError_t err = launch_f32_family(fam, e->dm, mode, d_z, seed, path0, philox, w, scr, tape, d_vbar, e->stream);
@@ -1042,17 +1059,17 @@ int lmm_swaption_breakdown_f64_device(lmm_engine *e, const double *d_z, int64_t 
 // pieces on the engine's copy stream; the fused kernel of piece c starts as
 // soon as piece c has landed, while the later pieces are still in flight.
 // Relative piece sizes kHostSplit: the first piece's copy is the only one
-// nothing overlaps, so it is small (1/72: one wave of the split-reverse
-// kernel, 9 MB of 671 MB at 4M paths, 0.04 ms at the measured 211 GB/s), and
-// each later piece, about three times the one before, lands before the
-// compute of the pieces ahead of it ends (a wave computes in about 0.14 ms
-// and copies in 0.04 ms). Measured on GB300 at 4,194,304 paths: four equal
+// nothing overlaps, so it is small (1/72: one wave of the rate-block kernel, 12 MB
+// of 671 MB at 4M paths, 0.06 ms at the measured 211 GB/s), and each later piece,
+// about three times the one before, lands before the compute of the pieces ahead
+// of it ends (a wave computes in 0.19 ms). Measured on GB300 at 4,194,304 paths: four equal
 // pieces cost 0.6 ms per call more than {1,3,6,6}/16 (an earlier kernel);
 // piece boundaries on whole device waves: 363 -> 369 M paths/s;
 // {1,3,10,22}/36: 369 -> 373 M paths/s; with the 9.8 ms kernel,
 // {1,3,10,22}, {1,2,5,10,18}, {1,2,4,8,21}, {1,3,8,24}, {1,4,31}: 10.07,
 // 10.05, 10.06, 10.03, 11.70 ms per call, and {1,3,8,24}, {1,3,9,27,32},
-// {1,2,6,18,45}, {1,4,16,51}, {1,3,9,59}: 10.04, 10.02, 10.02, 10.23, 11.32.
+// {1,2,6,18,45}, {1,4,16,51}, {1,3,9,59}: 10.04, 10.02, 10.02, 10.23, 11.32; with
+// the 9.28 ms kernel, {1,3,8,24,36}: 9.39.
 // Each piece writes its own range of partial sums and one ordered k_finalize
 // covers them all. Single-scenario engines only.
 #ifndef LMM_HOST_SPLIT
@@ -1113,14 +1130,9 @@ int run_f32_host_pipelined(lmm_engine *e, const float *z, int64_t paths)
     }
     LMM_TRY(e->partial.ensure(sizeof(double) * (size_t)total_items * 2 * nout));
     float *wscr = nullptr;
-    if (fam == 2 || fam == 5 || fam == 6 || fam == 7) {
-        int64_t most = 0;
-        for (int c = 0; c < C; ++c) most = std::max(most, std::min<int64_t>(cplan[c].items, (int64_t)e->sms * bps));
-        // the pieces run one after another
-        LMM_TRY(fam == 2 ? wpp_scratch(e, most, &wscr)
-                         : fam == 5 ? tp2_scratch(e, most, &wscr)
-                                    : fam == 6 ? tpb_scratch(e, most, &wscr) : tpq_scratch(e, most, &wscr));
-    }
+    int64_t most = 0;          // the pieces run one after another
+    for (int c = 0; c < C; ++c) most = std::max(most, std::min<int64_t>(cplan[c].items, (int64_t)e->sms * bps));
+    LMM_TRY(family_scratch(e, fam, Mode::Fused, most, &wscr));
     LMM_TRY(next_stamp(e));
     for (int c = 0; c < C; ++c)
         if (!e->copy_ev[c]) LMM_CK(cudaEventCreateWithFlags(&e->copy_ev[c], cudaEventDisableTiming));
@@ -1162,9 +1174,17 @@ int lmm_greeks_f32_host(lmm_engine *e, const float *z, int64_t paths, double *ou
     const size_t zb = sizeof(float) * (size_t)paths * e->nmat;
     LMM_TRY(e->z32.ensure(zb));
     LMM_TRY(ensure_outputs(e, 1 + 2 * e->nn));
-    if (e->nscen == 1 && paths >= kPipelineMinPaths) {
-        LMM_TRY(run_f32_host_pipelined(e, z, paths));
-    } else {
+    bool pieces = e->nscen == 1 && paths >= kPipelineMinPaths;
+    if (pieces) {
+        const int rc = run_f32_host_pipelined(e, z, paths);
+        if (rc == LMM_ERR_OUT_OF_MEMORY) {       // in one piece, which may take a kernel of less scratch
+            cudaGetLastError();
+            pieces = false;
+        } else {
+            LMM_TRY(rc);
+        }
+    }
+    if (!pieces) {
         LMM_CK(cudaMemcpyAsync(e->z32.p, z, zb, cudaMemcpyHostToDevice, e->stream));
         LMM_TRY(run_f32(e, Mode::Fused, e->z32.as<float>(), 0, 0, false, paths, nullptr, nullptr,
                         e->out.as<double>(), e->se.as<double>()));
@@ -1204,12 +1224,16 @@ int lmm_tape_create(lmm_engine *e, int64_t paths, lmm_tape **out)
     t->paths = paths;
     // The rate-block (nn=80, nmat=40) and thread-pair (nn=160, nmat=120) pairs
     // keep the terminal rates and the per-step drift sums, the thread pair also
-    // those at the half boundary; the others' backward recomputes its forward
-    // from the same normals and needs no tape.
+    // those at the half boundary; for few paths of these shapes, whose backward
+    // runs its forward again, the normals are kept, so that here too the caller may
+    // overwrite them after the forward. The other shapes' backward reads the
+    // caller's normals and needs no tape.
     int fam = 0;
     LMM_TRY(family_at(e, Mode::Forward, paths, &fam));
-    const size_t rows = fam == 5 ? (size_t)e->nn + 2 * (size_t)e->nmat : fam == 6 ? (size_t)lmm::tpb_tape_rows(e->nn, e->nmat) : 0;
-    if (rows) LMM_TRY(t->buf.ensure(sizeof(float) * rows * e->nscen * (size_t)paths));
+    const bool taped = lmm::f32_tp2_supports(e->nn, e->nmat) || lmm::tpb_tape_rows(e->nn, e->nmat) > 0;
+    const size_t nn = e->nn, nmat = e->nmat;
+    const size_t row = !taped ? 0 : fam == 2 ? nmat : e->nscen * (nn + (fam == 5 ? 2 : 1) * nmat);     // floats a path
+    if (row) LMM_TRY(t->buf.ensure(sizeof(float) * row * (size_t)paths));
     *out = t.release();
     return LMM_OK;
 }

@@ -261,10 +261,10 @@ struct ZChunk {
 };
 
 // MODE: Fused (value + all Greeks), Forward (value only) or Backward (Greeks
-// of vbar[scen] x value; the forward is recomputed from the same normals, so
-// no tape is needed). ytop: gridDim.x * kWppWarps blocks of
-// wpp_scratch_floats(nmat, S, m.ckpt) floats of scratch, one per resident warp
-// (unused in Forward mode).
+// of vbar[scen] x value; the forward is recomputed from the same normals).
+// ytop: gridDim.x * kWppWarps blocks of wpp_scratch_floats(nmat, S, m.ckpt) floats
+// of scratch, one per resident warp. Forward: where the normals are kept for the
+// backward, [paths][nmat], or null.
 template <int S, bool PHILOX, Mode MODE>
 __global__ void __launch_bounds__(kWppBlock, wpp_min_blocks(S))
 k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path0, const Work w,
@@ -346,6 +346,8 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     for (int s = 0; s < S; ++s) ck[((n / ckn) * S + s) * 32] = L[s];
                 }
                 const float sqez = sqd * zc.get(n, zp, nmat, seed, gpath, lane);
+                if (MODE == Mode::Forward && !PHILOX && ytop && scen == 0 && (n & 31) == 0 && n + lane < nmat)
+                    ytop[p * nmat + n + lane] = zc.v[0];
                 const float y = wpp_fwd_step<S>(L, D, L0, base, n, sqez, lane, kc_s, delta);
                 if (MODE != Mode::Forward) yt[n * 32] = y;
             }

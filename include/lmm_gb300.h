@@ -100,8 +100,8 @@ int lmm_engine_destroy(lmm_engine *e);
 /* Use `stream` (a cudaStream_t, NULL = legacy default stream) from now on.
  * CUDA graphs: once a device call (lmm_greeks_f32_device, lmm_greeks_philox_device,
  * lmm_greeks_f64_device, the mrg32k3a/normals generators) has run for a
- * given engine and path count, repeating it enqueues only kernels and async
- * memsets on the stream and allocates nothing, so it can be recorded by a
+ * given engine and path count, repeating it enqueues only kernels on the
+ * stream and allocates nothing, so it can be recorded by a
  * stream capture and replayed. */
 int lmm_engine_set_stream(lmm_engine *e, void *stream);
 /* Checkpoint interval of the FP32 reverse sweep (fused calls). Storing the
@@ -170,9 +170,10 @@ int lmm_greeks_philox_device(lmm_engine *e, uint64_t seed, int64_t path0, int64_
  * inverse terminal rates 1/L and the per-step drift sums the reverse sweep
  * restarts from: (nn + nmat) floats. For nn = 160, nmat = 120 (two threads
  * per path) it also holds the per-step drift sums at rate nn/2 - 1:
- * (nn + 2 nmat) floats. For the other shapes (warp-per-path kernels) the
- * backward recomputes the forward from the same normals d_z, and the tape
- * holds no device memory. */
+ * (nn + 2 nmat) floats. For few paths of these two shapes the tape holds the
+ * normals instead (nmat floats) and the backward recomputes the forward from
+ * them. For the other shapes the backward recomputes the forward from the
+ * same normals d_z, and the tape holds no device memory. */
 int lmm_tape_create(lmm_engine *e, int64_t paths, lmm_tape **out);
 int lmm_tape_destroy(lmm_tape *t);
 /* Forward: value per scenario (d_value[nscen], d_value_se[nscen] or NULL). */
@@ -272,7 +273,7 @@ int lmm_mrg32k3a_normals_f32_device(uint32_t seed, int64_t first, int64_t count,
  * FP32 value + Greeks launch like lmm_greeks_f32_device, without an engine
  * and without any allocation (no cudaMalloc, no cudaFree, no allocating
  * library call). It runs the one-pass kernel, which needs no per-path
- * scratch; the engine's fused call runs the split-reverse kernel, and the
+ * scratch; the engine's fused call runs the rate-block kernel, and the
  * two agree within the FP32 tolerance (same cells, rounded in another
  * order). The caller passes the parameters, the device normals d_z and the
  * device outputs d_out/d_se (layout as above); everything else -- model

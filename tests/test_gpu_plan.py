@@ -113,3 +113,32 @@ def test_scenarios_of_a_shape_beyond_the_line():
     rng = np.random.default_rng(1)
     cfg.L0 = rng.uniform(0.02, 0.07, (5, 50))
     _run(cfg, 4001, 8, pair=True)
+
+
+@pytest.mark.parametrize("wl,curves,paths", [(4, 1, 1), (4, 1, 3001), (4, 1, 20_001), (3, 1, 500), (3, 1, 9_001), (5, 3, 777)])
+def test_normals_may_change_between_forward_and_backward(wl, curves, paths):
+    """The 80/40 and 160/120 tapes hold what the backward needs, whichever
+    kernels the size selects."""
+    import torch
+    P = pkg()
+    cfg = cfgs().workload(wl, paths)
+    if curves > 1:
+        cfg.L0 = np.ascontiguousarray(cfg.L0[:curves])
+    z = torch.randn(paths * cfg.nmat, device="cuda")
+    grads = []
+    for spoil in (False, True):
+        with P.Engine(cfg) as e:
+            t = e.tape(paths)
+            zz, v = z.clone(), torch.zeros(e.nscen, dtype=torch.float64, device="cuda")
+            g = torch.zeros(e.nscen, 2 * e.nn, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            e.forward_f32_device(zz.data_ptr(), paths, t, v.data_ptr())
+            e.synchronize()
+            if spoil:
+                zz.fill_(3.0)
+                torch.cuda.synchronize()
+            e.backward_f32_device(zz.data_ptr(), t, [1.0] * e.nscen, g.data_ptr())
+            e.synchronize()
+            t.close()
+            grads.append(g.cpu())
+    assert torch.equal(*grads)
