@@ -21,11 +21,12 @@
 // so 16 warps cover the chains (ncu at 1,089,536 paths, 80/40: issue active 76%,
 // dispatch stalls 0.6 of an issue). GB300, 80/40, against the kernel that held
 // 40 rates and 12 warps: 256 curves x 16,384 paths 10.07 -> 9.19 ms, 16,777,216
-// Philox paths 40.57 -> 38.85 ms, 131,072 paths 0.422 -> 0.325 ms. Steps on the
+// Philox paths 40.57 -> 38.5 ms, 131,072 paths 0.422 -> 0.323 ms. Steps on the
 // way (Philox paths): constants read from shared memory (one 16-byte broadcast a
 // position) instead of the parameter bank 39.4 -> 38.4 ms; one barrier per batch
-// instead of one every second step group 40.4 -> 39.4 ms, none 58 ms (the warps
-// drift apart on the code: instruction cache); blocks of 40 / 10 / 8 rates 41.2 /
+// instead of one every second step group 40.4 -> 39.4 ms, one every second batch
+// 40.8, before each reverse half 39.3, none 58 ms (the warps drift apart on the code:
+// instruction cache); blocks of 40 / 10 / 8 rates 41.2 /
 // 42.3 / 45 ms; groups of 5 steps 41.4 ms; ragged batches 38.4 -> 39.7 ms; packed
 // column sums 39.7 -> 38.85 ms. Two paths a thread in packed FP32
 // (fma.rn.f32x2) reads as many operands for a path and ran 40.5 ms.
@@ -560,6 +561,10 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                     for (int i = 0; i < kRR; ++i) sc[(Ly.s_d + LO + i) * B] = Pb[i] * il0_s[LO + i];
                 }
             }
+
+            // a second barrier, of the warps that have paths, before the sums pays with Philox normals
+            // only: 16,777,216 paths 38.90 -> 38.55 ms; 256 curves x 16,384 paths from memory 9.20 -> 9.25
+            if (FIX && PHILOX) asm volatile("bar.sync 1, %0;" ::"r"((batch_left(w, item, jb) + 31) & ~31) : "memory");
 
             // ---- cross-path reduction of this batch ----
             const bool active = tid < batch_left(w, item, jb);
