@@ -287,9 +287,7 @@ int family_at(lmm_engine *e, Mode mode, int64_t paths, int *fam)
 {
     *fam = family_for(e, mode);
     if (*fam == 0 || *fam == 2 || !lmm::f32_wpp_supports(e->nn, e->nmat)) return LMM_OK;
-    int bps = 0;
-    LMM_TRY(blocks_per_sm(e, 2, Mode::Fused, false, &bps));
-    const double fill = (double)e->sms * bps * batch_paths(e, 2);
+    const double fill = (double)e->sms * lmm::wpp_resident(e->nn, e->nmat) * batch_paths(e, 2);
     const double line = fill * wpp_fills(e->nn, e->nmat, family_for(e, Mode::Fused) == 6);
     if (paths * e->nscen <= (int64_t)line) *fam = 2;
     return LMM_OK;

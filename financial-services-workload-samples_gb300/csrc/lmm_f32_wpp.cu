@@ -34,6 +34,8 @@
 // a swaption before, none now). 3,001 paths of 80/40 0.054 -> 0.049 ms.
 #include "lmm_device.cuh"
 
+#include <algorithm>
+
 namespace lmm {
 namespace {
 
@@ -565,6 +567,15 @@ bool f32_wpp_supports(int nn, int nmat)
 }
 
 int wpp_block_threads() { return kWppBlock; }
+
+// Resident blocks of the fused kernel an SM by its registers (wpp_min_blocks) and
+// shared memory (228 KB, 1 KB of it taken for each block): the launch plan's line
+// without an occupancy query, which took 70 us of a new engine's tape.
+int wpp_resident(int nn, int nmat)
+{
+    const int S = wpp_slots(nn);
+    return std::min(wpp_min_blocks(S), (int)(228 * 1024 / (wpp_layout(nn, nmat, S).bytes + 1024)));
+}
 
 cudaError_t wpp_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks)
 {

@@ -104,6 +104,7 @@ cudaError_t launch_tp2_any(const DevModel &m, Mode mode, const float *z, uint64_
 // the saved rates every DevModel::ckpt steps).
 bool f32_wpp_supports(int nn, int nmat);
 int wpp_block_threads();
+int wpp_resident(int nn, int nmat);
 cudaError_t wpp_blocks_per_sm(int nn, int nmat, Mode mode, bool philox, int *blocks);
 // Device scratch the warp-per-path kernels take per warp (floats): the
 // forward's per-step drift sums at each lane's top rate, and rate checkpoints
