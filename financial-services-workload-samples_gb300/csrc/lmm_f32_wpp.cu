@@ -14,7 +14,8 @@
 // every ck steps (DevModel::ckpt, the engine's checkpoint interval; 0: none).
 // The reverse restarts each step from Y_top and runs
 // the Euler step backwards down the lane's own slots,
-//   L_{n,i} = L_{n+1,i} 2^-(a_k Y_i + c_k),  Y_{i-1} = Y_i - delta^2 lambda_k t_i,
+//   IL_{n,i} = IL_{n+1,i} 2^(a_k Y_i + c_k),  Y_{i-1} = Y_i - delta^2 lambda_k t_i
+// on the inverse rates IL = 1/L (t = 1/(IL + delta); a rate that outgrows FP32 is 0),
 // so the serial chain is S cells long, not NN; at every ck-th step it
 // replaces the rebuilt rates by the saved ones, so FP32 rounding of the
 // reconstruction accumulates over at most ck steps. The adjoint in log form
@@ -30,9 +31,11 @@
 // would collect a rounding of L each, and the payoff's factors 1/(1 + delta L)
 // keep their rounding: fewer swaptions at the money pay or not unlike the exact
 // path (100 sets of normals, 80/40, 3,001 paths, median error of the Greeks 2.3e-7 ->
-// 5.6e-8; 50/20, 1,500 paths 4.5e-7 -> 7.9e-8; the latter with 2 sets that differ in
+// 3.8e-8; 50/20, 1,500 paths 4.5e-7 -> 3.1e-8; the latter with 2 sets that differ in
 // a swaption before, none now). 3,001 paths of 80/40 0.054 -> 0.049 ms.
 #include "lmm_device.cuh"
+
+#include "lmm_f32_payoff.cuh"
 
 #include <algorithm>
 
@@ -69,7 +72,7 @@ __host__ __device__ constexpr size_t al16(size_t x) { return (x + 15) & ~size_t(
 // Shared-memory layout (bytes), shared by host and device.
 struct WppLay {
     int nn, nmat, S, nout, M;
-    size_t kc, l0, il0, ost, okf, owf, okk, warp0, per_warp, vg, lw, bw, acc, bytes;
+    size_t kc, il0, ost, okf, owf, okk, warp0, per_warp, vg, lw, bw, acc, bytes;
 };
 
 // Rows in front of the tables: row k + head holds k; rows below head are zero
@@ -86,7 +89,6 @@ __host__ __device__ inline WppLay wpp_layout(int nn, int nmat, int S, Mode mode 
     L.nout = mode == Mode::Fused ? 1 + 2 * nn : (mode == Mode::Forward ? 1 : 2 * nn);
     size_t o = 0;
     L.kc = o; o = al16(o + 16 * (size_t)(nn + wpp_head(nmat)));   // head zero rows, then constants of k
-    L.l0 = o; o = al16(o + 4 * (size_t)nn);
     L.il0 = o; o = al16(o + 4 * (size_t)nn);
     L.ost = o; o = al16(o + 4 * (size_t)(L.M + 1));
     L.okf = o; o = al16(o + 4 * (size_t)kMaxNopt);
@@ -157,11 +159,11 @@ __device__ __forceinline__ int wpp_row(const int (&base)[S], int s, int n)
     return LMM_WPP_PAD ? base[s] - n : max(base[s] - n, 0);
 }
 
-// One forward step n over the lane's slots, on D = log2(L/L0) and the rates L that
-// follow from it; returns Y at the lane's top slot (its drift sum plus
+// One forward step n over the lane's slots, on D = log2(L/L0) and the inverse rates
+// that follow from it; returns Y at the lane's top slot (its drift sum plus
 // sqrt(delta) z), from which the reverse restarts.
 template <int S>
-__device__ __forceinline__ float wpp_fwd_step(float (&L)[S], float (&D)[S], const float (&L0)[S], const int (&base)[S], int n,
+__device__ __forceinline__ float wpp_fwd_step(float (&IL)[S], float (&D)[S], const float (&IL0)[S], const int (&base)[S], int n,
                                               float sqez, int lane, const float4 *kc, float delta)
 {
     float a[S];
@@ -170,26 +172,25 @@ __device__ __forceinline__ float wpp_fwd_step(float (&L)[S], float (&D)[S], cons
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         kk[s] = kc[wpp_row(base, s, n)];
-        const float r = rcp_approx(fmaf(delta, L[s], 1.0f));
-        P = fmaf(kk[s].z, L[s] * r, P);
+        P = fmaf(kk[s].z, rcp_approx(IL[s] + delta), P);
         a[s] = P;                                   // local inclusive prefix
     }
     const float X = warp_excl_prefix(P, lane) + sqez;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         D[s] += fmaf(kk[s].x, X + a[s], kk[s].y);
-        L[s] = L0[s] * ex2_approx(D[s]);
+        IL[s] = IL0[s] * ex2_approx(-D[s]);
     }
     return X + a[S - 1];
 }
 
-// Reverse step n (path_calc_b2 :100-112 in log-adjoint form) + vega: L holds
-// L_{n+1} on entry and L_n on exit; ytop is the forward's Y at the lane's top
+// Reverse step n (path_calc_b2 :100-112 in log-adjoint form) + vega: IL holds
+// 1/L_{n+1} on entry and 1/L_n on exit; ytop is the forward's Y at the lane's top
 // slot. The suffix sum, taken over the log-adjoints before the step's update,
 // is carried as S' = delta^2 S (sums of delta^2 lambda_k Pb), so that
 // Pb += lambda_k r t S' and the vega term t S' need no further factor.
 template <int S>
-__device__ __forceinline__ void wpp_rev_step(float (&L)[S], float (&Pb)[S], const int (&base)[S], int n,
+__device__ __forceinline__ void wpp_rev_step(float (&IL)[S], float (&Pb)[S], const int (&base)[S], int n,
                                              int lane, float ytop, const float4 *kc, float *vg, float delta)
 {
     float b[S];
@@ -205,27 +206,17 @@ __device__ __forceinline__ void wpp_rev_step(float (&L)[S], float (&Pb)[S], cons
     float Y = ytop;
 #pragma unroll
     for (int s = S - 1; s >= 0; --s) {
-        const float Ln = L[s] * ex2_approx(-fmaf(kk[s].x, Y, kk[s].y));
-        const float r = rcp_approx(fmaf(delta, Ln, 1.0f));
-        const float t = Ln * r;
+        IL[s] *= ex2_approx(fmaf(kk[s].x, Y, kk[s].y));
+        const float t = rcp_approx(IL[s] + delta);
         const float tS = t * (Yx + b[s]);
         vg[wpp_row(base, s, n)] += fmaf(Pb[s], fmaf(-delta, kk[s].w, Y), tS);
-        Pb[s] = fmaf(kk[s].w * r, tS, Pb[s]);
-        L[s] = Ln;
+        // r = IL t keeps its precision on high rates, where 1 - delta t would cancel; t = 0 beside IL = inf
+        Pb[s] = fmaf(kk[s].w * (fminf(IL[s], 1e30f) * t), tS, Pb[s]);
         Y = fmaf(-kk[s].z, t, Y);
     }
     // The next step's vega rows overlap neighbouring lanes' rows of this
     // step: order the shared-memory read-modify-writes across the warp.
     __syncwarp();
-}
-
-// 1/(1 + delta L), with the rounding of the reciprocal and of the sum while
-// delta L < 1.
-__device__ __forceinline__ F2 wpp_ratio(float L, float delta)
-{
-    const float q = fmaf(delta, L, 1.0f), r = __frcp_rn(q);
-    const float e = __fmaf_rn(delta, L, __fsub_rn(1.0f, q));
-    return {r, q < 2.0f ? r * __fmaf_rn(-r, e, __fmaf_rn(-r, q, 1.0f)) : 0.0f};
 }
 
 template <bool PHILOX>
@@ -277,7 +268,6 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     const WppLay Ly = wpp_layout(nn, nmat, S, MODE);
     const int M = Ly.M, nout = Ly.nout;
     float4 *kc_s = reinterpret_cast<float4 *>(smem + Ly.kc);
-    float *l0_s = reinterpret_cast<float *>(smem + Ly.l0);
     float *il0_s = reinterpret_cast<float *>(smem + Ly.il0);
     int *ost_s = reinterpret_cast<int *>(smem + Ly.ost);
     float *okf_s = reinterpret_cast<float *>(smem + Ly.okf);
@@ -319,11 +309,8 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     const int units = m.nscen * w.items;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
         const int scen = unit / w.items, item = unit % w.items;
-        __syncthreads();          // the previous unit's reads of l0/il0 are done
-        for (int i = tid; i < nn; i += kWppBlock) {
-            l0_s[i] = m.L0f[scen * nn + i];
-            il0_s[i] = m.invL0f[scen * nn + i];
-        }
+        __syncthreads();          // the previous unit's reads of il0 are done
+        for (int i = tid; i < nn; i += kWppBlock) il0_s[i] = m.invL0f[scen * nn + i];
         for (int i = lane; i < 2 * nout; i += 32) acc[i] = 0.0;
         __syncthreads();
 
@@ -334,23 +321,23 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             const uint64_t gpath = (uint64_t)(path0 + p);
             ZChunk<PHILOX> zc;
 
-            float L[S], Pb[S], L0[S], D[S];
+            float IL[S], Pb[S], IL0[S], D[S];
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int i = S * lane + s;
-                L[s] = L0[s] = i < nn ? l0_s[i] : 1.0f;
+                IL[s] = IL0[s] = i < nn ? il0_s[i] : 1.0f;
                 D[s] = 0.0f;
             }
             // ---- forward ----
             for (int n = 0; n < nmat; ++n) {
                 if (MODE != Mode::Forward && ckn > 0 && n % ckn == 0) {
 #pragma unroll
-                    for (int s = 0; s < S; ++s) ck[((n / ckn) * S + s) * 32] = L[s];
+                    for (int s = 0; s < S; ++s) ck[((n / ckn) * S + s) * 32] = IL[s];
                 }
                 const float sqez = sqd * zc.get(n, zp, nmat, seed, gpath, lane);
                 if (MODE == Mode::Forward && !PHILOX && ytop && scen == 0 && (n & 31) == 0 && n + lane < nmat)
                     ytop[p * nmat + n + lane] = zc.v[0];
-                const float y = wpp_fwd_step<S>(L, D, L0, base, n, sqez, lane, kc_s, delta);
+                const float y = wpp_fwd_step<S>(IL, D, IL0, base, n, sqez, lane, kc_s, delta);
                 if (MODE != Mode::Forward) yt[n * 32] = y;
             }
             // ---- payoff (double-FP32 products) and its adjoint ----
@@ -358,12 +345,12 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int i = S * lane + s;
-                L[s] = L0[s] * ex2_ulp(D[s]);
-                const F2 r = wpp_ratio(L[s], delta);
+                IL[s] = IL0[s] * ex2_ulp(-D[s]);
+                const F2 r = bond_ratio2(IL[s], delta);
                 if (i < nmat) {
                     dprod = f2_mul(dprod, r);
                 } else if (i < nn) {
-                    lw_s[i] = L[s];
+                    lw_s[i] = rcp_approx(IL[s] + delta);
                     rt_s[i - nmat] = r.hi;
                     bw_s[i - nmat] = r.lo;
                 }
@@ -429,7 +416,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
                 const float scale = -vb * dprod.hi * delta;
                 for (int mm = m1 - 1; mm >= m0; --mm) {
                     W += bw_s[mm];
-                    lw_s[nmat + mm] = scale * W * (lw_s[nmat + mm] * rt_s[mm]);
+                    lw_s[nmat + mm] *= scale * W;
                 }
             }
             V = __shfl_sync(0xffffffffu, V, 0);
@@ -447,7 +434,7 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int i = S * lane + s;
-                if (i < nmat) Pb[s] = vsd * (L[s] * __frcp_rn(fmaf(delta, L[s], 1.0f)));
+                if (i < nmat) Pb[s] = vsd * rcp_approx(IL[s] + delta);
                 else Pb[s] = i < nn ? lw_s[i] : 0.0f;
             }
             // ---- reverse: each step rebuilt from the forward's Y_top ----
@@ -455,10 +442,10 @@ k_wpp(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
             for (int n = nmat - 1; n >= 0; --n) {
                 const float y = ynext;
                 if (n > 0) ynext = yt[(n - 1) * 32];
-                wpp_rev_step<S>(L, Pb, base, n, lane, y, kc_s, vg_s, delta);
+                wpp_rev_step<S>(IL, Pb, base, n, lane, y, kc_s, vg_s, delta);
                 if (ckn > 0 && n % ckn == 0) {
 #pragma unroll
-                    for (int s = 0; s < S; ++s) L[s] = ck[((n / ckn) * S + s) * 32];
+                    for (int s = 0; s < S; ++s) IL[s] = ck[((n / ckn) * S + s) * 32];
                 }
             }
             // ---- accumulate this path: value, deltas, vegas ----

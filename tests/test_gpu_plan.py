@@ -142,3 +142,20 @@ def test_normals_may_change_between_forward_and_backward(wl, curves, paths):
             t.close()
             grads.append(g.cpu())
     assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("wl,paths", [(3, 2000), (3, 9001), (4, 3000), (4, 20_001)])
+@pytest.mark.parametrize("shock", [30.0, 100.0, -100.0])
+def test_rates_beyond_fp32(wl, paths, shock):
+    """One path whose rates outgrow FP32: its discount factor is 0, and the call
+    prices the others, whichever kernel the size selects."""
+    cfg = cfgs().workload(wl, paths)
+    z = np.random.default_rng(3).standard_normal(paths * cfg.nmat).astype(np.float32)
+    z[cfg.nmat * 7 + 3] = shock
+    ref = np.delete(z.reshape(paths, cfg.nmat), 7, 0).ravel()
+    with pkg().Engine(cfg) as e:
+        out, _ = e.greeks_f32(z, paths)
+        base, _ = e.greeks_f32(ref, paths - 1)
+    assert np.isfinite(out).all()
+    # one path more or less moves the mean by at most its share of the largest values
+    np.testing.assert_allclose(out.reshape(-1)[0], base.reshape(-1)[0], rtol=10.0 / paths)
