@@ -101,9 +101,11 @@ __host__ __device__ constexpr TpbLay tpb_layout(int nn, int nmat, Mode mode, int
     L.s_x = L.s_s + nmat;
     L.s_d = L.s_x + kFR * L.nf;
     L.s_b = L.s_d + kRR * L.nr;
-    L.s_p = L.s_b + L.M;
-    L.s_q = L.s_p + nmat;
-    L.s_g = L.s_q + nmat;
+    // 80/40 keeps its annuity factors in shared memory and the normal terms in the drift sums
+    const bool lean = nn == 80 && nmat == 40;
+    L.s_p = L.s_b + (lean ? 0 : L.M);
+    L.s_q = L.s_p + (lean ? 0 : nmat);
+    L.s_g = L.s_q + (lean ? 0 : nmat);
     L.s_a = L.s_g + (win ? kRR * L.nr : 0);
     L.s_ck = L.s_a + (win ? (1 + 2 * nn + 7) / 8 : 0);      // 2 nout doubles a warp
     return L;
@@ -265,7 +267,7 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
       float *__restrict__ tape, const double *__restrict__ vbar, int mode_arg)
 {
     constexpr bool FIX = NN > 0;
-    constexpr bool LOGS = !FIX, CK = !FIX || WIN;
+    constexpr bool LOGS = !FIX, CK = !FIX;
     constexpr bool TAPED = !CK && MODE == Mode::Backward;
     constexpr int NW = B / 32;
     const Mode mode = FIX ? MODE : (Mode)mode_arg;
@@ -310,7 +312,8 @@ k_tpb(const DevModel m, const float *__restrict__ z, uint64_t seed, int64_t path
     float *vg0 = vg_s + (WIN ? 0 : kRG * B) + tid;
     float *sc = sb + tid;                                            // sc[row * B]
     const bool vec = FIX ? NMAT % 4 == 0 : (nmat & 3) == 0;
-    const bool bsm = FIX ? 2 * (NN - NMAT) <= (WIN ? tpb_win(Ly.seg) : kRR * ((NN + kRR - 1) / kRR)) : false;   // annuity factors in shared memory
+    static_assert(!FIX || (NN == 80 && NMAT == 40 && !WIN), "the scratch rows of 80/40");
+    constexpr bool bsm = FIX;      // annuity factors in shared memory
 
     const int units = m.nscen * w.items;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
